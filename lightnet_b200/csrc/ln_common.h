@@ -33,8 +33,7 @@ struct ln_ctx {
     std::map<void*, size_t> live_blocks;       // true size of every block handed out
     size_t pool_bytes = 0;                     // bytes held from the device: live + cached
     size_t cached_bytes = 0;
-    int* d_status = nullptr;  // device status word written by kernels whose bounded waits give up
-    int* h_status = nullptr;  // pinned mirror
+    int* h_status = nullptr;  // status word in page-locked memory, written by kernels whose bounded waits give up
     ln_encode_tiled_fn encode_tiled = nullptr;
     long long* debug_cycles = nullptr;  // when set (LN_DEBUG_CYCLES=1), the tensor-core convolution records role timings of CTA 0
     std::set<const void*> configured_kernels;  // kernels whose dynamic shared memory limit has been raised
@@ -78,6 +77,8 @@ struct ln_conv_weights {
 };
 
 int ln_fail(ln_ctx* ctx, int code, const char* fmt, ...);
+int ln_status(ln_ctx* ctx, const char* where);        // after a synchronisation: LN_OK or LN_ERR_TIMEOUT (and clears the word)
+int ln_check_status(ln_ctx* ctx, const char* where);  // synchronises the ctx stream first
 int ln_image_preprocess_enqueue(ln_ctx* ctx, cudaStream_t stream, const uint8_t* pixels_host, const int64_t* offsets, const int32_t* widths,
                                 const int32_t* heights, int32_t count, int32_t mode, int32_t dst_w, int32_t dst_h, float* dst, void** staging,
                                 size_t* staging_bytes);

@@ -130,9 +130,6 @@ int ln_conv_stem_launch(ln_ctx* ctx, int kind, const float* x_nchw, float inv_sx
                         const float2* mb, int F, int k, int stride, int pad, int OH, int OW, int act, float inv_sy, void* out,
                         long long out_pixel_stride, int s2d_out = 0);
 
-// Reads the device status word; returns LN_OK or LN_ERR_TIMEOUT (and clears the word).
-int ln_check_status(ln_ctx* ctx, const char* where);
-
 // The fast int8 epilogue converts an accumulator to binary32 by adding it to the bits of 1.5 * 2^23, which needs |accumulator| < 2^22.
 // Where the bound 127 * max_l1 (max_l1 = largest sum of |weight code| of a filter) is larger, the low `shift` bits are dropped
 // first; that moves a pre-activation by at most 2^(shift - 1) accumulator units (the mean is put back into the bias), i.e.

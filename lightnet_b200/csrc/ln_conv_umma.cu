@@ -85,7 +85,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         if ((it & 255u) == 255u && *abort_flag) return false;
     }
     *abort_flag = 1;
-    atomicExch(status, code);
+    *(volatile int*)status = code;  // page-locked host memory: the host reads it after its next synchronisation
+    __threadfence_system();
     return false;
 }
 
@@ -1165,7 +1166,7 @@ int ln_conv_umma_plan_build(ln_ctx* ctx, ln_conv_umma_plan* plan, const ln_conv_
     p.res = g.res; p.res_pixel_stride = g.res_pixel_stride; p.s_c = g.s_c; p.s_res = g.s_res; p.inv_sy2 = g.inv_sy2;
     if (g.res && (g.out_kind != LN_OUT_Q || g.kind != LN_KIND_I8 || g.F % 32 != 0 || (((uintptr_t)g.res) & 15) || (g.res_pixel_stride & 15)))
         return ln_fail(ctx, LN_ERR_UNSUPPORTED, "tensor-core convolution: a fused shortcut needs int8 output, filters a multiple of 32 and 16-byte aligned residuals");
-    p.status = ctx->d_status;
+    p.status = ctx->h_status;
     p.debug = ctx->debug_cycles;
     p.mb = mb;
     p.mb_folded = nullptr;
@@ -1324,10 +1325,10 @@ static int32_t mma_peak_run(ln_ctx* ctx, int32_t dtype, int32_t n, int32_t pair_
         cudaError_t e;                                                                                                       \
         if (pair) {                                                                                                          \
             e = cudaFuncSetAttribute(mma_peak_kernel<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);      \
-            if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, mma_peak_kernel<K, true>, it, (int)n, variant, ctx->d_status);         \
+            if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, mma_peak_kernel<K, true>, it, (int)n, variant, ctx->h_status);         \
         } else {                                                                                                             \
             e = cudaFuncSetAttribute(mma_peak_kernel<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
-            if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, mma_peak_kernel<K, false>, it, (int)n, variant, ctx->d_status);        \
+            if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, mma_peak_kernel<K, false>, it, (int)n, variant, ctx->h_status);        \
         }                                                                                                                    \
         return e;                                                                                                            \
     }

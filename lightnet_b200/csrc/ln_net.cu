@@ -262,7 +262,7 @@ struct ln_net {
     size_t slot_staging_bytes[2] = {0, 0};
     long long submitted = 0, collected = 0;
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
-    float times_ms[2] = {0, 0};
+    int timed = 0;  // events ln_net_last_times has to read: 0 none, 1 of this network, 2 of the two part networks
     // CUDA graph of the 8-bit plan (one graph = the whole batch: every micro-batch, every layer)
     bool fuse_shortcut = true;  // a linear [shortcut] whose input is a convolution nobody else reads runs in that convolution's epilogue
     std::vector<char> fused_into_next;  // per layer (8-bit plan): 1 = runs in the next layer's shortcut epilogue, no output; 2 = output kept in space-to-depth layout
@@ -1013,7 +1013,8 @@ int run_plan(ln_net* net, const float* input_dev_f32) {
     return LN_OK;
 }
 
-int forward_any(ln_net* net, const ln_tensor* input) {
+// `wait` = false: the caller synchronises the stream and reads the status word itself (the detect calls, after decode + NMS).
+int forward_any(ln_net* net, const ln_tensor* input, bool wait = true) {
     ln_ctx* ctx = net->ctx;
     if (!net->weights_loaded) return ln_fail(ctx, LN_ERR_ARG, "weights are not loaded");
     if (!input || input->dtype != LN_F32 || input->n != net->batch || input->c != net->channels || input->h != net->height || input->w != net->width)
@@ -1066,7 +1067,6 @@ int forward_any(ln_net* net, const ln_tensor* input) {
             }
             slot->used = ++net->graph_clock;
         }
-        if (rc == LN_OK) rc = ln_check_status(ctx, "ln_net_forward");
     }
     if (rc) return rc;
     // anchor-free heads: the head layer's own forward, on the raw f32 tensor the convolution before it wrote: the output activation
@@ -1089,7 +1089,7 @@ int forward_any(ln_net* net, const ln_tensor* input) {
         }
     }
     LN_CUDA(ctx, cudaEventRecord(net->ev[1], ctx->stream));
-    return LN_OK;
+    return wait && net->precision != LN_F32 && net->precision != LN_F16 ? ln_check_status(ctx, "ln_net_forward") : LN_OK;
 }
 
 int fill_heads(ln_net* net, std::vector<ln_yolo_head>& hs, const std::vector<ln_tensor*>* tensors = nullptr) {
@@ -1429,18 +1429,17 @@ int32_t ln_net_layer_output(ln_net* net, int32_t layer, ln_tensor** out) {
 int32_t ln_net_detect_device(ln_net* net, const ln_tensor* input, const int32_t* image_w, const int32_t* image_h, const ln_detect_options* opts,
                              ln_detection* records_host, int32_t* counts_host) {
     if (!net || !image_w || !image_h || !opts || !records_host || !counts_host) return ln_fail(net ? net->ctx : nullptr, LN_ERR_ARG, "ln_net_detect: NULL argument");
-    int rc = forward_any(net, input);
+    int rc = forward_any(net, input, false);
     if (rc) return rc;
     std::vector<ln_yolo_head> hs;
     rc = fill_heads(net, hs);
     if (rc) return rc;
-    rc = ln_yolo_decode_nms(net->ctx, hs.data(), (int)hs.size(), net->width, net->height, image_w, image_h, opts, records_host, counts_host);
-    if (rc) return rc;
     ln_ctx* ctx = net->ctx;
+    rc = ln_yolo_decode_nms(ctx, hs.data(), (int)hs.size(), net->width, net->height, image_w, image_h, opts, records_host, counts_host);
+    const int waited = ln_check_status(ctx, "ln_net_forward");
+    if (waited || rc) return waited ? waited : rc;
     LN_CUDA(ctx, cudaEventRecord(net->ev[2], ctx->stream));
-    LN_CUDA(ctx, cudaEventSynchronize(net->ev[2]));
-    cudaEventElapsedTime(&net->times_ms[0], net->ev[0], net->ev[1]);
-    cudaEventElapsedTime(&net->times_ms[1], net->ev[1], net->ev[2]);
+    net->timed = 1;
     return LN_OK;
 }
 
@@ -1473,21 +1472,17 @@ int32_t ln_net_detect(ln_net* net, const float* input_host, const int32_t* image
         for (int h = 0; h < 2; ++h) {
             ln_net* c = net->pipe[h];
             LN_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, net->copy_ev[h], 0));
-            rc = forward_any(c, c->input_dev);
+            rc = forward_any(c, c->input_dev, false);
             if (rc) return rc;
         }
         std::vector<ln_yolo_head> hs;
         rc = fill_heads(net, hs, &net->pipe_heads);
         if (rc) return rc;
         rc = ln_yolo_decode_nms(ctx, hs.data(), (int)hs.size(), net->width, net->height, image_w, image_h, opts, records_host, counts_host);
-        if (rc) return rc;
+        const int waited = ln_check_status(ctx, "ln_net_forward");
+        if (waited || rc) return waited ? waited : rc;
         LN_CUDA(ctx, cudaEventRecord(net->ev[2], ctx->stream));
-        LN_CUDA(ctx, cudaEventSynchronize(net->ev[2]));
-        float part[2] = {0.0f, 0.0f}, nms = 0.0f;
-        for (int h = 0; h < 2; ++h) cudaEventElapsedTime(&part[h], net->pipe[h]->ev[0], net->pipe[h]->ev[1]);
-        cudaEventElapsedTime(&nms, net->pipe[1]->ev[1], net->ev[2]);
-        net->times_ms[0] = part[0] + part[1];
-        net->times_ms[1] = nms;
+        net->timed = 2;
         return LN_OK;
     }
     int rc = stage_input(net, input_host);
@@ -1587,9 +1582,14 @@ int32_t ln_net_detect_u8(ln_net* net, const uint8_t* pixels_host, const int64_t*
     }
     // (the two-part pipeline of ln_net_detect does not pay here: the 8-bit upload is a quarter of the f32 one, and two part-batch
     // networks with two decode + NMS calls cost more than overlapping it saves -- measured 4212 against 4630 images/s with halves)
-    int rc = ln_image_preprocess_into(ctx, pixels_host, offsets, widths, heights, net->batch, mode, net->width, net->height, (float*)net->input_dev->ptr);
-    if (rc) return rc;
-    return ln_net_detect_device(net, net->input_dev, widths, heights, opts, records_host, counts_host);
+    void* staging = nullptr;
+    size_t staging_bytes = 0;
+    int rc = ln_image_preprocess_enqueue(ctx, ctx->stream, pixels_host, offsets, widths, heights, net->batch, mode, net->width, net->height,
+                                         (float*)net->input_dev->ptr, &staging, &staging_bytes);
+    if (rc == LN_OK) rc = ln_net_detect_device(net, net->input_dev, widths, heights, opts, records_host, counts_host);
+    if (rc) cudaStreamSynchronize(ctx->stream);  // (every path that succeeds has synchronised: the pixels are the caller's again)
+    if (staging) ln_pool_free(ctx, staging, staging_bytes);
+    return rc;
 }
 
 int32_t ln_net_set_host_pipeline(ln_net* net, int32_t on) {
@@ -1634,8 +1634,17 @@ int32_t ln_net_profile(const ln_net* net, float* per_layer_ms, int32_t num_layer
 
 int32_t ln_net_last_times(const ln_net* net, float times_ms[2]) {
     if (!net || !times_ms) return LN_ERR_ARG;
-    times_ms[0] = net->times_ms[0];
-    times_ms[1] = net->times_ms[1];
+    times_ms[0] = times_ms[1] = 0.0f;
+    if (net->timed && cudaEventSynchronize(net->ev[2]) == cudaSuccess) {
+        for (int h = 0; h < net->timed; ++h) {
+            const ln_net* c = net->timed == 1 ? net : net->pipe[h];
+            float ms = 0.0f;
+            if (!c || cudaEventElapsedTime(&ms, c->ev[0], c->ev[1]) != cudaSuccess) continue;
+            times_ms[0] += ms;
+            if (cudaEventElapsedTime(&ms, c->ev[1], net->ev[2]) == cudaSuccess) times_ms[1] = ms;
+        }
+        (void)cudaGetLastError();
+    }
     return LN_OK;
 }
 

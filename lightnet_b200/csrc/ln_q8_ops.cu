@@ -933,11 +933,14 @@ int kind_of(int dtype) { return dtype == LN_F8 ? LN_KIND_F8 : LN_KIND_I8; }
 }  // namespace
 
 int ln_check_status(ln_ctx* ctx, const char* where) {
-    LN_CUDA(ctx, cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     LN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    int s = *ctx->h_status;
+    return ln_status(ctx, where);
+}
+
+int ln_status(ln_ctx* ctx, const char* where) {
+    const int s = *(volatile int*)ctx->h_status;
     if (s == LN_STATUS_OK) return LN_OK;
-    cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream);
+    *ctx->h_status = LN_STATUS_OK;
     return ln_fail(ctx, LN_ERR_TIMEOUT, "%s: a bounded device-side wait gave up (status %d: %s)", where, s,
                    s == LN_STATUS_PRODUCER_TIMEOUT ? "TMA producer" : s == LN_STATUS_MMA_TIMEOUT ? "MMA issuer" : s == LN_STATUS_EPILOGUE_TIMEOUT ? "epilogue" : "unknown");
 }

@@ -149,9 +149,8 @@ int32_t ln_ctx_create(int32_t device, ln_ctx** out) {
     ctx->sm_count = prop.multiProcessorCount;
     e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) { delete ctx; return ln_fail(nullptr, LN_ERR_CUDA, "cudaStreamCreate: %s", cudaGetErrorString(e)); }
-    e = cudaMalloc(&ctx->d_status, 64);
-    if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_status, 0, 64, ctx->stream);
-    if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_status, 64);
+    e = cudaMallocHost(&ctx->h_status, 64);  // (unified addressing: kernels write it through the same pointer)
+    if (e == cudaSuccess) memset(ctx->h_status, 0, 64);
     if (e != cudaSuccess) { delete ctx; return ln_fail(nullptr, LN_ERR_CUDA, "status word allocation: %s", cudaGetErrorString(e)); }
     void* fn = nullptr;
     cudaDriverEntryPointQueryResult qres;
@@ -175,7 +174,6 @@ int32_t ln_ctx_destroy(ln_ctx* ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     for (auto& kv : ctx->free_blocks) cudaFree(kv.second);
-    if (ctx->d_status) cudaFree(ctx->d_status);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
     cudaStreamDestroy(ctx->stream);

@@ -24,6 +24,12 @@
 // that is followed by the next one further down.  The head tensors are the only large input: they are read
 // twice per pool, and nothing of their size is written.
 //
+// At an ordinary threshold all candidates of an image fit in one band, and the selection has nothing to select: a call with a
+// threshold of kDirectThr or more therefore starts with the fill pass alone (every candidate straight into the band) and NMS;
+// an image with more candidates than a band holds falls back to the two stages above.  Host and device meet once per round: the
+// kernels of a round are enqueued back to back (each skips the images that are not in its phase), records and per-image
+// outcome are written to page-locked host memory by the NMS kernel itself.
+//
 // Most of the candidates only need their histogram bin, not their exact bits.  The passes over the heads
 // therefore evaluate the class sigmoid with the hardware ex2 / rcp approximations first and fall back to the
 // exact evaluation only when the approximate key is within kKeySlack units of a boundary that matters (a bin
@@ -54,7 +60,11 @@ constexpr unsigned kKeySlack = 256;
 constexpr long long kPoolBytesTarget = 1ll << 30;  // pools of one call together, unless every candidate fits in less
 
 enum { PHASE_POOL = 0, PHASE_FILL = 1, PHASE_SELECT = 2, PHASE_BAND = 3, PHASE_DONE = 4 };
-enum { FLAG_SELECT_PENDING = 0, FLAG_ACTIVE = 1, FLAG_POOL_PENDING = 2, FLAG_NEED_POOL = 3 };
+
+// Smallest confidence threshold at which the direct fill is tried first.  Below it a detector head passes far more candidates than
+// a band holds (the stress workload at 0.001: 150 k of 2 M per image), and the first pass over the heads would be for nothing; above
+// it an overflow is rare and cheap, because a block that finds its image's band full leaves at once.
+constexpr float kDirectThr = 0.04f;
 
 struct HeadDev {
     const float* raw;  // [batch][n_anchor*(5+classes)][gh*gw]
@@ -159,17 +169,17 @@ __device__ __forceinline__ Box decode_box(const HeadDev& h, const float* img, in
     return b;
 }
 
-// detect.rs:1486-1503 bbox_iou with detection_geometry.rs:14-30 edges
-__device__ __forceinline__ float box_iou(const Box& a, const Box& b) {
+// detect.rs:1486-1503 bbox_iou with detection_geometry.rs:14-30 edges: intersection and union, whose quotient it is (0 when the
+// intersection is not positive)
+__device__ __forceinline__ void box_overlap(const Box& a, const Box& b, float& inter, float& denom) {
     const float al = __fsub_rn(a.x, __fmul_rn(a.w, 0.5f)), at = __fsub_rn(a.y, __fmul_rn(a.h, 0.5f));
     const float ar = __fadd_rn(a.x, __fmul_rn(a.w, 0.5f)), ab = __fadd_rn(a.y, __fmul_rn(a.h, 0.5f));
     const float bl = __fsub_rn(b.x, __fmul_rn(b.w, 0.5f)), bt = __fsub_rn(b.y, __fmul_rn(b.h, 0.5f));
     const float br = __fadd_rn(b.x, __fmul_rn(b.w, 0.5f)), bb = __fadd_rn(b.y, __fmul_rn(b.h, 0.5f));
     const float iw = fmaxf(__fsub_rn(fminf(ar, br), fmaxf(al, bl)), 0.0f), ih = fmaxf(__fsub_rn(fminf(ab, bb), fmaxf(at, bt)), 0.0f);
-    const float inter = __fmul_rn(iw, ih);
-    if (inter <= 0.0f) return 0.0f;
+    inter = __fmul_rn(iw, ih);
     const float aa = __fmul_rn(fmaxf(a.w, 0.0f), fmaxf(a.h, 0.0f)), ba = __fmul_rn(fmaxf(b.w, 0.0f), fmaxf(b.h, 0.0f));
-    return __fdiv_rn(inter, __fsub_rn(__fadd_rn(aa, ba), inter));
+    denom = __fsub_rn(__fadd_rn(aa, ba), inter);
 }
 
 __device__ __forceinline__ int find_head(const YoloParams& p, int ca) {
@@ -348,6 +358,7 @@ __global__ void __launch_bounds__(256) yolo_head_fill_kernel(const __grid_consta
     unsigned long long* dst = st.direct ? band + (size_t)img * p.band_max : pool + (size_t)img * p.pool_max;
     int* fill = st.direct ? band_fill + img : pool_fill + img;
     const int dst_cap = st.direct ? p.band_max : p.pool_max;
+    if (*(volatile int*)fill > dst_cap) return;  // overflowed already: the image starts over, what is missing does not matter
     const int ca = blockIdx.x * blockDim.x + threadIdx.x;
     if (ca < p.total_ca) {
         const HeadDev& h = p.heads[find_head(p, ca)];
@@ -375,6 +386,7 @@ __global__ void __launch_bounds__(256) yolo_head_fill_kernel(const __grid_consta
         t_or |= key;
     };
     auto publish_and_or = [&]() {
+        if (st.direct) return;  // (only the selection inside a pool uses them)
         for (int o = 16; o > 0; o >>= 1) {
             t_and &= __shfl_xor_sync(0xffffffffu, t_and, o);
             t_or |= __shfl_xor_sync(0xffffffffu, t_or, o);
@@ -473,7 +485,7 @@ __device__ __forceinline__ void load_hist_desc(unsigned* h, int nb, unsigned* s_
 // compared with a margin of one half, and an image whose boundary bin looks too large for a pool starts over with the
 // full histogram.  The fill pass counts exactly; should it overflow all the same, the image starts over as well.
 __global__ void __launch_bounds__(256) yolo_pool_select_kernel(const __grid_constant__ YoloParams p, ImgState* __restrict__ states,
-                                                               unsigned* __restrict__ hist, int* __restrict__ flags) {
+                                                               unsigned* __restrict__ hist) {
     const int img = blockIdx.x;
     ImgState st = states[img];
     if (st.phase != PHASE_POOL) return;
@@ -521,7 +533,6 @@ __global__ void __launch_bounds__(256) yolo_pool_select_kernel(const __grid_cons
                 st.prefix = (st.level == 0 ? 0ull : (st.prefix << bits)) | (unsigned long long)b;
                 st.level += 1;
             }
-            atomicAdd(&flags[FLAG_POOL_PENDING], 1);
             states[img] = st;
             return;
         }
@@ -541,8 +552,7 @@ __global__ void __launch_bounds__(256) yolo_pool_select_kernel(const __grid_cons
 // keys than its destination holds (possible only after a sampled histogram) is thrown away and the image starts over
 // with the full histogram.
 __global__ void yolo_after_fill_kernel(ImgState* __restrict__ states, int* __restrict__ band_fill, int* __restrict__ pool_fill, int batch,
-                                       int band_max, int pool_max, int hist_stride, int* __restrict__ flags,
-                                       unsigned long long* __restrict__ key_and_or) {
+                                       int band_max, int pool_max, int hist_stride, unsigned long long* __restrict__ key_and_or) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= batch || states[i].phase != PHASE_FILL) return;
     int* fill = states[i].direct ? band_fill + i : pool_fill + i;
@@ -554,7 +564,6 @@ __global__ void yolo_after_fill_kernel(ImgState* __restrict__ states, int* __res
         states[i].phase = PHASE_POOL;
         states[i].sampled = 0;
         states[i].level = 0;
-        atomicAdd(&flags[FLAG_POOL_PENDING], 1);
         return;
     }
     states[i].sampled = hist_stride > 1 ? 1 : 0;  // for the next pool of this image
@@ -651,8 +660,7 @@ __global__ void __launch_bounds__(256) yolo_pool_scan_kernel(const __grid_consta
 // One block per image: walk the digit histogram of the pool from the top, either fix the band's lower bound or descend
 // into the digit that holds too many candidates (skipping the digits all keys under it share).  Leaves the histogram zeroed.
 __global__ void __launch_bounds__(256) yolo_select_kernel(const __grid_constant__ YoloParams p, ImgState* __restrict__ states,
-                                                          unsigned* __restrict__ hist, unsigned long long* __restrict__ key_and_or,
-                                                          int* __restrict__ flags) {
+                                                          unsigned* __restrict__ hist, unsigned long long* __restrict__ key_and_or) {
     const int img = blockIdx.x;
     ImgState st = states[img];
     if (st.phase != PHASE_SELECT) return;
@@ -719,169 +727,289 @@ __global__ void __launch_bounds__(256) yolo_select_kernel(const __grid_constant_
                 st.level += 1;
             }
         }
-        atomicAdd(&flags[FLAG_SELECT_PENDING], 1);
     }
     states[img] = st;
 }
 
-
-__device__ __forceinline__ void bitonic_sort_desc(unsigned long long* keys, int n_pow2) {
+// Sorts the n keys at `src` in descending order into shared memory.  Bitonic network over n_pow2 (a power of two >= n, at most
+// 1024 * E) slots with E consecutive slots per thread in registers: distances below E are exchanges inside a thread, below 32 E
+// shuffles, and only the rest goes through shared memory (slot e of thread t at e * 1024 + t: no bank conflicts).  Every step
+// through shared memory moves the whole array twice and costs two barriers; with 16 K keys 15 of the 105 steps are left there.
+template <int E>
+__device__ __forceinline__ void block_sort_desc(const unsigned long long* __restrict__ src, int n, int n_pow2, unsigned long long* __restrict__ s) {
+    const int t = (int)threadIdx.x;
+    unsigned long long r[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) r[e] = t * E + e < n ? src[t * E + e] : 0ull;
     for (int k = 2; k <= n_pow2; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < n_pow2; i += blockDim.x) {
-                const int ixj = i ^ j;
-                if (ixj > i) {
-                    const unsigned long long a = keys[i], b = keys[ixj];
-                    const bool desc = (i & k) == 0;
-                    if (desc ? a < b : a > b) { keys[i] = b; keys[ixj] = a; }
-                }
-            }
+        int j = k >> 1;
+        for (; j >= 32 * E; j >>= 1) {
             __syncthreads();
+#pragma unroll
+            for (int e = 0; e < E; ++e) s[e * 1024 + t] = r[e];
+            __syncthreads();
+            const bool keep_max = (((t * E) & j) == 0) == (((t * E) & k) == 0);
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const unsigned long long o = s[e * 1024 + (t ^ (j / E))];
+                r[e] = keep_max ? (r[e] > o ? r[e] : o) : (r[e] < o ? r[e] : o);
+            }
+        }
+        for (; j >= E; j >>= 1) {
+            const bool keep_max = (((t * E) & j) == 0) == (((t * E) & k) == 0);
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const unsigned long long o = __shfl_xor_sync(0xffffffffu, r[e], j / E);
+                r[e] = keep_max ? (r[e] > o ? r[e] : o) : (r[e] < o ? r[e] : o);
+            }
+        }
+#pragma unroll
+        for (int jj = E / 2; jj >= 1; jj >>= 1) {
+            if (jj > j) continue;
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                if (e & jj) continue;
+                const bool desc = ((t * E + e) & k) == 0;
+                const unsigned long long lo = r[e], hi = r[e | jj];
+                const bool swap = desc ? lo < hi : lo > hi;
+                r[e] = swap ? hi : lo;
+                r[e | jj] = swap ? lo : hi;
+            }
         }
     }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < E; ++e) s[t * E + e] = r[e];
+    __syncthreads();
 }
 
-// One CTA per image: sort the band, then greedy per-class NMS chunk by chunk.
+// box_iou(a, b) > thr with the division left out where it cannot matter: the rounded quotient of positive operands is within a few
+// units in the last place of the real one, so a numerator 0.1 % away from thr * denominator decides by itself.
+__device__ __forceinline__ bool iou_above(const float4& a4, const float4& b4, float thr) {
+    Box a, b;
+    a.x = a4.x; a.y = a4.y; a.w = a4.z; a.h = a4.w;
+    b.x = b4.x; b.y = b4.y; b.w = b4.z; b.h = b4.w;
+    float inter, denom;
+    box_overlap(a, b, inter, denom);
+    if (inter <= 0.0f) return 0.0f > thr;
+    const float edge = thr * denom;
+    if (denom > 0.0f && edge > 1e-30f) {
+        if (inter < 0.999f * edge) return false;
+        if (inter > 1.001f * edge) return true;
+    }
+    return __fdiv_rn(inter, denom) > thr;
+}
+
+constexpr int kBuckets = 128;  // survivors and chunk candidates are looked up by class modulo this
+
+// Shared memory of the NMS kernel: sorted keys, survivors (box, class, list of the bucket), the chunk (box, class, objectness,
+// suppressor rows, bucket bitmaps).
+constexpr size_t nms_smem_bytes(int band_max, int k_eff) {
+    return (size_t)band_max * 8 + (size_t)(k_eff + kChunk) * sizeof(float4) + (size_t)kChunk * (kChunk / 32) * 4 + (size_t)kBuckets * (kChunk / 32) * 4 +
+           (size_t)k_eff * 8 + (size_t)kChunk * 12 + (size_t)kBuckets * 4 + 3 * (kChunk / 32) * 4;
+}
+
+// One CTA per image: sort the band, then greedy per-class NMS chunk by chunk.  Only candidates of one class can suppress one
+// another, so a candidate is compared with the survivors of its class bucket (a linked list, both halves of the CTA taking every
+// second entry) and with the earlier candidates of the chunk that share the bucket (128 bitmaps of 512 bits).  The chunk is then
+// resolved in rounds instead of candidate by candidate: a candidate with a kept suppressor is out, one whose suppressors are all
+// out is kept, and the chains are short.  (One image of 608 x 608 with 900 survivors: 515 us when every candidate was compared with
+// every survivor and one warp walked the chunk.)
+// Also takes images whose band was filled directly (PHASE_FILL): too many candidates send them back to PHASE_POOL.
+// counts[img]: records kept once the image is done, -1 - phase while it is not.
 __global__ void __launch_bounds__(1024, 1) yolo_nms_kernel(const __grid_constant__ YoloParams p, ImgState* __restrict__ states,
                                                            const unsigned long long* __restrict__ band, int* __restrict__ band_fill,
                                                            float4* __restrict__ kept_box, int* __restrict__ kept_cls,
-                                                           ln_detection* __restrict__ records, int* __restrict__ flags) {
-    extern __shared__ unsigned char smem[];
-    const int img = blockIdx.x;
+                                                           float* __restrict__ records, int* __restrict__ counts) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int W = kChunk / 32;
+    static_assert(kChunk * 28 <= kChunk * W * 4, "the record staging of a chunk reuses the suppressor rows");
+    const int img = blockIdx.x, tid = (int)threadIdx.x;
     ImgState st = states[img];
-    if (st.phase != PHASE_BAND) return;
-    unsigned long long* keys = reinterpret_cast<unsigned long long*>(smem);             // band_max
-    float4* kbox = reinterpret_cast<float4*>(keys + p.band_max);                          // k_eff survivors
-    float4* cbox = kbox + p.k_eff;                                                       // kChunk
-    unsigned* mask = reinterpret_cast<unsigned*>(cbox + kChunk);                         // kChunk x 16 words
-    int* kcls = reinterpret_cast<int*>(mask + kChunk * (kChunk / 32));                   // k_eff
-    int* ccls = kcls + p.k_eff;                                                          // kChunk
-    float* cobj = reinterpret_cast<float*>(ccls + kChunk);                               // kChunk
-    int* cpos = reinterpret_cast<int*>(cobj + kChunk);                                   // kChunk: survivor slot or -1
-    unsigned* alive_words = reinterpret_cast<unsigned*>(cpos + kChunk);                  // 16
-    __shared__ int s_kept;
-
     int n = band_fill[img];
-    if (n > p.band_max) n = p.band_max;
-    int n2 = 1;
-    while (n2 < n) n2 <<= 1;
-    for (int i = threadIdx.x; i < n2; i += blockDim.x) keys[i] = i < n ? band[(size_t)img * p.band_max + i] : 0ull;
-    for (int i = threadIdx.x; i < st.kept; i += blockDim.x) {
-        kbox[i] = kept_box[(size_t)img * p.k_eff + i];
-        kcls[i] = kept_cls[(size_t)img * p.k_eff + i];
+    if (st.phase == PHASE_FILL && n > p.band_max) {
+        if (tid == 0) {
+            band_fill[img] = 0;
+            states[img].phase = PHASE_POOL;
+            counts[img] = -1 - PHASE_POOL;
+        }
+        return;
     }
-    if (threadIdx.x == 0) s_kept = st.kept;
-    __syncthreads();
-    bitonic_sort_desc(keys, n2);
+    if (st.phase != PHASE_BAND && st.phase != PHASE_FILL) {
+        if (tid == 0 && st.phase != PHASE_DONE) counts[img] = -1 - st.phase;
+        return;
+    }
+    unsigned long long* keys = reinterpret_cast<unsigned long long*>(smem);    // band_max
+    float4* kbox = reinterpret_cast<float4*>(keys + p.band_max);               // k_eff survivors
+    float4* cbox = kbox + p.k_eff;                                             // kChunk
+    unsigned* mask = reinterpret_cast<unsigned*>(cbox + kChunk);               // kChunk x W words: row i = earlier candidates that suppress i
+    unsigned* cbits = mask + kChunk * W;                                       // kBuckets x W words: candidates of the chunk by bucket
+    int* kcls = reinterpret_cast<int*>(cbits + kBuckets * W);                  // k_eff
+    int* knext = kcls + p.k_eff;                                               // k_eff: next survivor of the bucket, -1 = last
+    int* ccls = knext + p.k_eff;                                               // kChunk
+    float* cobj = reinterpret_cast<float*>(ccls + kChunk);                     // kChunk
+    unsigned* row_words = reinterpret_cast<unsigned*>(cobj + kChunk);          // kChunk: which words of the row are not zero
+    int* khead = reinterpret_cast<int*>(row_words + kChunk);                   // kBuckets
+    unsigned* alive_words = reinterpret_cast<unsigned*>(khead + kBuckets);     // W
+    volatile unsigned* kept_words = alive_words + W;                           // W
+    volatile unsigned* out_words = alive_words + 2 * W;                        // W
 
-    for (int base = 0; base < n; base += kChunk) {
+    if (n > p.band_max) n = p.band_max;
+    int n2 = 32;
+    while (n2 < n) n2 <<= 1;
+    for (int i = tid; i < kBuckets; i += 1024) khead[i] = -1;
+    __syncthreads();
+    for (int i = tid; i < st.kept; i += 1024) {
+        const int c = kept_cls[(size_t)img * p.k_eff + i];
+        kbox[i] = kept_box[(size_t)img * p.k_eff + i];
+        kcls[i] = c;
+        knext[i] = atomicExch(&khead[c % kBuckets], i);
+    }
+    const unsigned long long* src = band + (size_t)img * p.band_max;
+    if (n2 <= 1024) block_sort_desc<1>(src, n, n2, keys);
+    else if (n2 == 2048) block_sort_desc<2>(src, n, n2, keys);
+    else if (n2 == 4096) block_sort_desc<4>(src, n, n2, keys);
+    else if (n2 == 8192) block_sort_desc<8>(src, n, n2, keys);
+    else block_sort_desc<16>(src, n, n2, keys);
+
+    int kept = st.kept;
+    for (int base = 0; base < n && kept < p.k_eff; base += kChunk) {
         const int m = min(kChunk, n - base);
-        const int kept_before = s_kept;
-        // ---- decode the chunk and test it against the survivors so far
-        bool alive = false;
-        if ((int)threadIdx.x < m) {
-            const unsigned long long key = keys[base + threadIdx.x];
-            const unsigned eidx = 0xFFFFFFFFu - (unsigned)(key & 0xFFFFFFFFull);
-            const int cls = (int)(eidx % (unsigned)p.classes), ca = (int)(eidx / (unsigned)p.classes);
-            const int hd = find_head(p, ca);
-            const HeadDev& h = p.heads[hd];
-            const int stride = h.gw * h.gh, epa = h.classes + 5;
-            const int local = ca - h.ca_base, a = local / stride, idx = local - a * stride;
-            const float* img_raw = h.raw + (size_t)img * h.n_anchor * epa * stride;
-            const Box b = decode_box(h, img_raw, a, idx, p.net_w, p.net_h, st.img_w, st.img_h, p.letterbox);
-            cbox[threadIdx.x] = make_float4(b.x, b.y, b.w, b.h);
-            ccls[threadIdx.x] = cls;
-            cobj[threadIdx.x] = head_act(img_raw[(size_t)(a * epa + 4) * stride + idx], h.new_coords);
-            alive = true;
-            for (int k = 0; k < kept_before; ++k) {
-                if (kcls[k] != cls) continue;
-                const float4 kb = kbox[k];
-                Box q; q.x = kb.x; q.y = kb.y; q.w = kb.z; q.h = kb.w;
-                if (box_iou(q, b) > p.nms_thr) { alive = false; break; }
+        const int slot = tid & (kChunk - 1), half = tid / kChunk;  // threads 512 and up help candidate slot
+        for (int i = tid; i < kBuckets * W; i += 1024) cbits[i] = 0u;
+        if (tid < W) { alive_words[tid] = 0u; kept_words[tid] = 0u; }
+        // ---- decode the chunk
+        if (tid < kChunk) {
+            row_words[tid] = 0u;
+            if (tid < m) {
+                const unsigned eidx = 0xFFFFFFFFu - (unsigned)(keys[base + tid] & 0xFFFFFFFFull);
+                const int cls = (int)(eidx % (unsigned)p.classes), ca = (int)(eidx / (unsigned)p.classes);
+                const HeadDev& h = p.heads[find_head(p, ca)];
+                const int stride = h.gw * h.gh, epa = h.classes + 5;
+                const int local = ca - h.ca_base, a = local / stride, idx = local - a * stride;
+                const float* img_raw = h.raw + (size_t)img * h.n_anchor * epa * stride;
+                const float obj_raw = img_raw[(size_t)(a * epa + 4) * stride + idx];
+                const Box b = decode_box(h, img_raw, a, idx, p.net_w, p.net_h, st.img_w, st.img_h, p.letterbox);
+                cbox[tid] = make_float4(b.x, b.y, b.w, b.h);
+                ccls[tid] = cls;
+                cobj[tid] = head_act(obj_raw, h.new_coords);
             }
         }
-        if (threadIdx.x < kChunk) {
-            const unsigned bal = __ballot_sync(0xffffffffu, alive);
-            if ((threadIdx.x & 31) == 0) alive_words[threadIdx.x >> 5] = bal;
-            cpos[threadIdx.x] = -1;
+        __syncthreads();
+        // ---- against the survivors so far
+        bool hit = false;
+        if (slot < m) {
+            const int cls = ccls[slot];
+            const float4 b = cbox[slot];
+            for (int k = khead[cls % kBuckets]; k >= 0 && !hit; k = knext[k])
+                if ((k & 1) == half && kcls[k] == cls) hit = iou_above(kbox[k], b, p.nms_thr);
+        }
+        const unsigned bal = __ballot_sync(0xffffffffu, hit);
+        if (half == 0 && (tid & 31) == 0) out_words[slot >> 5] = bal;
+        __syncthreads();
+        if (half == 1 && (tid & 31) == 0) out_words[slot >> 5] |= bal;
+        __syncthreads();
+        const bool alive = tid < m && !((out_words[(tid & (kChunk - 1)) >> 5] >> (tid & 31)) & 1u);
+        if (alive) atomicOr(&cbits[(ccls[tid] % kBuckets) * W + (tid >> 5)], 1u << (tid & 31));
+        if (tid < kChunk) {
+            const unsigned ab = __ballot_sync(0xffffffffu, alive);
+            if ((tid & 31) == 0) alive_words[tid >> 5] = ab;
         }
         __syncthreads();
-        // ---- same-class IoU bitmask: bit j of row i set when j > i suppresses under i
-        for (int item = threadIdx.x; item < kChunk * (kChunk / 32); item += blockDim.x) {
-            const int i = item >> 4, wd = item & 15;
-            unsigned bitsv = 0;
-            if (i < m && ((alive_words[i >> 5] >> (i & 31)) & 1u) && (wd << 5) + 31 > i) {
-                const float4 bi4 = cbox[i];
-                Box bi; bi.x = bi4.x; bi.y = bi4.y; bi.w = bi4.z; bi.h = bi4.w;
+        // ---- suppressor rows: bit j of row i set when the earlier candidate j suppresses i if it is kept
+        for (int item = tid; item < kChunk * W; item += 1024) {
+            const int i = item / W, wd = item & (W - 1);
+            unsigned bitsv = 0u;
+            if (i < m && wd <= (i >> 5) && ((alive_words[i >> 5] >> (i & 31)) & 1u)) {
                 const int ci = ccls[i];
-                for (int jj = 0; jj < 32; ++jj) {
-                    const int j = (wd << 5) + jj;
-                    if (j <= i || j >= m || ccls[j] != ci) continue;
-                    const float4 bj4 = cbox[j];
-                    Box bj; bj.x = bj4.x; bj.y = bj4.y; bj.w = bj4.z; bj.h = bj4.w;
-                    if (box_iou(bi, bj) > p.nms_thr) bitsv |= 1u << jj;
+                unsigned cand = cbits[(ci % kBuckets) * W + wd];
+                if (wd == (i >> 5)) cand &= (1u << (i & 31)) - 1u;
+                if (cand) {
+                    const float4 bi = cbox[i];
+                    while (cand) {
+                        const int b = __ffs(cand) - 1, j = wd * 32 + b;
+                        cand &= cand - 1u;
+                        if (ccls[j] == ci && iou_above(cbox[j], bi, p.nms_thr)) bitsv |= 1u << b;
+                    }
+                    if (bitsv) atomicOr(&row_words[i], 1u << wd);
                 }
             }
             mask[item] = bitsv;
         }
         __syncthreads();
-        // ---- one warp resolves the chunk in order
-        if (threadIdx.x < 32) {
-            const int lane = threadIdx.x;
-            unsigned removed = lane < 16 ? ~alive_words[lane] : 0xFFFFFFFFu;
-            int kept_now = kept_before;
-            // the mask row of candidate i + 1 is fetched while candidate i is decided: the loop is a chain of dependent steps and
-            // the shared-memory latency would otherwise sit on it
-            unsigned row = lane < 16 ? mask[lane] : 0u;
-            for (int i = 0; i < m && kept_now < p.k_eff; ++i) {
-                const unsigned next = (lane < 16 && i + 1 < m) ? mask[(i + 1) * 16 + lane] : 0u;
-                const unsigned r = __shfl_sync(0xffffffffu, removed, i >> 5);
-                if (!((r >> (i & 31)) & 1u)) {
-                    removed |= row;
-                    if (lane == 0) cpos[i] = kept_now;
-                    ++kept_now;
+        // ---- resolve: facts only ever get added to kept_words / out_words, so reading them while others write is harmless
+        bool undecided = alive;
+        bool is_kept = false;
+        if (tid < W) out_words[tid] = ~alive_words[tid];
+        __syncthreads();
+        for (int round = 0; round < kChunk; ++round) {  // (every round decides at least the first undecided candidate)
+            bool k = false, o = false;
+            if (undecided) {
+                bool open = false;
+                for (unsigned ws = row_words[tid]; ws && !o; ws &= ws - 1u) {
+                    const int wd = __ffs(ws) - 1;
+                    const unsigned sup = mask[tid * W + wd];
+                    o = (sup & kept_words[wd]) != 0u;
+                    open = open || (sup & ~out_words[wd]) != 0u;
                 }
-                row = next;
+                k = !o && !open;
+                undecided = !(k || o);
+                is_kept = is_kept || k;
             }
-            if (lane == 0) s_kept = kept_now;
+            if (tid < kChunk) {
+                const unsigned kb = __ballot_sync(0xffffffffu, k), ob = __ballot_sync(0xffffffffu, o);
+                if ((tid & 31) == 0) {
+                    if (kb) kept_words[tid >> 5] |= kb;
+                    if (ob) out_words[tid >> 5] |= ob;
+                }
+            }
+            if (!__syncthreads_or(undecided ? 1 : 0)) break;
+        }
+        // ---- append the new survivors, in order, up to k_eff; their records leave through shared memory as one contiguous range
+        const int kept_before = kept;
+        int before = 0, total = 0;
+        for (int w = 0; w < W; ++w) {
+            const int c = __popc(kept_words[w]);
+            if (w < (tid >> 5)) before += c;
+            total += c;
+        }
+        kept = min(kept_before + total, p.k_eff);
+        float* stage = reinterpret_cast<float*>(mask);
+        if (is_kept) {
+            const int rank = before + __popc(kept_words[tid >> 5] & ((1u << (tid & 31)) - 1u)), pos = kept_before + rank;
+            if (pos < p.k_eff) {
+                const float4 b = cbox[tid];
+                const int cls = ccls[tid];
+                kbox[pos] = b;
+                kcls[pos] = cls;
+                knext[pos] = atomicExch(&khead[cls % kBuckets], pos);
+                kept_box[(size_t)img * p.k_eff + pos] = b;
+                kept_cls[(size_t)img * p.k_eff + pos] = cls;
+                float* d = stage + rank * 7;  // ln_detection
+                d[0] = (float)cls;
+                d[1] = key_conf((unsigned)(keys[base + tid] >> 32));
+                d[2] = cobj[tid];
+                d[3] = b.x; d[4] = b.y; d[5] = b.z; d[6] = b.w;
+            }
         }
         __syncthreads();
-        // ---- append the new survivors
-        if ((int)threadIdx.x < m && cpos[threadIdx.x] >= 0) {
-            const int pos = cpos[threadIdx.x];
-            kbox[pos] = cbox[threadIdx.x];
-            kcls[pos] = ccls[threadIdx.x];
-            kept_box[(size_t)img * p.k_eff + pos] = cbox[threadIdx.x];
-            kept_cls[(size_t)img * p.k_eff + pos] = ccls[threadIdx.x];
-            if (pos < p.max_per_image) {
-                const unsigned long long key = keys[base + threadIdx.x];
-                ln_detection d;
-                d.class_id = (float)ccls[threadIdx.x];
-                d.confidence = key_conf((unsigned)(key >> 32));
-                d.objectness = cobj[threadIdx.x];
-                const float4 b = cbox[threadIdx.x];
-                d.x = b.x; d.y = b.y; d.w = b.z; d.h = b.w;
-                records[(size_t)img * p.max_per_image + pos] = d;
-            }
-        }
+        float* dst = records + ((size_t)img * p.max_per_image + kept_before) * 7;
+        for (int i = tid; i < (kept - kept_before) * 7; i += 1024) dst[i] = stage[i];
         __syncthreads();
-        if (s_kept >= p.k_eff) break;
     }
-    if (threadIdx.x == 0) {
-        st.last_gain = s_kept - st.kept;
+    if (tid == 0) {
+        st.last_gain = kept - st.kept;
         st.band_count = n;
-        st.kept = s_kept;
+        st.kept = kept;
         st.hi = st.lo;
         band_fill[img] = 0;
         if (st.kept >= p.k_eff || (st.exhausted && st.pool_lo == 0ull)) st.phase = PHASE_DONE;
         else {
-            atomicAdd(&flags[FLAG_ACTIVE], 1);
             st.level = 0;
             if (st.exhausted) {  // the pool is used up: the next one starts below it
                 st.phase = PHASE_POOL;
                 st.prefix = 0;
                 st.above = 0;
-                atomicAdd(&flags[FLAG_NEED_POOL], 1);
             } else {
                 st.phase = PHASE_SELECT;
                 st.level = st.start_level;
@@ -890,25 +1018,25 @@ __global__ void __launch_bounds__(1024, 1) yolo_nms_kernel(const __grid_constant
             }
         }
         states[img] = st;
+        counts[img] = st.phase == PHASE_DONE ? min(kept, p.max_per_image) : -1 - st.phase;
     }
 }
 
-__global__ void yolo_init_states_kernel(ImgState* states, unsigned long long* key_and_or, const int* img_w, const int* img_h, int batch, int hist_stride) {
+// Starts every image: with `direct` by the fill pass over everything above the threshold, else by the histogram of a pool.
+__global__ void yolo_init_states_kernel(ImgState* states, unsigned long long* key_and_or, int* fills, const int* img_w, const int* img_h, int batch, int hist_stride,
+                                        int direct) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= batch) return;
     ImgState s;
     s.hi = ~0ull; s.lo = 0; s.prefix = 0; s.pool_lo = 0;
-    s.level = 0; s.phase = PHASE_POOL; s.cap = 0; s.above = 0; s.band_count = 0; s.kept = 0; s.exhausted = 0;
-    s.img_w = img_w[i]; s.img_h = img_h[i]; s.last_gain = -1; s.direct = 0; s.pool_count = 0; s.sampled = hist_stride > 1 ? 1 : 0;
+    s.level = 0; s.phase = direct ? PHASE_FILL : PHASE_POOL; s.cap = 0; s.above = 0; s.band_count = 0; s.kept = 0; s.exhausted = direct;
+    s.img_w = img_w[i]; s.img_h = img_h[i]; s.last_gain = -1; s.direct = direct; s.pool_count = 0; s.sampled = hist_stride > 1 ? 1 : 0;
     s.start_level = 0; s.fresh = 1; s.start_prefix = 0;
     states[i] = s;
+    fills[i] = 0;
+    fills[batch + i] = 0;
     key_and_or[2 * i] = ~0ull;
     key_and_or[2 * i + 1] = 0ull;
-}
-
-__global__ void yolo_counts_kernel(const ImgState* states, int* counts, int batch, int max_per_image) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < batch) counts[i] = states[i].kept < max_per_image ? states[i].kept : max_per_image;
 }
 
 // Largest distance between the approximate and the exact confidence key over a sweep of logits (debug aid that
@@ -1002,7 +1130,7 @@ int fill_params(ln_ctx* ctx, YoloParams* p, const ln_yolo_head* heads, int32_t n
 }
 
 struct Scratch {
-    size_t sz_states, sz_hist, sz_band, sz_fill, sz_kbox, sz_kcls, sz_rec, sz_dims, sz_cnt, sz_andor, sz_flags, sz_pool, total;
+    size_t sz_states, sz_hist, sz_band, sz_fill, sz_kbox, sz_kcls, sz_rec, sz_dims, sz_cnt, sz_andor, sz_pool, total;
 };
 
 // Sizes of the working arrays of one call.  pool_entries = 0 picks the pool size: every candidate of an image when that
@@ -1031,10 +1159,9 @@ void scratch_layout(YoloParams* p, int pool_entries, Scratch* s) {
     s->sz_dims = (size_t)ln_round_up(B * 8, 256);
     s->sz_cnt = (size_t)ln_round_up(B * 4, 256);
     s->sz_andor = (size_t)ln_round_up(B * 16, 256);
-    s->sz_flags = 256;
     s->sz_pool = (size_t)B * (size_t)pm * 8;
     s->total = s->sz_states + s->sz_hist + s->sz_band + s->sz_fill + s->sz_kbox + s->sz_kcls + s->sz_rec + s->sz_dims + s->sz_cnt + s->sz_andor +
-               s->sz_flags + s->sz_pool;
+               s->sz_pool;
 }
 
 int check_options(ln_ctx* ctx, YoloParams* p, const ln_detect_options* opts, const int32_t* image_w, const int32_t* image_h, int band_max, const char* who) {
@@ -1052,9 +1179,21 @@ int check_options(ln_ctx* ctx, YoloParams* p, const ln_detect_options* opts, con
     return LN_OK;
 }
 
+// Page-locked host memory of one call: image sizes in, outcome per image and records out.  Kernels read and write it directly.
+size_t stage_bytes(const YoloParams& p) { return (size_t)ln_round_up((int64_t)p.batch * 12, 128) + (size_t)p.batch * p.max_per_image * sizeof(ln_detection); }
+
+// Device address of page-locked host memory, or null for any other pointer.
+void* mapped_pointer(void* host) {
+    cudaPointerAttributes a;
+    const bool ok = cudaPointerGetAttributes(&a, host) == cudaSuccess && a.type == cudaMemoryTypeHost && a.devicePointer;
+    (void)cudaGetLastError();  // (an unregistered pointer is not an error here)
+    return ok ? a.devicePointer : nullptr;
+}
+
 // The whole decode + NMS call over working memory that the caller provides (s.total bytes at `scratch`, 256-byte aligned).
+// `stage`: stage_bytes(p) of page-locked memory, or null (sizes and results then go through device memory and copies).
 int run_decode_nms(ln_ctx* ctx, const YoloParams& p, const Scratch& s, unsigned char* scratch, const int32_t* image_w, const int32_t* image_h,
-                   ln_detection* records_host, int32_t* counts_host, const char* who, void* pinned_stage = nullptr) {
+                   ln_detection* records_host, int32_t* counts_host, const char* who, void* stage = nullptr) {
     const int B = p.batch;
     unsigned char* q = scratch;
     ImgState* states = (ImgState*)q; q += s.sz_states;
@@ -1063,11 +1202,10 @@ int run_decode_nms(ln_ctx* ctx, const YoloParams& p, const Scratch& s, unsigned 
     int* band_fill = (int*)q; int* pool_fill = band_fill + B; q += s.sz_fill;
     float4* kept_box = (float4*)q; q += s.sz_kbox;
     int* kept_cls = (int*)q; q += s.sz_kcls;
-    ln_detection* records = (ln_detection*)q; q += s.sz_rec;
+    float* records = (float*)q; q += s.sz_rec;
     int* dims = (int*)q; q += s.sz_dims;
     int* counts = (int*)q; q += s.sz_cnt;
     unsigned long long* key_and_or = (unsigned long long*)q; q += s.sz_andor;
-    int* flags = (int*)q; q += s.sz_flags;
     unsigned long long* pool = (unsigned long long*)q;
 #define LN_Y(call)                                                                                     \
     do {                                                                                               \
@@ -1077,100 +1215,105 @@ int run_decode_nms(ln_ctx* ctx, const YoloParams& p, const Scratch& s, unsigned 
     const bool dbg = getenv("LN_DEBUG_NMS") != nullptr;
     auto now = []() { timespec ts; clock_gettime(CLOCK_MONOTONIC, &ts); return ts.tv_sec * 1e3 + ts.tv_nsec * 1e-6; };
     const double t_begin = dbg ? now() : 0;
-    // the working memory keeps whatever an earlier call left: clear everything the kernels expect to start at zero
-    LN_Y(cudaMemsetAsync(hist, 0, s.sz_hist, ctx->stream));
-    LN_Y(cudaMemsetAsync(band_fill, 0, s.sz_fill, ctx->stream));
-    LN_Y(cudaMemsetAsync(flags, 0, s.sz_flags, ctx->stream));
-    LN_Y(cudaMemcpyAsync(dims, image_w, (size_t)B * 4, cudaMemcpyHostToDevice, ctx->stream));
-    LN_Y(cudaMemcpyAsync(dims + B, image_h, (size_t)B * 4, cudaMemcpyHostToDevice, ctx->stream));
-    yolo_init_states_kernel<<<(B + 127) / 128, 128, 0, ctx->stream>>>(states, key_and_or, dims, dims + B, B, p.hist_stride);
+    const int* outcome = counts_host;  // what the host reads after a round
+    float* stage_records = nullptr;    // records wait here for the copy into the caller's array
+    if (stage) {
+        int* st = (int*)stage;
+        memcpy(st, image_w, (size_t)B * 4);
+        memcpy(st + B, image_h, (size_t)B * 4);
+        dims = st;
+        counts = st + 2 * B;
+        outcome = counts;
+        // a caller that passes a page-locked record array gets its records written in place
+        if (void* m = mapped_pointer(records_host)) records = (float*)m;
+        else records = stage_records = (float*)((unsigned char*)stage + ln_round_up((int64_t)B * 12, 128));
+    } else {
+        LN_Y(cudaMemcpyAsync(dims, image_w, (size_t)B * 4, cudaMemcpyHostToDevice, ctx->stream));
+        LN_Y(cudaMemcpyAsync(dims + B, image_h, (size_t)B * 4, cudaMemcpyHostToDevice, ctx->stream));
+    }
+    const bool direct = p.thr >= kDirectThr;
+    yolo_init_states_kernel<<<(B + 127) / 128, 128, 0, ctx->stream>>>(states, key_and_or, band_fill, dims, dims + B, B, p.hist_stride, direct ? 1 : 0);
     ctx->launches++;
 
-    const size_t nms_smem = (size_t)p.band_max * 8 + (size_t)(p.k_eff + kChunk) * sizeof(float4) + (size_t)kChunk * (kChunk / 32) * 4 +
-                            (size_t)(p.k_eff + kChunk) * 4 + (size_t)kChunk * 8 + 64;
+    const size_t nms_smem = nms_smem_bytes(p.band_max, p.k_eff);
     LN_Y(cudaFuncSetAttribute(yolo_nms_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nms_smem));
     const dim3 scan_grid((p.total_ca + 255) / 256, B);
     const dim3 pool_grid((unsigned)((p.pool_max + kPoolChunk - 1) / kPoolChunk), B);
-    int* h_flags = ctx->h_status + 4;  // 4 ints
-    const int max_rounds = 4096;
+    const int max_rounds = 1 << 16;
     // with LN_DEBUG_NMS set, every kernel is followed by a synchronize and its wall time is added to its class
     double t_k[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     double t_mark = 0;
     auto tick = [&]() { if (dbg) { cudaStreamSynchronize(ctx->stream); t_mark = now(); } };
     auto tock = [&](int k) { if (dbg) { cudaStreamSynchronize(ctx->stream); t_k[k] += now() - t_mark; } };
     int n_full = 0, n_pool_passes = 0, round = 0;
-    bool need_pool = true;
+    bool need_pool = !direct, hist_clear = false;
     for (; round < max_rounds; ++round) {
-        // selection: pools for the images that need one, then a band inside every pool; repeated while some image descends a digit
-        for (int step = 0; step < 2 * kLevels + 2; ++step) {
+        if (direct && round == 0) {
+            tick();
+            yolo_head_fill_kernel<<<scan_grid, 256, 0, ctx->stream>>>(p, states, band, band_fill, pool, pool_fill, key_and_or);
+            tock(2);
+            ctx->launches++;
+            n_full++;
+        } else {
+            // selection: pools for the images that need one, then a band inside every pool (one digit per round; an image that has to
+            // descend another digit sits out the rest of the round)
+            if (!hist_clear) {  // (the selections leave the histograms zeroed)
+                LN_Y(cudaMemsetAsync(hist, 0, s.sz_hist, ctx->stream));
+                hist_clear = true;
+            }
             if (need_pool) {
+                if (round > 0) LN_Y(cudaMemsetAsync(pool_fill, 0, (size_t)B * 4, ctx->stream));
                 tick();
                 yolo_head_hist_kernel<<<scan_grid, 256, 0, ctx->stream>>>(p, states, hist);
                 tock(0); tick();
-                yolo_pool_select_kernel<<<B, 256, 0, ctx->stream>>>(p, states, hist, flags);
+                yolo_pool_select_kernel<<<B, 256, 0, ctx->stream>>>(p, states, hist);
                 tock(1); tick();
                 yolo_head_fill_kernel<<<scan_grid, 256, 0, ctx->stream>>>(p, states, band, band_fill, pool, pool_fill, key_and_or);
                 tock(2);
-                yolo_after_fill_kernel<<<(B + 127) / 128, 128, 0, ctx->stream>>>(states, band_fill, pool_fill, B, p.band_max, p.pool_max, p.hist_stride, flags, key_and_or);
+                yolo_after_fill_kernel<<<(B + 127) / 128, 128, 0, ctx->stream>>>(states, band_fill, pool_fill, B, p.band_max, p.pool_max, p.hist_stride, key_and_or);
                 ctx->launches += 4;
                 n_full += 2;
             }
             tick();
             yolo_pool_scan_kernel<0><<<pool_grid, 256, 0, ctx->stream>>>(p, states, hist, key_and_or, band, band_fill, pool);
             tock(3); tick();
-            yolo_select_kernel<<<B, 256, 0, ctx->stream>>>(p, states, hist, key_and_or, flags);
-            tock(4);
-            ctx->launches += 2;
+            yolo_select_kernel<<<B, 256, 0, ctx->stream>>>(p, states, hist, key_and_or);
+            tock(4); tick();
+            yolo_pool_scan_kernel<1><<<pool_grid, 256, 0, ctx->stream>>>(p, states, hist, key_and_or, band, band_fill, pool);
+            tock(5);
+            ctx->launches += 3;
             ++n_pool_passes;
-            LN_Y(cudaMemcpyAsync(h_flags, flags, 16, cudaMemcpyDeviceToHost, ctx->stream));
-            LN_Y(cudaMemsetAsync(flags, 0, 16, ctx->stream));
-            LN_Y(cudaStreamSynchronize(ctx->stream));
-            need_pool = h_flags[FLAG_POOL_PENDING] != 0;
-            if (!need_pool && h_flags[FLAG_SELECT_PENDING] == 0) break;
         }
         tick();
-        yolo_pool_scan_kernel<1><<<pool_grid, 256, 0, ctx->stream>>>(p, states, hist, key_and_or, band, band_fill, pool);
-        tock(5); tick();
-        yolo_nms_kernel<<<B, 1024, nms_smem, ctx->stream>>>(p, states, band, band_fill, kept_box, kept_cls, records, flags);
+        yolo_nms_kernel<<<B, 1024, nms_smem, ctx->stream>>>(p, states, band, band_fill, kept_box, kept_cls, records, counts);
         tock(6);
-        ctx->launches += 2;
-        LN_Y(cudaMemcpyAsync(h_flags, flags, 16, cudaMemcpyDeviceToHost, ctx->stream));
-        LN_Y(cudaMemsetAsync(flags, 0, 16, ctx->stream));
-        LN_Y(cudaMemsetAsync(pool_fill, 0, (size_t)B * 4, ctx->stream));
+        ctx->launches++;
+        LN_Y(cudaGetLastError());
+        if (!stage) LN_Y(cudaMemcpyAsync(counts_host, counts, (size_t)B * 4, cudaMemcpyDeviceToHost, ctx->stream));
         LN_Y(cudaStreamSynchronize(ctx->stream));
-        if (h_flags[FLAG_ACTIVE] == 0) break;
-        need_pool = need_pool || h_flags[FLAG_NEED_POOL] != 0;
+        bool active = false;
+        need_pool = false;
+        for (int i = 0; i < B; ++i) {
+            active = active || outcome[i] < 0;
+            need_pool = need_pool || outcome[i] == -1 - PHASE_POOL;
+        }
+        if (!active) break;
     }
     const double t_loop = dbg ? now() : 0;
     if (dbg) fprintf(stderr, "[ln_yolo] batch %d: %d rounds, %d passes over the heads, %d pool passes; ms: head histogram %.3f, pool select %.3f, head fill %.3f, "
                      "pool histogram %.3f, band select %.3f, band collect %.3f, sort + nms %.3f; band_max %d, pool_max %d, k_eff %d\n",
                      B, round + 1, n_full, n_pool_passes, t_k[0], t_k[1], t_k[2], t_k[3], t_k[4], t_k[5], t_k[6], p.band_max, p.pool_max, p.k_eff);
     if (round == max_rounds) return ln_fail(ctx, LN_ERR_TIMEOUT, "%s: NMS did not finish in %d rounds", who, max_rounds);
-    yolo_counts_kernel<<<(B + 127) / 128, 128, 0, ctx->stream>>>(states, counts, B, p.max_per_image);
-    ctx->launches++;
-    LN_Y(cudaGetLastError());
-    const size_t rec_bytes = (size_t)B * p.max_per_image * sizeof(ln_detection);
-    // a caller that passes page-locked buffers gets its records by DMA, without the staging copy below
-    if (pinned_stage) {
-        cudaPointerAttributes pa_r, pa_c;
-        if (cudaPointerGetAttributes(&pa_r, records_host) == cudaSuccess && cudaPointerGetAttributes(&pa_c, counts_host) == cudaSuccess &&
-            pa_r.type == cudaMemoryTypeHost && pa_c.type == cudaMemoryTypeHost)
-            pinned_stage = nullptr;
-        (void)cudaGetLastError();  // (an unregistered pointer is not an error here)
-    }
-    if (pinned_stage) {
-        // through pinned memory: the copy runs at link speed instead of being staged page by page by the driver
-        LN_Y(cudaMemcpyAsync(pinned_stage, records, rec_bytes, cudaMemcpyDeviceToHost, ctx->stream));
-        LN_Y(cudaMemcpyAsync((unsigned char*)pinned_stage + rec_bytes, counts, (size_t)B * 4, cudaMemcpyDeviceToHost, ctx->stream));
-        LN_Y(cudaStreamSynchronize(ctx->stream));
-        memcpy(records_host, pinned_stage, rec_bytes);
-        memcpy(counts_host, (unsigned char*)pinned_stage + rec_bytes, (size_t)B * 4);
+    if (stage) {
+        memcpy(counts_host, counts, (size_t)B * 4);
+        if (stage_records)
+            for (int i = 0; i < B; ++i)
+                memcpy(records_host + (size_t)i * p.max_per_image, stage_records + (size_t)i * p.max_per_image * 7, (size_t)counts_host[i] * sizeof(ln_detection));
     } else {
-        LN_Y(cudaMemcpyAsync(counts_host, counts, (size_t)B * 4, cudaMemcpyDeviceToHost, ctx->stream));
-        LN_Y(cudaMemcpyAsync(records_host, records, rec_bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        LN_Y(cudaMemcpyAsync(records_host, records, (size_t)B * p.max_per_image * sizeof(ln_detection), cudaMemcpyDeviceToHost, ctx->stream));
         LN_Y(cudaStreamSynchronize(ctx->stream));
     }
-    if (dbg) fprintf(stderr, "[ln_yolo] whole call %.3f ms, of which the read-back of counts and records %.3f ms\n", now() - t_begin, now() - t_loop);
+    if (dbg) fprintf(stderr, "[ln_yolo] whole call %.3f ms, of which handing over counts and records %.3f ms\n", now() - t_begin, now() - t_loop);
 #undef LN_Y
     return LN_OK;
 }
@@ -1194,12 +1337,12 @@ int32_t ln_yolo_decode_nms(ln_ctx* ctx, const ln_yolo_head* heads, int32_t n_hea
     cudaSetDevice(ctx->device);
     unsigned char* scratch = (unsigned char*)ln_pool_alloc(ctx, s.total);
     if (!scratch) return LN_ERR_CUDA;
-    const size_t stage_bytes = (size_t)p.batch * p.max_per_image * sizeof(ln_detection) + (size_t)p.batch * 4;
-    if (ctx->h_stage_bytes < stage_bytes) {
+    const size_t need = stage_bytes(p);
+    if (ctx->h_stage_bytes < need) {
         if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
         ctx->h_stage = nullptr;
         ctx->h_stage_bytes = 0;
-        if (cudaMallocHost(&ctx->h_stage, stage_bytes) == cudaSuccess) ctx->h_stage_bytes = stage_bytes;
+        if (cudaMallocHost(&ctx->h_stage, need) == cudaSuccess) ctx->h_stage_bytes = need;
         else { ctx->h_stage = nullptr; cudaGetLastError(); }  // no pinned memory to be had: read back directly
     }
     rc = run_decode_nms(ctx, p, s, scratch, image_w, image_h, records_host, counts_host, who, ctx->h_stage);
