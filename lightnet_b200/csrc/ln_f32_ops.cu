@@ -1,7 +1,7 @@
 // f32 NCHW operators: the F32TensorOpsBackend subset on the detector path
-// (lightnet-cuda/src/lib.rs:460).  Plain CUDA-core kernels: this path exists for
-// trait fidelity, for calibration and as the f32 parity target; the throughput path
-// is the 8-bit one.
+// (lightnet-cuda/src/lib.rs:460).  CUDA-core kernels in binary32 throughout (no
+// reduced-precision tensor-core formats): this path exists for trait fidelity, for
+// calibration and as the f32 parity target; the throughput path is the 8-bit one.
 #include "ln_common.h"
 
 namespace {
@@ -9,9 +9,198 @@ namespace {
 constexpr int kThreads = 256;
 inline int blocks_for(int64_t n, int per_block = kThreads) { return (int)((n + per_block - 1) / per_block); }
 
-// Direct convolution, one thread per (pixel, group of FPT filters).  Semantics of
-// runtime/forward_layers.rs:646-695: taps outside the image are skipped, groups partition
-// channels, weights are [filters][C/groups][k][k].
+// Convolution as a blocked GEMM: y[f][pixel] = sum over k = (channel, ky, kx) of w[f][k] * x[tap k of pixel].  What bounds it is the
+// FMA rate (2 operations per weight-pixel pair against 4 bytes of either), so a thread keeps 8 filters x 8 pixels in registers and
+// every value it reads from shared memory serves eight of them; the products are formed two pixels at a time with packed
+// f32x2 FMAs, whose weight operand is stored twice in shared memory so that no instruction is spent on duplicating it.  The k
+// range advances in slices of 8, the next slice on its way from global memory into registers while the current one is multiplied.
+// Each output is one chain of fused multiply-adds in k order, the order of runtime/forward_layers.rs:646-695; only a split k range
+// (few tiles) sums the chains of its parts at the end.
+// BM filters x BN pixels per CTA.  KS: kernel size when it is 1 or 3, 0 = any.  Taps outside the image contribute 0.
+// (YOLOv4 608 x 608, batch 1: 69.4 ms with one thread per (pixel, 4 filters) reading both operands from L1.)
+constexpr int kSlice = 8;
+struct ConvF32 {
+    const float* x;
+    const float* w;
+    const float* bias;  // null = none
+    float* y;
+    int B, C, H, W, F, k, sx, sy, dil, pad, OH, OW, K, act;
+    int k_part;       // k range of one part (blockIdx.z), a multiple of kSlice
+    int64_t part_elems;  // > 0: part z writes raw sums to y + z * part_elems
+};
+
+__device__ __forceinline__ unsigned long long fma2_f32(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+template <int BM, int BN, int KS>
+__global__ void __launch_bounds__(BM * BN / 64, 32768 / (BM * BN)) conv2d_f32_gemm_kernel(const __grid_constant__ ConvF32 p) {
+    constexpr int T = BM * BN / 64, TX = BN / 8;
+    constexpr int PIX = BN > T ? BN / T : 1;      // pixels a thread gathers
+    constexpr int RSTEP = T > BN ? T / BN : 1;    // k rows gathered side by side
+    constexpr int ROWS = kSlice / RSTEP;          // k rows per thread and pixel
+    constexpr int WV = BM * 2 / T;                // groups of four weights per thread
+    __shared__ __align__(16) float2 s_w[2][kSlice][BM];
+    __shared__ __align__(16) float s_x[2][kSlice][BN];
+    const int tid = (int)threadIdx.x, tx = tid % TX, ty = tid / TX;
+    const int P = p.OH * p.OW, HW = p.H * p.W, NP = p.B * P;
+    const int n0 = (int)blockIdx.x * BN, f0 = (int)blockIdx.y * BM;
+    const int k_begin = (int)blockIdx.z * p.k_part, k_end = min(p.K, k_begin + p.k_part);
+    const int kk = KS ? KS * KS : p.k * p.k;
+    // the pixels this thread gathers: address of tap (0, 0) and which taps are inside the image (kernels up to 8 x 8; larger ones test)
+    const float* px[PIX];
+    unsigned long long inside[PIX];
+    int oy0[PIX], ox0[PIX];
+#pragma unroll
+    for (int j = 0; j < PIX; ++j) {
+        const int n = n0 + (tid % BN) + j * T;
+        const int b = n / P, r = n - b * P, oy = r / p.OW, ox = r - oy * p.OW;
+        oy0[j] = n < NP ? oy * p.sy - p.pad : -(1 << 28);
+        ox0[j] = ox * p.sx - p.pad;
+        px[j] = p.x + (int64_t)(n < NP ? b : 0) * p.C * HW + (int64_t)(n < NP ? oy0[j] : 0) * p.W + ox0[j];
+        inside[j] = 0ull;
+        const int ks = KS ? KS : p.k;
+        if (ks <= 8)
+            for (int t = 0; t < ks * ks; ++t) {
+                const int iy = oy0[j] + (t / ks) * p.dil, ix = ox0[j] + (t % ks) * p.dil;
+                if (iy >= 0 && iy < p.H && ix >= 0 && ix < p.W) inside[j] |= 1ull << t;
+            }
+    }
+    const int row0 = T > BN ? tid / BN : 0;
+    float gx[ROWS][PIX];
+    float4 gw[WV];
+    const bool w_vec = (p.K & 3) == 0 && (((uintptr_t)p.w) & 15) == 0;
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+            const int kr = k0 + row0 + i * RSTEP;
+            const int c = kr / kk, tap = kr - c * kk;
+            const int ks = KS ? KS : p.k;
+            const int ky = KS == 1 ? 0 : tap / ks, kx = KS == 1 ? 0 : tap - ky * ks;
+            const int64_t off = (int64_t)c * HW + (int64_t)(ky * p.dil) * p.W + kx * p.dil;
+#pragma unroll
+            for (int j = 0; j < PIX; ++j) {
+                bool ok = kr < k_end;
+                if (KS != 0 || p.k <= 8) ok = ok && ((inside[j] >> tap) & 1ull);
+                else {
+                    const int iy = oy0[j] + ky * p.dil, ix = ox0[j] + kx * p.dil;
+                    ok = ok && iy >= 0 && iy < p.H && ix >= 0 && ix < p.W;
+                }
+                gx[i][j] = ok ? __ldg(px[j] + off) : 0.0f;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < WV; ++i) {
+            const int v = tid + i * T, f = f0 + (v >> 1), kr = k0 + (v & 1) * 4;
+            float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (f < p.F) {
+                const float* wp = p.w + (int64_t)f * p.K + kr;
+                if (w_vec && kr + 4 <= k_end) q = __ldg(reinterpret_cast<const float4*>(wp));
+                else {
+                    if (kr < k_end) q.x = __ldg(wp);
+                    if (kr + 1 < k_end) q.y = __ldg(wp + 1);
+                    if (kr + 2 < k_end) q.z = __ldg(wp + 2);
+                    if (kr + 3 < k_end) q.w = __ldg(wp + 3);
+                }
+            }
+            gw[i] = q;
+        }
+    };
+    auto store = [&](int buf) {
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+            for (int j = 0; j < PIX; ++j) s_x[buf][row0 + i * RSTEP][(tid % BN) + j * T] = gx[i][j];
+#pragma unroll
+        for (int i = 0; i < WV; ++i) {
+            const int v = tid + i * T, m = v >> 1, r = (v & 1) * 4;
+            s_w[buf][r][m] = make_float2(gw[i].x, gw[i].x);
+            s_w[buf][r + 1][m] = make_float2(gw[i].y, gw[i].y);
+            s_w[buf][r + 2][m] = make_float2(gw[i].z, gw[i].z);
+            s_w[buf][r + 3][m] = make_float2(gw[i].w, gw[i].w);
+        }
+    };
+    unsigned long long acc[8][4];
+#pragma unroll
+    for (int m = 0; m < 8; ++m)
+#pragma unroll
+        for (int n = 0; n < 4; ++n) acc[m][n] = 0ull;
+    fetch(k_begin);
+    store(0);
+    __syncthreads();
+    int buf = 0;
+    for (int k0 = k_begin; k0 < k_end; k0 += kSlice) {
+        const bool more = k0 + kSlice < k_end;
+        if (more) fetch(k0 + kSlice);
+#pragma unroll
+        for (int r = 0; r < kSlice; ++r) {
+            const ulonglong2 xa = *reinterpret_cast<const ulonglong2*>(&s_x[buf][r][tx * 4]), xb = *reinterpret_cast<const ulonglong2*>(&s_x[buf][r][BN / 2 + tx * 4]);
+#pragma unroll
+            for (int m = 0; m < 8; m += 2) {
+                const ulonglong2 w2 = *reinterpret_cast<const ulonglong2*>(&s_w[buf][r][ty * 8 + m]);
+                acc[m][0] = fma2_f32(w2.x, xa.x, acc[m][0]);
+                acc[m][1] = fma2_f32(w2.x, xa.y, acc[m][1]);
+                acc[m][2] = fma2_f32(w2.x, xb.x, acc[m][2]);
+                acc[m][3] = fma2_f32(w2.x, xb.y, acc[m][3]);
+                acc[m + 1][0] = fma2_f32(w2.y, xa.x, acc[m + 1][0]);
+                acc[m + 1][1] = fma2_f32(w2.y, xa.y, acc[m + 1][1]);
+                acc[m + 1][2] = fma2_f32(w2.y, xb.x, acc[m + 1][2]);
+                acc[m + 1][3] = fma2_f32(w2.y, xb.y, acc[m + 1][3]);
+            }
+        }
+        if (more) store(buf ^ 1);
+        __syncthreads();
+        buf ^= 1;
+    }
+    const bool part = p.part_elems > 0;
+    float* y = p.y + (part ? (int64_t)blockIdx.z * p.part_elems : 0);
+    const bool vec = (P & 3) == 0;  // four consecutive pixels lie in one image then, at a 16-byte boundary
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int n = n0 + h * (BN / 2) + tx * 4;
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            const int f = f0 + ty * 8 + m;
+            if (f >= p.F || n >= NP) continue;
+            float v[4];
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(acc[m][2 * h]));
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(v[2]), "=f"(v[3]) : "l"(acc[m][2 * h + 1]));
+            if (!part) {
+                const float bias = p.bias ? __ldg(p.bias + f) : 0.0f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[j] = ln_act_f32(p.act, p.bias ? v[j] + bias : v[j]);
+            }
+            if (vec) {
+                const int b = n / P;
+                *reinterpret_cast<float4*>(y + ((int64_t)b * p.F + f) * P + (n - b * P)) = make_float4(v[0], v[1], v[2], v[3]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (n + j < NP) {
+                        const int b = (n + j) / P;
+                        y[((int64_t)b * p.F + f) * P + (n + j - b * P)] = v[j];
+                    }
+            }
+        }
+    }
+}
+
+// Adds the parts of a split k range in order, then bias and activation.  blockIdx.y = (image, filter) plane.
+__global__ void conv2d_f32_sum_parts_kernel(const float* __restrict__ parts, int n_parts, int64_t part_elems, const float* __restrict__ bias, float* __restrict__ y, int F,
+                                            int P, int act) {
+    const int64_t plane = (int64_t)blockIdx.y * P;
+    const float b = bias ? __ldg(bias + (int)(blockIdx.y % (unsigned)F)) : 0.0f;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P; i += gridDim.x * blockDim.x) {
+        float v = 0.0f;
+        for (int s = 0; s < n_parts; ++s) v += parts[(int64_t)s * part_elems + plane + i];
+        y[plane + i] = ln_act_f32(act, bias ? v + b : v);
+    }
+}
+
+// Grouped convolutions: one thread per (pixel, group of FPT filters).  Semantics of runtime/forward_layers.rs:646-695: taps outside
+// the image are skipped, groups partition channels, weights are [filters][C/groups][k][k].
 template <int FPT>
 __global__ void conv2d_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y, int B, int C,
                                   int H, int W, int F, int k, int sx, int sy, int dil, int pad, int groups, int OH, int OW) {
@@ -72,7 +261,7 @@ __global__ void conv2d_f32_kernel(const float* __restrict__ x, const float* __re
 }
 
 // bias_add / activation / bias_activation: channel = (i / channel_stride) % channels (lightnet-kernels-shared/src/lib.rs:10-40)
-__global__ void bias_act_f32_kernel(const float* __restrict__ x, const float* __restrict__ bias, float* __restrict__ y, int64_t n,
+__global__ void bias_act_f32_kernel(const float* x, const float* __restrict__ bias, float* y, int64_t n,
                                     int64_t channels, int64_t channel_stride, int act) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         float v = x[i];
@@ -268,6 +457,58 @@ int grid_for(ln_ctx* ctx, int64_t n) {
 
 bool is_f32(const ln_tensor* t) { return t && t->dtype == LN_F32; }
 
+template <int BM, int BN>
+void launch_conv_f32(const ConvF32& p, dim3 grid, cudaStream_t stream) {
+    if (p.k == 1) conv2d_f32_gemm_kernel<BM, BN, 1><<<grid, BM * BN / 64, 0, stream>>>(p);
+    else if (p.k == 3) conv2d_f32_gemm_kernel<BM, BN, 3><<<grid, BM * BN / 64, 0, stream>>>(p);
+    else conv2d_f32_gemm_kernel<BM, BN, 0><<<grid, BM * BN / 64, 0, stream>>>(p);
+}
+
+// Ungrouped convolution with optional bias and activation.  Tile: 128 x 128 while that gives every SM two CTAs; narrow layers take the
+// narrowest tile that covers their filters; everything smaller takes 64 x 64, and the k range is split until there are about
+// eight CTAs (of 64 threads) per SM, in parts of at least 64 (a part costs a pass over the output).
+int conv_f32_run(ln_ctx* ctx, ConvF32 p, const char* who) {
+    const int64_t NP = (int64_t)p.B * p.OH * p.OW, planes = (int64_t)p.B * p.F;
+    auto tiles = [&](int bm, int bn) { return ((NP + bn - 1) / bn) * ((p.F + bm - 1) / bm); };
+    int bm = 64, bn = 64;
+    if (p.F <= 32 && tiles(32, 128) >= 4 * ctx->sm_count) { bm = 32; bn = 128; }
+    else if (p.F <= 64 && tiles(64, 128) >= 4 * ctx->sm_count) { bm = 64; bn = 128; }
+    else if (p.F > 64 && tiles(128, 128) >= 2 * ctx->sm_count) { bm = 128; bn = 128; }
+    int parts = 1;
+    if (bm == 64 && bn == 64) {
+        const int64_t want = (8ll * ctx->sm_count + tiles(64, 64) - 1) / tiles(64, 64);
+        parts = (int)(want < p.K / 64 ? want : p.K / 64);
+        if (parts > 32) parts = 32;
+        if (parts < 1 || planes > 65535) parts = 1;
+    }
+    p.k_part = (int)ln_round_up((p.K + parts - 1) / parts, kSlice);
+    parts = (p.K + p.k_part - 1) / p.k_part;
+    const dim3 grid((unsigned)((NP + bn - 1) / bn), (unsigned)((p.F + bm - 1) / bm), (unsigned)parts);
+    float* y = p.y;
+    void* ws = nullptr;
+    size_t ws_bytes = 0;
+    if (parts > 1) {
+        p.part_elems = planes * p.OH * p.OW;
+        ws_bytes = (size_t)parts * p.part_elems * 4;
+        ws = ln_pool_alloc(ctx, ws_bytes);
+        if (!ws) return LN_ERR_CUDA;
+        p.y = (float*)ws;
+    }
+    if (bm == 128) launch_conv_f32<128, 128>(p, grid, ctx->stream);
+    else if (bm == 32) launch_conv_f32<32, 128>(p, grid, ctx->stream);
+    else if (bn == 128) launch_conv_f32<64, 128>(p, grid, ctx->stream);
+    else launch_conv_f32<64, 64>(p, grid, ctx->stream);
+    ctx->launches++;
+    if (ws) {
+        const int P = p.OH * p.OW, t = P < 128 ? 64 : (P < 512 ? 128 : 256);
+        conv2d_f32_sum_parts_kernel<<<dim3((unsigned)((P + t - 1) / t), (unsigned)planes), t, 0, ctx->stream>>>(p.y, parts, p.part_elems, p.bias, y, p.F, P, p.act);
+        ctx->launches++;
+        ln_pool_free(ctx, ws, ws_bytes);
+    }
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? LN_OK : ln_fail(ctx, LN_ERR_CUDA, "%s launch: %s", who, cudaGetErrorString(e));
+}
+
 }  // namespace
 
 extern "C" {
@@ -275,6 +516,16 @@ extern "C" {
 int32_t ln_conv2d_f32(ln_ctx* ctx, const ln_tensor* x, const ln_tensor* weights, const int64_t output_shape[4],
                       int64_t input_channels, int64_t input_height, int64_t input_width, int64_t filters, int64_t kernel_size,
                       int64_t stride_x, int64_t stride_y, int64_t dilation, int64_t padding, int64_t groups, ln_tensor** out) {
+    return ln_conv2d_bias_act_f32(ctx, x, weights, nullptr, output_shape, input_channels, input_height, input_width, filters, kernel_size, stride_x, stride_y, dilation,
+                                  padding, groups, LN_ACT_LINEAR, out);
+}
+
+}  // extern "C"
+
+// conv2d_f32 followed by bias_activation_f32 (bias may be null) without the pass over memory between them
+int ln_conv2d_bias_act_f32(ln_ctx* ctx, const ln_tensor* x, const ln_tensor* weights, const ln_tensor* bias, const int64_t output_shape[4], int64_t input_channels,
+                           int64_t input_height, int64_t input_width, int64_t filters, int64_t kernel_size, int64_t stride_x, int64_t stride_y, int64_t dilation,
+                           int64_t padding, int64_t groups, int activation, ln_tensor** out) {
     if (!ctx || !out || !output_shape) return ln_fail(ctx, LN_ERR_ARG, "ln_conv2d_f32: NULL argument");
     if (!is_f32(x) || !is_f32(weights)) return ln_fail(ctx, LN_ERR_ARG, "ln_conv2d_f32: f32 tensors required");
     if (groups < 1 || filters % groups || input_channels % groups || kernel_size < 1 || stride_x < 1 || stride_y < 1 || dilation < 1)
@@ -297,17 +548,36 @@ int32_t ln_conv2d_f32(ln_ctx* ctx, const ln_tensor* x, const ln_tensor* weights,
     cudaSetDevice(ctx->device);
     ln_tensor* y = ln_tensor_new(ctx, LN_F32, x->n, filters, oh, ow);
     if (!y) return LN_ERR_CUDA;
-    int64_t total = x->n * ((filters + 3) / 4) * oh * ow;
-    conv2d_f32_kernel<4><<<grid_for(ctx, total), kThreads, 0, ctx->stream>>>(
-        (const float*)x->ptr, (const float*)weights->ptr, (float*)y->ptr, (int)x->n, (int)input_channels, (int)input_height,
-        (int)input_width, (int)filters, (int)kernel_size, (int)stride_x, (int)stride_y, (int)dilation, (int)padding, (int)groups,
-        (int)oh, (int)ow);
-    ctx->launches++;
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) { ln_tensor_release(y); return ln_fail(ctx, LN_ERR_CUDA, "conv2d_f32 launch: %s", cudaGetErrorString(e)); }
+    const float* b = bias ? (const float*)bias->ptr : nullptr;
+    int rc = LN_OK;
+    if (groups == 1 && x->n * oh * ow < (1ll << 30) && x->count() < (1ll << 40)) {
+        ConvF32 p = {};
+        p.x = (const float*)x->ptr; p.w = (const float*)weights->ptr; p.bias = b; p.y = (float*)y->ptr;
+        p.B = (int)x->n; p.C = (int)input_channels; p.H = (int)input_height; p.W = (int)input_width; p.F = (int)filters; p.k = (int)kernel_size;
+        p.sx = (int)stride_x; p.sy = (int)stride_y; p.dil = (int)dilation; p.pad = (int)padding; p.OH = (int)oh; p.OW = (int)ow;
+        p.K = (int)(input_channels * kernel_size * kernel_size);
+        p.act = activation;
+        rc = conv_f32_run(ctx, p, "conv2d_f32");
+    } else {
+        int64_t total = x->n * ((filters + 3) / 4) * oh * ow;
+        conv2d_f32_kernel<4><<<grid_for(ctx, total), kThreads, 0, ctx->stream>>>(
+            (const float*)x->ptr, (const float*)weights->ptr, (float*)y->ptr, (int)x->n, (int)input_channels, (int)input_height,
+            (int)input_width, (int)filters, (int)kernel_size, (int)stride_x, (int)stride_y, (int)dilation, (int)padding, (int)groups,
+            (int)oh, (int)ow);
+        ctx->launches++;
+        if (b || activation != LN_ACT_LINEAR) {
+            bias_act_f32_kernel<<<grid_for(ctx, y->count()), kThreads, 0, ctx->stream>>>((const float*)y->ptr, b, (float*)y->ptr, y->count(), filters, oh * ow, activation);
+            ctx->launches++;
+        }
+        cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) rc = ln_fail(ctx, LN_ERR_CUDA, "conv2d_f32 launch: %s", cudaGetErrorString(e));
+    }
+    if (rc) { ln_tensor_release(y); return rc; }
     *out = y;
     return LN_OK;
 }
+
+extern "C" {
 
 static int32_t bias_act_impl(ln_ctx* ctx, const ln_tensor* x, const ln_tensor* bias, int64_t channels, int64_t channel_stride,
                              int32_t activation, ln_tensor** out, const char* who) {

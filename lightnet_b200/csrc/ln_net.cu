@@ -471,11 +471,8 @@ int forward_f32(ln_net* net, const ln_tensor* input, unsigned* amax_dev) {
         int rc = LN_OK;
         switch (L.kind) {
             case K_CONV: {  // layers/convolutional/gpu.rs:138-209: conv2d_f32_with_precision + bias_activation_f32
-                ln_tensor* conv = nullptr;
-                rc = ln_conv2d_f32(ctx, x, L.w_f32, oshape, L.in.c, L.in.h, L.in.w, L.filters, L.size, L.stride_x, L.stride_y, L.dilation, L.padding,
-                                   L.groups, &conv);
-                if (rc == LN_OK) rc = ln_bias_activation_f32(ctx, conv, L.b_f32, L.filters, (int64_t)L.out.h * L.out.w, L.act, &y);
-                ln_tensor_release(conv);
+                rc = ln_conv2d_bias_act_f32(ctx, x, L.w_f32, L.b_f32, oshape, L.in.c, L.in.h, L.in.w, L.filters, L.size, L.stride_x, L.stride_y, L.dilation, L.padding,
+                                            L.groups, L.act, &y);
                 break;
             }
             case K_MAXPOOL:  // layers/pool/gpu.rs:13-42
@@ -514,6 +511,7 @@ int forward_f32(ln_net* net, const ln_tensor* input, unsigned* amax_dev) {
                     ln_tensor_release(acc);
                     acc = sum;
                 }
+                if (rc == LN_OK && L.act == LN_ACT_LINEAR) { y = acc; break; }
                 if (rc == LN_OK) rc = ln_activation_f32(ctx, acc, L.act, &y);
                 ln_tensor_release(acc);
                 break;
