@@ -2,31 +2,28 @@
 // (lightnet-cuda/src/lib.rs:460).  CUDA-core kernels in binary32 throughout (no
 // reduced-precision tensor-core formats): this path exists for trait fidelity, for
 // calibration and as the f32 parity target; the throughput path is the 8-bit one.
+#include <cooperative_groups.h>
+
 #include "ln_common.h"
+
+namespace cg = cooperative_groups;
 
 namespace {
 
 constexpr int kThreads = 256;
 inline int blocks_for(int64_t n, int per_block = kThreads) { return (int)((n + per_block - 1) / per_block); }
 
-// Convolution as a blocked GEMM: y[f][pixel] = sum over k = (channel, ky, kx) of w[f][k] * x[tap k of pixel].  What bounds it is the
-// FMA rate (2 operations per weight-pixel pair against 4 bytes of either), so a thread keeps 8 filters x 8 pixels in registers and
-// every value it reads from shared memory serves eight of them; the products are formed two pixels at a time with packed
-// f32x2 FMAs, whose weight operand is stored twice in shared memory so that no instruction is spent on duplicating it.  The k
-// range advances in slices of 8, the next slice on its way from global memory into registers while the current one is multiplied.
-// Each output is one chain of fused multiply-adds in k order, the order of runtime/forward_layers.rs:646-695; only a split k range
-// (few tiles) sums the chains of its parts at the end.
-// BM filters x BN pixels per CTA.  KS: kernel size when it is 1 or 3, 0 = any.  Taps outside the image contribute 0.
-// (YOLOv4 608 x 608, batch 1: 69.4 ms with one thread per (pixel, 4 filters) reading both operands from L1.)
-constexpr int kSlice = 8;
+// Convolution as a blocked GEMM: y[f][pixel] = sum over k = (channel, ky, kx) of w[f][k] * x[tap k of pixel].  Each output is one chain of
+// fused multiply-adds in k order, the order of runtime/forward_layers.rs:646-695; where tiles are few the k range is split over the
+// CTAs of a cluster (blockIdx.z), which add their chains up in order through distributed shared memory: no second pass over the
+// output and no second launch.  Taps outside the image contribute 0.
 struct ConvF32 {
     const float* x;
     const float* w;
     const float* bias;  // null = none
     float* y;
     int B, C, H, W, F, k, sx, sy, dil, pad, OH, OW, K, act;
-    int k_part;       // k range of one part (blockIdx.z), a multiple of kSlice
-    int64_t part_elems;  // > 0: part z writes raw sums to y + z * part_elems
+    int k_part;  // k range of one part, a multiple of the slice
 };
 
 __device__ __forceinline__ unsigned long long fma2_f32(unsigned long long a, unsigned long long b, unsigned long long c) {
@@ -35,168 +32,326 @@ __device__ __forceinline__ unsigned long long fma2_f32(unsigned long long a, uns
     return d;
 }
 
+// Hands the CTA's tile (one per part of a split k range, side by side in distributed shared memory) to y: the parts added up in order,
+// bias, activation, 16-byte stores where the planes allow them.  Called by all threads after the tile is written.
+template <int BM, int BN, int T>
+__device__ __forceinline__ void conv_f32_finish(const ConvF32& p, float (&tile)[BM][BN], int f0, int n0) {
+    cg::cluster_group cluster = cg::this_cluster();
+    const int P = p.OH * p.OW, NP = p.B * P, parts = (int)gridDim.z, share = BM / parts;
+    if (parts > 1) cluster.sync();
+    else __syncthreads();
+    const bool vec = (P & 3) == 0;  // four consecutive pixels lie in one image then, at a 16-byte boundary
+    for (int i = (int)threadIdx.x; i < share * (BN / 4); i += T) {
+        const int m = (int)blockIdx.z * share + i / (BN / 4), c = i % (BN / 4) * 4, f = f0 + m, n = n0 + c;
+        if (f >= p.F || n >= NP) continue;
+        float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        for (int s = 0; s < parts; ++s) {
+            const float4 q = *reinterpret_cast<const float4*>(parts > 1 ? cluster.map_shared_rank(&tile[m][c], s) : &tile[m][c]);
+            v[0] += q.x; v[1] += q.y; v[2] += q.z; v[3] += q.w;
+        }
+        const float bias = p.bias ? __ldg(p.bias + f) : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = ln_act_f32(p.act, p.bias ? v[j] + bias : v[j]);
+        const int b = n / P;
+        if (vec) *reinterpret_cast<float4*>(p.y + ((int64_t)b * p.F + f) * P + (n - b * P)) = make_float4(v[0], v[1], v[2], v[3]);
+        else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (n + j < NP) {
+                    const int bj = (n + j) / P;
+                    p.y[((int64_t)bj * p.F + f) * P + (n + j - bj * P)] = v[j];
+                }
+        }
+    }
+    if (parts > 1) cluster.sync();  // nobody leaves while its tile is being read
+}
+
+// The main kernel: 1x1 without padding (KS = 1) and 3x3 without dilation (KS = 3), k a multiple of 4.  64 filters x BN pixels per CTA.
+// What bounds it is the FMA pipe, and next to it the issue slots and the shared-memory port, so
+//   - a thread keeps 8 filters x 8 pixels in registers and multiplies two pixels at a time with packed f32x2 FMAs, each of which takes one
+//     issue slot for two cycles of the pipe;
+//   - both operands go from global to shared memory with cp.async, a slice of 36 (4 channels x 9 taps: the taps are constant
+//     offsets from one pointer, valid or not by one bit of a mask computed once) or 32 channels ahead of the multiplication:
+//     no registers, no store instructions, and zero fill for what is outside;
+//   - weights stay in their own order, [filter][k], copied 16 bytes at a time and read four k at a time; the eight filters of a thread are
+//     eight rows apart, which keeps the reads free of bank conflicts.
+// (3x3 C256 -> K512 at 38x38: 146 us with operands staged through registers and k decoded per element -- 38 % of the instructions were
+// FMAs --, 139 us with weights transposed into shared memory four bytes at a time: the scatter filled the shared-memory port.)
+template <int BN, int KS>
+struct ConvF32Shared {
+    static constexpr int SL = KS == 3 ? 36 : 32, WL = SL + 4;
+    union {
+        struct { float w[2][64][WL]; float x[2][SL][BN]; } op;
+        float tile[64][BN];
+    };
+};
+
+template <int BN, int KS>
+__global__ void __launch_bounds__(BN, 512 / BN) conv2d_f32_async_kernel(const __grid_constant__ ConvF32 p) {
+    using Shared = ConvF32Shared<BN, KS>;
+    constexpr int T = BN, TX = BN / 8, SL = Shared::SL, WCOPIES = (64 * SL / 4 + T - 1) / T;
+    extern __shared__ __align__(16) unsigned char smem[];
+    Shared& sm = *reinterpret_cast<Shared*>(smem);
+    const int tid = (int)threadIdx.x, tx = tid % TX, ty = tid / TX;
+    const int P = p.OH * p.OW, HW = p.H * p.W, NP = p.B * P;
+    const int n0 = (int)blockIdx.x * BN, f0 = (int)blockIdx.y * 64;
+    const int k_begin = (int)blockIdx.z * p.k_part, k_end = min(p.K, k_begin + p.k_part);
+    // this thread's pixel: address of tap (0, 0) of the first channel of the range, and the taps inside the image as 4-byte copy sizes
+    const int n = n0 + tid;
+    const bool real = n < NP;
+    const int b = real ? n / P : 0, r = real ? n - b * P : 0, oy = r / p.OW, ox = r - oy * p.OW;
+    const int iy0 = oy * p.sy - p.pad, ix0 = ox * p.sx - p.pad;
+    const float* px = p.x + ((int64_t)b * p.C + k_begin / (KS * KS)) * HW + (int64_t)iy0 * p.W + ix0;
+    unsigned inside = 0u;  // bit t + 2 = tap t
+    if (real) {
+        if (KS == 1) inside = 4u;
+        else
+#pragma unroll
+            for (int t = 0; t < 9; ++t)
+                if (iy0 + t / 3 >= 0 && iy0 + t / 3 < p.H && ix0 + t % 3 >= 0 && ix0 + t % 3 < p.W) inside |= 4u << t;
+    }
+    // 1x1 stride 1 over planes of a multiple of 4: the tile's pixels are consecutive in memory, four per copy (thread: row tid / (BN / 4))
+    const bool x_vec = KS == 1 && p.sx == 1 && p.sy == 1 && (P & 3) == 0 && (((uintptr_t)p.x) & 15) == 0;
+    const int vn = n0 + (tid % (BN / 4)) * 4, vb = vn < NP ? vn / P : 0;
+    const float* vx = p.x + ((int64_t)vb * p.C + k_begin + tid / (BN / 4)) * HW + (vn < NP ? vn - vb * P : 0);
+    const float* wbase = p.w + (int64_t)f0 * p.K;
+    auto copy4 = [](const void* dst, const float* src, unsigned bytes) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+    };
+    auto copy16 = [](const void* dst, const float* src, unsigned bytes) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+    };
+    auto copy_slice = [&](int k0, int buf) {
+        const int left = k_end - k0;  // rows of the range from here on; the rest of the slice is filled with zeros
+#pragma unroll
+        for (int q = 0; q < WCOPIES; ++q) {
+            const int i = tid + q * T, m = i / (SL / 4), t = i % (SL / 4) * 4;
+            if ((64 * SL / 4) % T != 0 && m >= 64) break;
+            const bool ok = f0 + m < p.F && t < left;
+            copy16(&sm.op.w[buf][m][t], ok ? wbase + (int64_t)m * p.K + (k0 + t) : p.w, ok ? 16u : 0u);
+        }
+        if (KS == 3) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const bool ok = c * 9 < left;
+                const float* q0 = ok ? px : p.x;
+                const float* q1 = q0 + (ok ? p.W : 0);
+                const float* q2 = q1 + (ok ? p.W : 0);
+                const unsigned mask = ok ? inside : 0u;
+#pragma unroll
+                for (int t = 0; t < 9; ++t) copy4(&sm.op.x[buf][c * 9 + t][tid], (mask >> t) & 4u ? (t < 3 ? q0 : (t < 6 ? q1 : q2)) + t % 3 : p.x, (mask >> t) & 4u);
+                px += HW;
+            }
+        } else if (x_vec) {
+#pragma unroll
+            for (int q = 0; q < SL / 4; ++q) {
+                const int row = tid / (BN / 4) + q * 4;
+                const bool ok = vn < NP && row < left;
+                copy16(&sm.op.x[buf][row][(tid % (BN / 4)) * 4], ok ? vx : p.x, ok ? 16u : 0u);
+                vx += (int64_t)4 * HW;
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < SL; ++c) {
+                const bool ok = inside && c < left;
+                copy4(&sm.op.x[buf][c][tid], ok ? px : p.x, ok ? 4u : 0u);
+                px += HW;
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    unsigned long long acc[8][4];  // filter ty + 8 i x pixel pairs
+#pragma unroll
+    for (int m = 0; m < 8; ++m)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[m][q] = 0ull;
+    if (k_begin < k_end) copy_slice(k_begin, 0);  // (rounding the parts to whole slices can leave the last one empty)
+    int buf = 0;
+    for (int k0 = k_begin; k0 < k_end; k0 += SL) {
+        if (k0 + SL < k_end) {
+            copy_slice(k0 + SL, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+#pragma unroll
+        for (int g = 0; g < SL / 4; ++g) {
+            float4 w[8];
+#pragma unroll
+            for (int m = 0; m < 8; ++m) w[m] = *reinterpret_cast<const float4*>(&sm.op.w[buf][ty + 8 * m][4 * g]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const ulonglong2 xa = *reinterpret_cast<const ulonglong2*>(&sm.op.x[buf][4 * g + e][tx * 4]), xb = *reinterpret_cast<const ulonglong2*>(&sm.op.x[buf][4 * g + e][BN / 2 + tx * 4]);
+#pragma unroll
+                for (int m = 0; m < 8; ++m) {
+                    const float v = e == 0 ? w[m].x : (e == 1 ? w[m].y : (e == 2 ? w[m].z : w[m].w));
+                    unsigned long long w2;
+                    asm("mov.b64 %0, {%1, %1};" : "=l"(w2) : "f"(v));
+                    acc[m][0] = fma2_f32(w2, xa.x, acc[m][0]);
+                    acc[m][1] = fma2_f32(w2, xa.y, acc[m][1]);
+                    acc[m][2] = fma2_f32(w2, xb.x, acc[m][2]);
+                    acc[m][3] = fma2_f32(w2, xb.y, acc[m][3]);
+                }
+            }
+        }
+        __syncthreads();
+        buf ^= 1;
+    }
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+        *reinterpret_cast<ulonglong2*>(&sm.tile[ty + 8 * m][tx * 4]) = make_ulonglong2(acc[m][0], acc[m][1]);
+        *reinterpret_cast<ulonglong2*>(&sm.tile[ty + 8 * m][BN / 2 + tx * 4]) = make_ulonglong2(acc[m][2], acc[m][3]);
+    }
+    conv_f32_finish<64, BN, T>(p, sm.tile, f0, n0);
+}
+
+// Layers of few filters and every other geometry: BM filters x BN pixels, operands staged through registers (the weights with 4-byte
+// copies), slices of one channel for 3x3 kernels (KS = 3) and of eight k otherwise (KS = 1: 1x1 without padding, 0: anything).
+constexpr int conv_slice(int ks) { return ks == 3 ? 9 : 8; }
+
 template <int BM, int BN, int KS>
 __global__ void __launch_bounds__(BM * BN / 64, 32768 / (BM * BN)) conv2d_f32_gemm_kernel(const __grid_constant__ ConvF32 p) {
-    constexpr int T = BM * BN / 64, TX = BN / 8;
-    constexpr int PIX = BN > T ? BN / T : 1;      // pixels a thread gathers
-    constexpr int RSTEP = T > BN ? T / BN : 1;    // k rows gathered side by side
-    constexpr int ROWS = kSlice / RSTEP;          // k rows per thread and pixel
-    constexpr int WV = BM * 2 / T;                // groups of four weights per thread
-    __shared__ __align__(16) float2 s_w[2][kSlice][BM];
-    __shared__ __align__(16) float s_x[2][kSlice][BN];
+    constexpr int T = BM * BN / 64, TX = BN / 8, SL = conv_slice(KS);
+    static_assert(BN % T == 0, "every thread gathers whole columns of x");
+    constexpr int PIX = BN / T;                   // pixels a thread gathers
+    constexpr int WQ = (BM * SL + T - 1) / T;     // weights a thread copies: element tid + q * T of [filter][k of the slice]
+    constexpr int WL = BM + 4;                    // (padded: the copies of a warp scatter over several rows)
+    struct Operands { float w[2][SL][WL]; float2 x[2][SL][BN]; };
+    __shared__ __align__(16) union { Operands op; float tile[BM][BN]; } sm;
     const int tid = (int)threadIdx.x, tx = tid % TX, ty = tid / TX;
     const int P = p.OH * p.OW, HW = p.H * p.W, NP = p.B * P;
     const int n0 = (int)blockIdx.x * BN, f0 = (int)blockIdx.y * BM;
     const int k_begin = (int)blockIdx.z * p.k_part, k_end = min(p.K, k_begin + p.k_part);
-    const int kk = KS ? KS * KS : p.k * p.k;
-    // the pixels this thread gathers: address of tap (0, 0) and which taps are inside the image (kernels up to 8 x 8; larger ones test)
+    // the pixels this thread gathers: address of tap (0, 0) of the first channel of the range, and which taps are inside the image
     const float* px[PIX];
-    unsigned long long inside[PIX];
+    unsigned inside[PIX];
     int oy0[PIX], ox0[PIX];
+    const int c_begin = KS == 3 ? k_begin / 9 : (KS == 1 ? k_begin : 0);
 #pragma unroll
     for (int j = 0; j < PIX; ++j) {
-        const int n = n0 + (tid % BN) + j * T;
+        const int n = n0 + tid + j * T;
+        const bool real = n < NP;
         const int b = n / P, r = n - b * P, oy = r / p.OW, ox = r - oy * p.OW;
-        oy0[j] = n < NP ? oy * p.sy - p.pad : -(1 << 28);
+        oy0[j] = real ? oy * p.sy - p.pad : -(1 << 28);
         ox0[j] = ox * p.sx - p.pad;
-        px[j] = p.x + (int64_t)(n < NP ? b : 0) * p.C * HW + (int64_t)(n < NP ? oy0[j] : 0) * p.W + ox0[j];
-        inside[j] = 0ull;
-        const int ks = KS ? KS : p.k;
-        if (ks <= 8)
-            for (int t = 0; t < ks * ks; ++t) {
-                const int iy = oy0[j] + (t / ks) * p.dil, ix = ox0[j] + (t % ks) * p.dil;
-                if (iy >= 0 && iy < p.H && ix >= 0 && ix < p.W) inside[j] |= 1ull << t;
+        px[j] = p.x + ((int64_t)(real ? b : 0) * p.C + c_begin) * HW + (int64_t)(real ? oy0[j] : 0) * p.W + ox0[j];
+        inside[j] = 0u;
+        if (KS == 1) inside[j] = real ? 1u : 0u;
+        if (KS == 3)
+#pragma unroll
+            for (int t = 0; t < 9; ++t) {
+                const int iy = oy0[j] + t / 3, ix = ox0[j] + t % 3;
+                if (iy >= 0 && iy < p.H && ix >= 0 && ix < p.W) inside[j] |= 1u << t;
             }
     }
-    const int row0 = T > BN ? tid / BN : 0;
-    float gx[ROWS][PIX];
-    float4 gw[WV];
-    const bool w_vec = (p.K & 3) == 0 && (((uintptr_t)p.w) & 15) == 0;
-    auto fetch = [&](int k0) {
+    const float* wbase = p.w + (int64_t)f0 * p.K;
+    int woff[WQ];  // from wbase, -1: no such filter
 #pragma unroll
-        for (int i = 0; i < ROWS; ++i) {
-            const int kr = k0 + row0 + i * RSTEP;
-            const int c = kr / kk, tap = kr - c * kk;
-            const int ks = KS ? KS : p.k;
-            const int ky = KS == 1 ? 0 : tap / ks, kx = KS == 1 ? 0 : tap - ky * ks;
-            const int64_t off = (int64_t)c * HW + (int64_t)(ky * p.dil) * p.W + kx * p.dil;
+    for (int q = 0; q < WQ; ++q) {
+        const int i = tid + q * T, m = i / SL;
+        woff[q] = m < BM && f0 + m < p.F ? m * p.K + (i - m * SL) : -1;
+    }
+    float gx[SL][PIX];
+    auto fetch = [&](int k0) {
+        if constexpr (KS == 3) {
 #pragma unroll
             for (int j = 0; j < PIX; ++j) {
-                bool ok = kr < k_end;
-                if (KS != 0 || p.k <= 8) ok = ok && ((inside[j] >> tap) & 1ull);
-                else {
-                    const int iy = oy0[j] + ky * p.dil, ix = ox0[j] + kx * p.dil;
-                    ok = ok && iy >= 0 && iy < p.H && ix >= 0 && ix < p.W;
-                }
-                gx[i][j] = ok ? __ldg(px[j] + off) : 0.0f;
-            }
-        }
+                const float* q0 = px[j];
+                const float* q1 = q0 + p.W;
+                const float* q2 = q1 + p.W;
 #pragma unroll
-        for (int i = 0; i < WV; ++i) {
-            const int v = tid + i * T, f = f0 + (v >> 1), kr = k0 + (v & 1) * 4;
-            float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (f < p.F) {
-                const float* wp = p.w + (int64_t)f * p.K + kr;
-                if (w_vec && kr + 4 <= k_end) q = __ldg(reinterpret_cast<const float4*>(wp));
-                else {
-                    if (kr < k_end) q.x = __ldg(wp);
-                    if (kr + 1 < k_end) q.y = __ldg(wp + 1);
-                    if (kr + 2 < k_end) q.z = __ldg(wp + 2);
-                    if (kr + 3 < k_end) q.w = __ldg(wp + 3);
+                for (int t = 0; t < 9; ++t) gx[t][j] = (inside[j] >> t) & 1u ? __ldg((t < 3 ? q0 : (t < 6 ? q1 : q2)) + t % 3) : 0.0f;
+                px[j] += HW;
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < PIX; ++j) {
+                if constexpr (KS == 1) {
+                    const float* q = px[j];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        gx[i][j] = inside[j] && k0 + i < k_end ? __ldg(q) : 0.0f;
+                        q += HW;
+                    }
+                    px[j] = q;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int kr = k0 + i, c = kr / (p.k * p.k), tap = kr - c * p.k * p.k, ky = tap / p.k, kx = tap - ky * p.k;
+                        const int iy = oy0[j] + ky * p.dil, ix = ox0[j] + kx * p.dil;
+                        const bool ok = kr < k_end && iy >= 0 && iy < p.H && ix >= 0 && ix < p.W;
+                        gx[i][j] = ok ? __ldg(px[j] + (int64_t)c * HW + (int64_t)(ky * p.dil) * p.W + kx * p.dil) : 0.0f;
+                    }
                 }
             }
-            gw[i] = q;
         }
+    };
+    auto copy_weights = [&](int k0, int buf) {
+#pragma unroll
+        for (int q = 0; q < WQ; ++q) {
+            const int i = tid + q * T, m = i / SL, t = i - m * SL;
+            if ((BM * SL) % T != 0 && m >= BM) break;
+            const bool ok = woff[q] >= 0 && (KS == 3 || k0 + t < k_end);
+            const float* src = wbase + (ok ? woff[q] + k0 : 0);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(&sm.op.w[buf][t][m])), "l"(src), "r"(ok ? 4 : 0) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
     auto store = [&](int buf) {
 #pragma unroll
-        for (int i = 0; i < ROWS; ++i)
+        for (int i = 0; i < SL; ++i)
 #pragma unroll
-            for (int j = 0; j < PIX; ++j) s_x[buf][row0 + i * RSTEP][(tid % BN) + j * T] = gx[i][j];
-#pragma unroll
-        for (int i = 0; i < WV; ++i) {
-            const int v = tid + i * T, m = v >> 1, r = (v & 1) * 4;
-            s_w[buf][r][m] = make_float2(gw[i].x, gw[i].x);
-            s_w[buf][r + 1][m] = make_float2(gw[i].y, gw[i].y);
-            s_w[buf][r + 2][m] = make_float2(gw[i].z, gw[i].z);
-            s_w[buf][r + 3][m] = make_float2(gw[i].w, gw[i].w);
-        }
+            for (int j = 0; j < PIX; ++j) sm.op.x[buf][i][tid + j * T] = make_float2(gx[i][j], gx[i][j]);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
     };
-    unsigned long long acc[8][4];
+    unsigned long long acc[4][8];  // filters 2i, 2i + 1 of the thread x its eight pixels
 #pragma unroll
-    for (int m = 0; m < 8; ++m)
+    for (int m = 0; m < 4; ++m)
 #pragma unroll
-        for (int n = 0; n < 4; ++n) acc[m][n] = 0ull;
-    fetch(k_begin);
-    store(0);
+        for (int n = 0; n < 8; ++n) acc[m][n] = 0ull;
+    if (k_begin < k_end) {  // (rounding the parts to whole slices can leave the last one empty)
+        copy_weights(k_begin, 0);
+        fetch(k_begin);
+        store(0);
+    }
     __syncthreads();
     int buf = 0;
-    for (int k0 = k_begin; k0 < k_end; k0 += kSlice) {
-        const bool more = k0 + kSlice < k_end;
-        if (more) fetch(k0 + kSlice);
+    for (int k0 = k_begin; k0 < k_end; k0 += SL) {
+        const bool more = k0 + SL < k_end;
+        if (more) {
+            copy_weights(k0 + SL, buf ^ 1);
+            fetch(k0 + SL);
+        }
 #pragma unroll
-        for (int r = 0; r < kSlice; ++r) {
-            const ulonglong2 xa = *reinterpret_cast<const ulonglong2*>(&s_x[buf][r][tx * 4]), xb = *reinterpret_cast<const ulonglong2*>(&s_x[buf][r][BN / 2 + tx * 4]);
+        for (int r = 0; r < SL; ++r) {
+            const ulonglong2 wa = *reinterpret_cast<const ulonglong2*>(&sm.op.w[buf][r][ty * 8]), wb = *reinterpret_cast<const ulonglong2*>(&sm.op.w[buf][r][ty * 8 + 4]);
 #pragma unroll
-            for (int m = 0; m < 8; m += 2) {
-                const ulonglong2 w2 = *reinterpret_cast<const ulonglong2*>(&s_w[buf][r][ty * 8 + m]);
-                acc[m][0] = fma2_f32(w2.x, xa.x, acc[m][0]);
-                acc[m][1] = fma2_f32(w2.x, xa.y, acc[m][1]);
-                acc[m][2] = fma2_f32(w2.x, xb.x, acc[m][2]);
-                acc[m][3] = fma2_f32(w2.x, xb.y, acc[m][3]);
-                acc[m + 1][0] = fma2_f32(w2.y, xa.x, acc[m + 1][0]);
-                acc[m + 1][1] = fma2_f32(w2.y, xa.y, acc[m + 1][1]);
-                acc[m + 1][2] = fma2_f32(w2.y, xb.x, acc[m + 1][2]);
-                acc[m + 1][3] = fma2_f32(w2.y, xb.y, acc[m + 1][3]);
+            for (int q = 0; q < 4; ++q) {  // pixels 2 tx + (BN / 4) q and the one after it
+                const ulonglong2 x2 = *reinterpret_cast<const ulonglong2*>(&sm.op.x[buf][r][q * (BN / 4) + tx * 2]);
+                acc[0][2 * q] = fma2_f32(wa.x, x2.x, acc[0][2 * q]);
+                acc[1][2 * q] = fma2_f32(wa.y, x2.x, acc[1][2 * q]);
+                acc[2][2 * q] = fma2_f32(wb.x, x2.x, acc[2][2 * q]);
+                acc[3][2 * q] = fma2_f32(wb.y, x2.x, acc[3][2 * q]);
+                acc[0][2 * q + 1] = fma2_f32(wa.x, x2.y, acc[0][2 * q + 1]);
+                acc[1][2 * q + 1] = fma2_f32(wa.y, x2.y, acc[1][2 * q + 1]);
+                acc[2][2 * q + 1] = fma2_f32(wb.x, x2.y, acc[2][2 * q + 1]);
+                acc[3][2 * q + 1] = fma2_f32(wb.y, x2.y, acc[3][2 * q + 1]);
             }
         }
         if (more) store(buf ^ 1);
         __syncthreads();
         buf ^= 1;
     }
-    const bool part = p.part_elems > 0;
-    float* y = p.y + (part ? (int64_t)blockIdx.z * p.part_elems : 0);
-    const bool vec = (P & 3) == 0;  // four consecutive pixels lie in one image then, at a 16-byte boundary
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int n = n0 + h * (BN / 2) + tx * 4;
+    for (int m = 0; m < 4; ++m)
 #pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            const int f = f0 + ty * 8 + m;
-            if (f >= p.F || n >= NP) continue;
-            float v[4];
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(acc[m][2 * h]));
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(v[2]), "=f"(v[3]) : "l"(acc[m][2 * h + 1]));
-            if (!part) {
-                const float bias = p.bias ? __ldg(p.bias + f) : 0.0f;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) v[j] = ln_act_f32(p.act, p.bias ? v[j] + bias : v[j]);
-            }
-            if (vec) {
-                const int b = n / P;
-                *reinterpret_cast<float4*>(y + ((int64_t)b * p.F + f) * P + (n - b * P)) = make_float4(v[0], v[1], v[2], v[3]);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (n + j < NP) {
-                        const int b = (n + j) / P;
-                        y[((int64_t)b * p.F + f) * P + (n + j - b * P)] = v[j];
-                    }
-            }
+        for (int q = 0; q < 4; ++q) {
+            float a0, b0, a1, b1;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(b0) : "l"(acc[m][2 * q]));
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(a1), "=f"(b1) : "l"(acc[m][2 * q + 1]));
+            *reinterpret_cast<float2*>(&sm.tile[ty * 8 + 2 * m][q * (BN / 4) + tx * 2]) = make_float2(a0, a1);
+            *reinterpret_cast<float2*>(&sm.tile[ty * 8 + 2 * m + 1][q * (BN / 4) + tx * 2]) = make_float2(b0, b1);
         }
-    }
-}
-
-// Adds the parts of a split k range in order, then bias and activation.  blockIdx.y = (image, filter) plane.
-__global__ void conv2d_f32_sum_parts_kernel(const float* __restrict__ parts, int n_parts, int64_t part_elems, const float* __restrict__ bias, float* __restrict__ y, int F,
-                                            int P, int act) {
-    const int64_t plane = (int64_t)blockIdx.y * P;
-    const float b = bias ? __ldg(bias + (int)(blockIdx.y % (unsigned)F)) : 0.0f;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P; i += gridDim.x * blockDim.x) {
-        float v = 0.0f;
-        for (int s = 0; s < n_parts; ++s) v += parts[(int64_t)s * part_elems + plane + i];
-        y[plane + i] = ln_act_f32(act, bias ? v + b : v);
-    }
+    conv_f32_finish<BM, BN, T>(p, sm.tile, f0, n0);
 }
 
 // Grouped convolutions: one thread per (pixel, group of FPT filters).  Semantics of runtime/forward_layers.rs:646-695: taps outside
@@ -364,8 +519,16 @@ __global__ void yolo_activate_f32_kernel(const float* __restrict__ x, float* __r
     }
 }
 
+// (tensors start at 512-byte boundaries or at an image of a batch: four values at a time while the count allows)
 __global__ void add_f32_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ y, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) y[i] = a[i] + b[i];
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    const bool vec = ((((uintptr_t)a) | ((uintptr_t)b) | ((uintptr_t)y)) & 15) == 0;
+    const int64_t n4 = vec ? n / 4 : 0;
+    for (int64_t i = t; i < n4; i += step) {
+        const float4 u = reinterpret_cast<const float4*>(a)[i], v = reinterpret_cast<const float4*>(b)[i];
+        reinterpret_cast<float4*>(y)[i] = make_float4(u.x + v.x, u.y + v.y, u.z + v.z, u.w + v.w);
+    }
+    for (int64_t i = 4 * n4 + t; i < n; i += step) y[i] = a[i] + b[i];
 }
 
 // shortcut_fit: flat per-sample crop / zero-pad (lightnet-cuda/src/lib.rs:4036-4056)
@@ -378,14 +541,15 @@ __global__ void shortcut_fit_f32_kernel(const float* __restrict__ x, float* __re
     }
 }
 
-// route copy of one source's channel slice (runtime/layer_ops.rs:1850-1883)
-__global__ void route_copy_f32_kernel(const float* __restrict__ x, float* __restrict__ y, int64_t batch, int64_t src_total_c,
-                                      int64_t src_c0, int64_t chunk_c, int64_t dst_total_c, int64_t dst_c0, int64_t plane) {
-    int64_t n = batch * chunk_c * plane;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        int64_t p = i % plane, c = (i / plane) % chunk_c, b = i / (plane * chunk_c);
-        y[(b * dst_total_c + dst_c0 + c) * plane + p] = x[(b * src_total_c + src_c0 + c) * plane + p];
-    }
+// route copy of one source's channel slice (runtime/layer_ops.rs:1850-1883): per image one contiguous run of `run` floats.
+// blockIdx.y = image.  (With a 64-bit division per value the copies of YOLOv4 608 x 608 took 333 us per image.)
+__global__ void route_copy_f32_kernel(const float* __restrict__ x, float* __restrict__ y, int64_t run, int64_t x_image, int64_t y_image) {
+    const float* src = x + blockIdx.y * x_image;
+    float* dst = y + blockIdx.y * y_image;
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    const int64_t n4 = ((((uintptr_t)src) | ((uintptr_t)dst)) & 15) == 0 ? run / 4 : 0;
+    for (int64_t i = t; i < n4; i += step) reinterpret_cast<float4*>(dst)[i] = __ldg(reinterpret_cast<const float4*>(src) + i);
+    for (int64_t i = 4 * n4 + t; i < run; i += step) dst[i] = src[i];
 }
 
 // Darknet max-pool: window origin o*stride - padding/2, taps outside skipped, start at -inf
@@ -457,55 +621,54 @@ int grid_for(ln_ctx* ctx, int64_t n) {
 
 bool is_f32(const ln_tensor* t) { return t && t->dtype == LN_F32; }
 
-template <int BM, int BN>
-void launch_conv_f32(const ConvF32& p, dim3 grid, cudaStream_t stream) {
-    if (p.k == 1) conv2d_f32_gemm_kernel<BM, BN, 1><<<grid, BM * BN / 64, 0, stream>>>(p);
-    else if (p.k == 3) conv2d_f32_gemm_kernel<BM, BN, 3><<<grid, BM * BN / 64, 0, stream>>>(p);
-    else conv2d_f32_gemm_kernel<BM, BN, 0><<<grid, BM * BN / 64, 0, stream>>>(p);
+template <class K>
+cudaError_t launch_conv_f32(ln_ctx* ctx, K kernel, const ConvF32& p, int threads, size_t smem, dim3 grid) {
+    if (smem > 48 * 1024 && !ctx->configured_kernels.count((const void*)kernel)) {  // once per kernel per context
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        ctx->configured_kernels.insert((const void*)kernel);
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = grid.z;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    ctx->launches++;
+    return cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
-// Ungrouped convolution with optional bias and activation.  Tile: 128 x 128 while that gives every SM two CTAs; narrow layers take the
-// narrowest tile that covers their filters; everything smaller takes 64 x 64, and the k range is split until there are about
-// eight CTAs (of 64 threads) per SM, in parts of at least 64 (a part costs a pass over the output).
+// Ungrouped convolution with optional bias and activation.  Tile: 64 filters x 128 pixels while that gives every SM four CTAs (of four
+// warps) even without splitting, 64 x 64 below; layers of at most 32 filters 32 x 128.  The k range is split over clusters of up to eight
+// CTAs until there are about eight CTAs of two warps per SM, in parts of at least two slices.
 int conv_f32_run(ln_ctx* ctx, ConvF32 p, const char* who) {
-    const int64_t NP = (int64_t)p.B * p.OH * p.OW, planes = (int64_t)p.B * p.F;
+    const int64_t NP = (int64_t)p.B * p.OH * p.OW;
+    const int ks = p.k == 1 && p.pad == 0 ? 1 : (p.k == 3 && p.dil == 1 ? 3 : 0);
+    const bool async = ks != 0 && p.F > 32 && (p.K & 3) == 0 && (((uintptr_t)p.w) & 15) == 0;
     auto tiles = [&](int bm, int bn) { return ((NP + bn - 1) / bn) * ((p.F + bm - 1) / bm); };
-    int bm = 64, bn = 64;
-    if (p.F <= 32 && tiles(32, 128) >= 4 * ctx->sm_count) { bm = 32; bn = 128; }
-    else if (p.F <= 64 && tiles(64, 128) >= 4 * ctx->sm_count) { bm = 64; bn = 128; }
-    else if (p.F > 64 && tiles(128, 128) >= 2 * ctx->sm_count) { bm = 128; bn = 128; }
+    const bool narrow = !async && p.F <= 32;
+    const int64_t tail = ln_round_up(NP, 128) - NP;
+    const bool wide = async && tail * 10 <= NP && tiles(64, 128) * 8 >= 2ll * ctx->sm_count;
+    const int bm = narrow ? 32 : 64, bn = narrow || wide ? 128 : 64, slice = async ? (ks == 3 ? 36 : 32) : conv_slice(ks);
     int parts = 1;
-    if (bm == 64 && bn == 64) {
-        const int64_t want = (8ll * ctx->sm_count + tiles(64, 64) - 1) / tiles(64, 64);
-        parts = (int)(want < p.K / 64 ? want : p.K / 64);
-        if (parts > 32) parts = 32;
-        if (parts < 1 || planes > 65535) parts = 1;
-    }
-    p.k_part = (int)ln_round_up((p.K + parts - 1) / parts, kSlice);
-    parts = (p.K + p.k_part - 1) / p.k_part;
+    while (parts < 8 && tiles(bm, bn) * parts * 2 <= (wide ? 4ll : 8ll) * ctx->sm_count && p.K / (parts * 2) >= (async ? 2 : 4) * slice) parts *= 2;
+    p.k_part = (int)ln_round_up((p.K + parts - 1) / parts, slice);
     const dim3 grid((unsigned)((NP + bn - 1) / bn), (unsigned)((p.F + bm - 1) / bm), (unsigned)parts);
-    float* y = p.y;
-    void* ws = nullptr;
-    size_t ws_bytes = 0;
-    if (parts > 1) {
-        p.part_elems = planes * p.OH * p.OW;
-        ws_bytes = (size_t)parts * p.part_elems * 4;
-        ws = ln_pool_alloc(ctx, ws_bytes);
-        if (!ws) return LN_ERR_CUDA;
-        p.y = (float*)ws;
-    }
-    if (bm == 128) launch_conv_f32<128, 128>(p, grid, ctx->stream);
-    else if (bm == 32) launch_conv_f32<32, 128>(p, grid, ctx->stream);
-    else if (bn == 128) launch_conv_f32<64, 128>(p, grid, ctx->stream);
-    else launch_conv_f32<64, 64>(p, grid, ctx->stream);
-    ctx->launches++;
-    if (ws) {
-        const int P = p.OH * p.OW, t = P < 128 ? 64 : (P < 512 ? 128 : 256);
-        conv2d_f32_sum_parts_kernel<<<dim3((unsigned)((P + t - 1) / t), (unsigned)planes), t, 0, ctx->stream>>>(p.y, parts, p.part_elems, p.bias, y, p.F, P, p.act);
-        ctx->launches++;
-        ln_pool_free(ctx, ws, ws_bytes);
-    }
-    const cudaError_t e = cudaGetLastError();
+    cudaError_t e;
+    if (wide) e = ks == 1 ? launch_conv_f32(ctx, conv2d_f32_async_kernel<128, 1>, p, 128, sizeof(ConvF32Shared<128, 1>), grid)
+                          : launch_conv_f32(ctx, conv2d_f32_async_kernel<128, 3>, p, 128, sizeof(ConvF32Shared<128, 3>), grid);
+    else if (async) e = ks == 1 ? launch_conv_f32(ctx, conv2d_f32_async_kernel<64, 1>, p, 64, sizeof(ConvF32Shared<64, 1>), grid)
+                                : launch_conv_f32(ctx, conv2d_f32_async_kernel<64, 3>, p, 64, sizeof(ConvF32Shared<64, 3>), grid);
+    else if (narrow) e = ks == 1 ? launch_conv_f32(ctx, conv2d_f32_gemm_kernel<32, 128, 1>, p, 64, 0, grid)
+                                 : (ks == 3 ? launch_conv_f32(ctx, conv2d_f32_gemm_kernel<32, 128, 3>, p, 64, 0, grid) : launch_conv_f32(ctx, conv2d_f32_gemm_kernel<32, 128, 0>, p, 64, 0, grid));
+    else e = ks == 1 ? launch_conv_f32(ctx, conv2d_f32_gemm_kernel<64, 64, 1>, p, 64, 0, grid)
+                     : (ks == 3 ? launch_conv_f32(ctx, conv2d_f32_gemm_kernel<64, 64, 3>, p, 64, 0, grid) : launch_conv_f32(ctx, conv2d_f32_gemm_kernel<64, 64, 0>, p, 64, 0, grid));
     return e == cudaSuccess ? LN_OK : ln_fail(ctx, LN_ERR_CUDA, "%s launch: %s", who, cudaGetErrorString(e));
 }
 
@@ -550,7 +713,7 @@ int ln_conv2d_bias_act_f32(ln_ctx* ctx, const ln_tensor* x, const ln_tensor* wei
     if (!y) return LN_ERR_CUDA;
     const float* b = bias ? (const float*)bias->ptr : nullptr;
     int rc = LN_OK;
-    if (groups == 1 && x->n * oh * ow < (1ll << 30) && x->count() < (1ll << 40)) {
+    if (groups == 1 && x->n * oh * ow < (1ll << 30) && x->count() < (1ll << 40) && input_channels * kernel_size * kernel_size < (1ll << 24)) {
         ConvF32 p = {};
         p.x = (const float*)x->ptr; p.w = (const float*)weights->ptr; p.bias = b; p.y = (float*)y->ptr;
         p.B = (int)x->n; p.C = (int)input_channels; p.H = (int)input_height; p.W = (int)input_width; p.F = (int)filters; p.k = (int)kernel_size;
@@ -745,10 +908,12 @@ int32_t ln_route_concat_f32(ln_ctx* ctx, const ln_tensor* const* inputs, int32_t
     if (!o) return LN_ERR_CUDA;
     int64_t c0 = 0;
     for (int i = 0; i < n_inputs; ++i) {
-        int64_t n = o->n * input_channels[i] * channel_stride;
-        route_copy_f32_kernel<<<grid_for(ctx, n), kThreads, 0, ctx->stream>>>((const float*)inputs[i]->ptr, (float*)o->ptr, o->n,
-                                                                             input_total_channels[i], input_channel_offsets[i],
-                                                                             input_channels[i], o->c, c0, channel_stride);
+        const int64_t run = input_channels[i] * channel_stride;
+        for (int64_t b0 = 0; b0 < o->n; b0 += 65535) {  // (grid limit in y)
+            const int64_t images = o->n - b0 < 65535 ? o->n - b0 : 65535, x_image = input_total_channels[i] * channel_stride, y_image = o->c * channel_stride;
+            route_copy_f32_kernel<<<dim3((unsigned)grid_for(ctx, (run + 3) / 4), (unsigned)images), kThreads, 0, ctx->stream>>>(
+                (const float*)inputs[i]->ptr + b0 * x_image + input_channel_offsets[i] * channel_stride, (float*)o->ptr + b0 * y_image + c0 * channel_stride, run, x_image, y_image);
+        }
         ctx->launches++;
         c0 += input_channels[i];
     }

@@ -479,6 +479,11 @@ int forward_f32(ln_net* net, const ln_tensor* input, unsigned* amax_dev) {
                 rc = ln_maxpool_f32(ctx, x, oshape, L.in.c, L.in.h, L.in.w, L.size, L.stride_x, L.stride_y, L.padding, &y);
                 break;
             case K_ROUTE: {  // layers/route/gpu.rs:61-108
+                if (L.sources.size() == 1 && L.route_groups == 1) {  // the source itself: tensors are never written again
+                    y = net->out[L.sources[0]];
+                    ln_tensor_retain(y);
+                    break;
+                }
                 std::vector<const ln_tensor*> ins;
                 std::vector<int64_t> offs, chans, totals;
                 for (int src : L.sources) {
@@ -560,6 +565,11 @@ int forward_f16(ln_net* net, const ln_tensor* input) {
                 rc = ln_maxpool_f16(ctx, x, oshape, L.in.c, L.in.h, L.in.w, L.size, L.stride_x, L.stride_y, L.padding, &y);
                 break;
             case K_ROUTE: {
+                if (L.sources.size() == 1 && L.route_groups == 1) {
+                    y = net->out[L.sources[0]];
+                    ln_tensor_retain(y);
+                    break;
+                }
                 std::vector<const ln_tensor*> ins;
                 std::vector<int64_t> offs, chans, totals;
                 for (int src : L.sources) {

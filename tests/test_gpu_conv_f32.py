@@ -16,10 +16,11 @@ def be():
 
 # batch, channels, height, width, filters, kernel, stride, padding, dilation
 @pytest.mark.parametrize("geom", [
-    (1, 5, 161, 159, 129, 3, 1, 1, 1),   # 128 x 128 tiles, ragged on both sides, k range not a multiple of the slice
-    (1, 32, 160, 160, 256, 1, 1, 0, 1),  # 128 x 128 tiles, whole
-    (1, 3, 281, 279, 17, 3, 1, 1, 1),    # 32 x 128
-    (2, 4, 200, 201, 33, 3, 1, 1, 1),    # 64 x 128
+    (1, 5, 161, 159, 129, 3, 1, 1, 1),   # k range not a multiple of 4
+    (1, 32, 160, 160, 256, 1, 1, 0, 1),  # 64 x 128 tiles, whole
+    (1, 3, 281, 279, 17, 3, 1, 1, 1),    # 32 x 128, staged through registers
+    (2, 4, 200, 201, 33, 3, 1, 1, 1),    # one slice
+    (1, 36, 104, 104, 65, 3, 1, 1, 1),   # 64 x 128, split k range of several slices with a short last one
     (3, 64, 19, 19, 70, 3, 1, 1, 1),     # 64 x 64, split k range, pixels of two images in one group of four
     (1, 1024, 4, 4, 255, 1, 1, 0, 1),    # split, planes of 16
     (2, 20, 13, 11, 65, 3, 2, 1, 1),
