@@ -81,7 +81,7 @@ int ln_status(ln_ctx* ctx, const char* where);        // after a synchronisation
 int ln_check_status(ln_ctx* ctx, const char* where);  // synchronises the ctx stream first
 int ln_conv2d_bias_act_f32(ln_ctx* ctx, const ln_tensor* x, const ln_tensor* weights, const ln_tensor* bias, const int64_t output_shape[4], int64_t input_channels,
                            int64_t input_height, int64_t input_width, int64_t filters, int64_t kernel_size, int64_t stride_x, int64_t stride_y, int64_t dilation,
-                           int64_t padding, int64_t groups, int activation, ln_tensor** out);
+                           int64_t padding, int64_t groups, int activation, bool one_chain, ln_tensor** out);
 int ln_image_preprocess_enqueue(ln_ctx* ctx, cudaStream_t stream, const uint8_t* pixels_host, const int64_t* offsets, const int32_t* widths,
                                 const int32_t* heights, int32_t count, int32_t mode, int32_t dst_w, int32_t dst_h, float* dst, void** staging,
                                 size_t* staging_bytes);

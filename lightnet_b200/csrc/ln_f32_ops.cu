@@ -647,7 +647,9 @@ cudaError_t launch_conv_f32(ln_ctx* ctx, K kernel, const ConvF32& p, int threads
 // Ungrouped convolution with optional bias and activation.  Tile: 64 filters x 128 pixels while that gives every SM four CTAs (of four
 // warps) even without splitting, 64 x 64 below; layers of at most 32 filters 32 x 128.  The k range is split over clusters of up to eight
 // CTAs until there are about eight CTAs of two warps per SM, in parts of at least two slices.
-int conv_f32_run(ln_ctx* ctx, ConvF32 p, const char* who) {
+// one_chain: no split, so that every output is one chain of fused multiply-adds whatever the batch and the number of SMs.  Calibration
+// asks for it: the scales of an 8-bit network, and with them its codes, must not depend on how the work was cut.
+int conv_f32_run(ln_ctx* ctx, ConvF32 p, bool one_chain, const char* who) {
     const int64_t NP = (int64_t)p.B * p.OH * p.OW;
     const int ks = p.k == 1 && p.pad == 0 ? 1 : (p.k == 3 && p.dil == 1 ? 3 : 0);
     const bool async = ks != 0 && p.F > 32 && (p.K & 3) == 0 && (((uintptr_t)p.w) & 15) == 0;
@@ -657,7 +659,7 @@ int conv_f32_run(ln_ctx* ctx, ConvF32 p, const char* who) {
     const bool wide = async && tail * 10 <= NP && tiles(64, 128) * 8 >= 2ll * ctx->sm_count;
     const int bm = narrow ? 32 : 64, bn = narrow || wide ? 128 : 64, slice = async ? (ks == 3 ? 36 : 32) : conv_slice(ks);
     int parts = 1;
-    while (parts < 8 && tiles(bm, bn) * parts * 2 <= (wide ? 4ll : 8ll) * ctx->sm_count && p.K / (parts * 2) >= (async ? 2 : 4) * slice) parts *= 2;
+    while (!one_chain && parts < 8 && tiles(bm, bn) * parts * 2 <= (wide ? 4ll : 8ll) * ctx->sm_count && p.K / (parts * 2) >= (async ? 2 : 4) * slice) parts *= 2;
     p.k_part = (int)ln_round_up((p.K + parts - 1) / parts, slice);
     const dim3 grid((unsigned)((NP + bn - 1) / bn), (unsigned)((p.F + bm - 1) / bm), (unsigned)parts);
     cudaError_t e;
@@ -680,7 +682,7 @@ int32_t ln_conv2d_f32(ln_ctx* ctx, const ln_tensor* x, const ln_tensor* weights,
                       int64_t input_channels, int64_t input_height, int64_t input_width, int64_t filters, int64_t kernel_size,
                       int64_t stride_x, int64_t stride_y, int64_t dilation, int64_t padding, int64_t groups, ln_tensor** out) {
     return ln_conv2d_bias_act_f32(ctx, x, weights, nullptr, output_shape, input_channels, input_height, input_width, filters, kernel_size, stride_x, stride_y, dilation,
-                                  padding, groups, LN_ACT_LINEAR, out);
+                                  padding, groups, LN_ACT_LINEAR, false, out);
 }
 
 }  // extern "C"
@@ -688,7 +690,7 @@ int32_t ln_conv2d_f32(ln_ctx* ctx, const ln_tensor* x, const ln_tensor* weights,
 // conv2d_f32 followed by bias_activation_f32 (bias may be null) without the pass over memory between them
 int ln_conv2d_bias_act_f32(ln_ctx* ctx, const ln_tensor* x, const ln_tensor* weights, const ln_tensor* bias, const int64_t output_shape[4], int64_t input_channels,
                            int64_t input_height, int64_t input_width, int64_t filters, int64_t kernel_size, int64_t stride_x, int64_t stride_y, int64_t dilation,
-                           int64_t padding, int64_t groups, int activation, ln_tensor** out) {
+                           int64_t padding, int64_t groups, int activation, bool one_chain, ln_tensor** out) {
     if (!ctx || !out || !output_shape) return ln_fail(ctx, LN_ERR_ARG, "ln_conv2d_f32: NULL argument");
     if (!is_f32(x) || !is_f32(weights)) return ln_fail(ctx, LN_ERR_ARG, "ln_conv2d_f32: f32 tensors required");
     if (groups < 1 || filters % groups || input_channels % groups || kernel_size < 1 || stride_x < 1 || stride_y < 1 || dilation < 1)
@@ -720,7 +722,7 @@ int ln_conv2d_bias_act_f32(ln_ctx* ctx, const ln_tensor* x, const ln_tensor* wei
         p.sx = (int)stride_x; p.sy = (int)stride_y; p.dil = (int)dilation; p.pad = (int)padding; p.OH = (int)oh; p.OW = (int)ow;
         p.K = (int)(input_channels * kernel_size * kernel_size);
         p.act = activation;
-        rc = conv_f32_run(ctx, p, "conv2d_f32");
+        rc = conv_f32_run(ctx, p, one_chain, "conv2d_f32");
     } else {
         int64_t total = x->n * ((filters + 3) / 4) * oh * ow;
         conv2d_f32_kernel<4><<<grid_for(ctx, total), kThreads, 0, ctx->stream>>>(

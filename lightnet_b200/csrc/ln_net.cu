@@ -472,7 +472,7 @@ int forward_f32(ln_net* net, const ln_tensor* input, unsigned* amax_dev) {
         switch (L.kind) {
             case K_CONV: {  // layers/convolutional/gpu.rs:138-209: conv2d_f32_with_precision + bias_activation_f32
                 rc = ln_conv2d_bias_act_f32(ctx, x, L.w_f32, L.b_f32, oshape, L.in.c, L.in.h, L.in.w, L.filters, L.size, L.stride_x, L.stride_y, L.dilation, L.padding,
-                                            L.groups, L.act, &y);
+                                            L.groups, L.act, amax_dev != nullptr, &y);
                 break;
             }
             case K_MAXPOOL:  // layers/pool/gpu.rs:13-42

@@ -44,3 +44,17 @@ def test_conv2d_f32_tiles(be, geom):
     size = torch.nn.functional.conv2d(xd.abs(), wd.abs(), stride=s, dilation=dil)[:, :, :oh, :ow].numpy()
     # one rounding of 2^-24 per term of the chain, at most C k^2 of them and the sums over the parts of a split range
     assert (np.abs(got - ref) <= (C * k * k + 33) * 2.0 ** -24 * size).all()
+
+
+def test_calibrated_scales_do_not_depend_on_the_batch(be):
+    """One image, alone and eight times in a batch: the f32 convolutions cut their work differently, the scales stay bit for bit."""
+    import lightnet_b200 as ln
+    from lightnet_b200 import synth, zoo
+    x = synth.uniform_images(1, 3, 96, 160, 5)
+    scales = []
+    for batch in (1, 8):
+        net = ln.GpuExecutableNetwork(be, zoo.yolov3_tiny_cfg(160, 96), batch, ln.LN_Q8)
+        net.load_weights(synth.he_weights(net.layers(), 3))
+        net.calibrate(np.repeat(x, batch, 0))
+        scales.append(np.asarray(net.scales()))
+    np.testing.assert_array_equal(scales[0], scales[1])
