@@ -56,6 +56,10 @@ struct ln_conv_umma_params {
     // TW x (TH + 2) pixels, shifted by 0, 1, 2 pixels in x; the tap (r, s) reads box s from row r on.  a_stages such sets
     // are in flight; the weight tiles have their own ring (`stages`) unless they are resident.
     int halo, a_stages, box_bytes;
+    // Small grids (conv_umma_small_kernel): CTAs of one cluster that share a tile's k range (1, 2, 4 or 8; 0 = the persistent kernel),
+    // bytes of the ring of stages or of the tile's partial sums, whichever is larger, and whether weights and table may be read
+    // before the kernel in front of this one has finished (they were complete before it started)
+    int ksplit, small_region, early;
     int* status;
     long long* debug;  // optional: role timing of CTA 0 (32 counters), null = off
 };
@@ -71,6 +75,7 @@ struct ln_conv_umma_plan {
     size_t smem = 0;
     int grid = 0;
     int kind = LN_KIND_I8;
+    bool chained = false;  // launched as a programmatic dependent of the kernel in front of it (plans of a network)
 };
 
 // Geometry of one convolution as the planners see it.
@@ -110,6 +115,28 @@ inline int ln_conv_choose_bn(int64_t F) {
         if (best < 0 || fp <= best) { best = fp; bn = c; }
     }
     return bn;
+}
+
+// Filter tile and k split of the small-grid kernel for a layer of m pixel tiles; false: the layer is left to the persistent kernel.
+// A layer qualifies when some choice needs no more CTAs than fit the GPU at once, two per SM (beyond that the persistent kernel, which
+// overlaps epilogue and main loop, is the better one).  Among the choices the one with the shortest chain is taken, in cycles:
+// 180 per tensor instruction with its loads (half as much again where two CTAs share an SM), 1000 per piece of epilogue that a warp
+// does, 9000 for the exchange of partial sums with its two cluster barriers.  (YOLOv4 608 x 608 int8, one image, forward: 837 us with
+// 4000 for the exchange, 796 with 6500, 791 with 9000, 802 without any split.)  FP8 is not split: its codes would depend on the order of
+// the sum.
+inline bool ln_conv_choose_small(int sm_count, int kind, int64_t m, int64_t F, int64_t fpad, int kblocks, int bk, int* bn_out, int* ks_out) {
+    int64_t best = -1;
+    for (int bn = 32; bn <= 128; bn *= 2) {
+        if (fpad % bn != 0 || (bn > 32 && ln_round_up(F, 32) < bn)) continue;
+        const int64_t tiles = m * ((F + bn - 1) / bn);
+        for (int ks = 1; ks <= (kind == LN_KIND_F8 ? 1 : 8); ks *= 2) {
+            if (tiles * ks > 2 * sm_count || ks > kblocks || ks > bn / 8) break;
+            const int64_t instructions = (int64_t)((kblocks + ks - 1) / ks) * (bk / 32), rounds = (bn / 8 + ks * 8 - 1) / (ks * 8);
+            const int64_t cost = instructions * 180 * (tiles * ks > sm_count ? 3 : 2) / 2 + rounds * 1000 + (ks > 1 ? 9000 : 0);
+            if (best < 0 || cost < best) { best = cost; *bn_out = bn; *ks_out = ks; }
+        }
+    }
+    return best >= 0;
 }
 
 bool ln_conv_umma_supported(int64_t channels_padded, int64_t k, int64_t stride_x, int64_t stride_y, int64_t dilation, int64_t groups,

@@ -514,209 +514,7 @@ __device__ __forceinline__ void conv_epilogue_role(const ln_conv_umma_params& p)
             uint32_t acc[32];
             const long long tq0 = kRoleTiming && p.debug ? clock64() : 0;
             tmem_ld_32x32(taddr0 + (uint32_t)c0, acc);
-            const bool fast = KIND == LN_KIND_I8 && p.out_kind == LN_OUT_Q && f0 + c0 + 32 <= p.F;
-            // where this chunk goes: with pixel-group packing the columns [j * f_real, (j + 1) * f_real) are the filters of the
-            // j-th pixel of the row's group (f_real is a multiple of 32 then, so a chunk never straddles two pixels)
-            int64_t opix = pix;
-            int fo = f0 + c0;
-            if (p.pack > 1) {
-                int j = 0;
-                while (fo >= p.f_real) { fo -= p.f_real; ++j; }
-                opix = pix * p.pack + j;
-            }
-            if (fast) {
-                // ---- fast path: 32 valid filters, int8 out.  The {mult, bias} pairs (two per 16-byte load) are fetched
-                // while the TMEM load is in flight, so the arithmetic below runs from registers only.
-                const uint32_t mtab = tab_base + 8u * (uint32_t)(f0 + c0);
-                uint4 r0 = make_uint4(0u, 0u, 0u, 0u), r1 = r0;
-                if (p.res != nullptr && valid) {  // residual codes of the fused shortcut, fetched while TMEM is read
-                    const uint4* rp = (const uint4*)((const uint8_t*)p.res + opix * p.res_pixel_stride + fo);
-                    r0 = __ldg(rp);
-                    r1 = __ldg(rp + 1);
-                }
-                tmem_ld_wait();
-                const long long tq1 = kRoleTiming && p.debug ? clock64() : 0;
-                if (kRoleTiming && p.debug) dbg_ld += tq1 - tq0;
-                if (!valid) continue;
-                uint32_t packed[8];
-                // Four values at a time, each loop body fetching its own two table entries from shared memory, so that few
-                // values are live at once (the kernel has to fit in 96 registers).
-                if (folded) {
-                    // Fast mode, accumulators below 2^22.  Adding an accumulator to the bits of 1.5 * 2^23 gives the float
-                    // 1.5 * 2^23 + accumulator; the table holds {mult 2i, mult 2i+1, bias 2i, bias 2i+1} divided by the output scale,
-                    // the bias carrying -1.5 * 2^23 * mult, so one packed FMA yields two pre-activations in code units;
-                    // activation and rounding run in packed binary16.
-                    // Accumulators that may reach 2^22 lose their low p.acc_shift bits first (the table carries the larger
-                    // multiplier and the mean of what is dropped); the planner allows that only where it moves a
-                    // pre-activation by no more than 0.02 of a code.
-                    const __half2 kh = __float2half2_rn(p.sy_log2e), inv_h = __float2half2_rn(p.inv_sy);
-                    const int sh = p.acc_shift;
-                    if (sh == 0) {
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const float4 ma = lds_f4(mtab + 32u * j), mc = lds_f4(mtab + 32u * j + 16u);
-                            float t0, t1, t2, t3;
-                            ffma2(t0, t1, __int_as_float(0x4B400000 + (int)acc[4 * j]), __int_as_float(0x4B400000 + (int)acc[4 * j + 1]), ma.x, ma.y, ma.z, ma.w);
-                            ffma2(t2, t3, __int_as_float(0x4B400000 + (int)acc[4 * j + 2]), __int_as_float(0x4B400000 + (int)acc[4 * j + 3]), mc.x, mc.y, mc.z, mc.w);
-                            packed[j] = ln_h2_pack(ln_h2_code<ACT>(t0, t1, kh, inv_h), ln_h2_code<ACT>(t2, t3, kh, inv_h));
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const float4 ma = lds_f4(mtab + 32u * j), mc = lds_f4(mtab + 32u * j + 16u);
-                            float t0, t1, t2, t3;
-                            ffma2(t0, t1, __int_as_float(0x4B400000 + ((int)acc[4 * j] >> sh)), __int_as_float(0x4B400000 + ((int)acc[4 * j + 1] >> sh)), ma.x, ma.y, ma.z, ma.w);
-                            ffma2(t2, t3, __int_as_float(0x4B400000 + ((int)acc[4 * j + 2] >> sh)), __int_as_float(0x4B400000 + ((int)acc[4 * j + 3] >> sh)), mc.x, mc.y, mc.z, mc.w);
-                            packed[j] = ln_h2_pack(ln_h2_code<ACT>(t0, t1, kh, inv_h), ln_h2_code<ACT>(t2, t3, kh, inv_h));
-                        }
-                    }
-                } else {
-                    // int32 -> f32: below 2^22 through the bits of 1.5 * 2^23 (two FMA-pipe instructions, exact); otherwise the
-                    // conversion unit, or, for the transcendental epilogues that need that unit for ex2 / rcp, an exact ALU sequence
-                    const bool small = p.small_acc != 0;
-                    const __half2 inv_h = __float2half2_rn(p.inv_sy);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const float4 ma = lds_f4(mtab + 32u * j), mc = lds_f4(mtab + 32u * j + 16u);
-                        float x[4];
-#pragma unroll
-                        for (int b = 0; b < 4; ++b) {
-                            const int a = (int)acc[4 * j + b];
-                            x[b] = small ? __fadd_rn(__int_as_float(0x4B400000 + a), -12582912.0f) : (kTranscendental ? i2f_alu(a) : __int2float_rn(a));
-                        }
-                        const float v0 = __fmaf_rn(x[0], ma.x, ma.y), v1 = __fmaf_rn(x[1], ma.z, ma.w), v2 = __fmaf_rn(x[2], mc.x, mc.y), v3 = __fmaf_rn(x[3], mc.z, mc.w);
-                        if (EXACT)
-                            packed[j] = pack4_low_bytes(quant_i8_magic(ln_epilogue_act<true>(ACT, v0), p.inv_sy), quant_i8_magic(ln_epilogue_act<true>(ACT, v1), p.inv_sy),
-                                                        quant_i8_magic(ln_epilogue_act<true>(ACT, v2), p.inv_sy), quant_i8_magic(ln_epilogue_act<true>(ACT, v3), p.inv_sy));
-                        else
-                            packed[j] = ln_h2_pack(ln_h2_act_quant<ACT>(v0, v1, inv_h), ln_h2_act_quant<ACT>(v2, v3, inv_h));
-                    }
-                }
-                if (p.res != nullptr) {
-                    // fused shortcut, the arithmetic of the stand-alone shortcut kernel applied to the codes just produced
-                    const uint32_t rw[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
-                    // (two values per instruction where the packed f32x2 forms exist: every product, sum and fma rounds exactly
-                    // like its scalar twin, so the codes are those of the stand-alone kernel)
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        float c[4], r[4], v[4];
-                        s8x4_to_float(packed[j], c);
-                        s8x4_to_float(rw[j], r);
-                        uint32_t u[4];
-#pragma unroll
-                        for (int b = 0; b < 4; b += 2) {
-                            fmul2(v[b], v[b + 1], c[b], c[b + 1], p.s_c, p.s_c);
-                            ffma2(v[b], v[b + 1], r[b], r[b + 1], p.s_res, p.s_res, v[b], v[b + 1]);
-                            fmul2(v[b], v[b + 1], v[b], v[b + 1], p.inv_sy2, p.inv_sy2);
-                            v[b] = fminf(fmaxf(v[b], -127.0f), 127.0f);  // NaN -> -127, as in quant_i8_magic
-                            v[b + 1] = fminf(fmaxf(v[b + 1], -127.0f), 127.0f);
-                            fadd2(v[b], v[b + 1], v[b], v[b + 1], 12582912.0f, 12582912.0f);
-                            u[b] = __float_as_uint(v[b]);
-                            u[b + 1] = __float_as_uint(v[b + 1]);
-                        }
-                        packed[j] = pack4_low_bytes(u[0], u[1], u[2], u[3]);
-                    }
-                }
-                const long long tq2 = kRoleTiming && p.debug ? clock64() : 0;
-                uint4* o = (uint4*)((uint8_t*)p.out + opix * p.out_pixel_stride + fo);
-                o[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                o[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-                if (kRoleTiming && p.debug) { dbg_math += tq2 - tq1; dbg_st += clock64() - tq2; }
-                continue;
-            }
-            if (KIND == LN_KIND_F8 && folded && p.out_kind == LN_OUT_Q) {
-                // ---- FP8 fast path (the planner folds only when every chunk has its 32 filters): pre-activations in units of the
-                // output scale by one packed fma on the binary32 accumulators, activation in packed binary16, two E4M3 codes
-                // per conversion
-                const uint32_t mtab = tab_base + 8u * (uint32_t)(f0 + c0);
-                tmem_ld_wait();
-                if (!valid) continue;
-                const __half2 kh = __float2half2_rn(p.sy_log2e), inv_h = __float2half2_rn(p.inv_sy);
-                uint32_t packed[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const float4 ma = lds_f4(mtab + 32u * j), mc = lds_f4(mtab + 32u * j + 16u);
-                    float t0, t1, t2, t3;
-                    ffma2(t0, t1, __uint_as_float(acc[4 * j]), __uint_as_float(acc[4 * j + 1]), ma.x, ma.y, ma.z, ma.w);
-                    ffma2(t2, t3, __uint_as_float(acc[4 * j + 2]), __uint_as_float(acc[4 * j + 3]), mc.x, mc.y, mc.z, mc.w);
-                    packed[j] = ln_h2_to_e4m3x2(ln_h2_value<ACT>(t0, t1, kh, inv_h)) | (ln_h2_to_e4m3x2(ln_h2_value<ACT>(t2, t3, kh, inv_h)) << 16);
-                }
-                uint4* o = (uint4*)((uint8_t*)p.out + opix * p.out_pixel_stride + fo);
-                o[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                o[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-                continue;
-            }
-            // ---- general path: f32 / raw-accumulator outputs (NCHW), FP8, and int8 chunks with fewer than 32 real filters.
-            // The {mult, bias} pairs come two per 16-byte load (the table is padded to a multiple of 32 filters).
-            const int nf = p.F - (f0 + c0);  // real filters from this chunk's first column on (32 or more: all of the chunk)
-            tmem_ld_wait();
-            if (!valid || nf <= 0) continue;
-            if (p.out_kind == LN_OUT_ACC) {
-                // NCHW, raw accumulator bits (int32 or f32): consecutive lanes are consecutive pixels of a row, one plane per filter
-                const int64_t plane = (int64_t)p.OH * p.OW;
-                int32_t* o = (int32_t*)p.out + ((int64_t)n * p.F + (f0 + c0)) * plane + (int64_t)oh * p.OW + ow;
-#pragma unroll
-                for (int j = 0; j < 32; ++j, o += plane)
-                    if (j < nf) *o = (int32_t)acc[j];
-                continue;
-            }
-            float a[32];
-            const uint32_t mtab = tab_base + 8u * (uint32_t)(f0 + c0);  // (never the folded table: that one needs int8 output and full chunks)
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const float4 mj = lds_f4(mtab + 16u * j);
-                const float x0 = KIND == LN_KIND_I8 ? __int2float_rn((int)acc[2 * j]) : __uint_as_float(acc[2 * j]);
-                const float x1 = KIND == LN_KIND_I8 ? __int2float_rn((int)acc[2 * j + 1]) : __uint_as_float(acc[2 * j + 1]);
-                a[2 * j] = ln_epilogue_act<EXACT>(ACT, __fmaf_rn(x0, mj.x, mj.y));
-                a[2 * j + 1] = ln_epilogue_act<EXACT>(ACT, __fmaf_rn(x1, mj.z, mj.w));
-            }
-            if (p.out_kind == LN_OUT_F32) {
-                const int64_t plane = (int64_t)p.OH * p.OW;
-                float* o = (float*)p.out + ((int64_t)n * p.F + (f0 + c0)) * plane + (int64_t)oh * p.OW + ow;  // NCHW
-#pragma unroll
-                for (int j = 0; j < 32; ++j, o += plane)
-                    if (j < nf) *o = a[j];
-            } else {
-                if (KIND == LN_KIND_F16) {
-                    // binary16 NHWC: 32 filters = 64 bytes per pixel, rounded to nearest even, infinities kept
-                    uint32_t hw[16];
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const __half2 h = __floats2half2_rn(2 * j < nf ? a[2 * j] : 0.0f, 2 * j + 1 < nf ? a[2 * j + 1] : 0.0f);
-                        hw[j] = *reinterpret_cast<const uint32_t*>(&h);
-                    }
-                    uint4* o = (uint4*)((uint8_t*)p.out + opix * p.out_pixel_stride + 2 * fo);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) o[j] = make_uint4(hw[4 * j], hw[4 * j + 1], hw[4 * j + 2], hw[4 * j + 3]);
-                    continue;
-                }
-                uint32_t packed[8];
-                if (KIND == LN_KIND_I8) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        uint32_t v = 0;
-#pragma unroll
-                        for (int b = 0; b < 4; ++b) {
-                            const int q = 4 * j + b < nf ? ln_quant_i8(a[4 * j + b], p.inv_sy) : 0;
-                            v |= ((uint32_t)q & 0xFFu) << (8 * b);
-                        }
-                        packed[j] = v;
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a[4 * j] * p.inv_sy, a[4 * j + 1] * p.inv_sy), __NV_SATFINITE, __NV_E4M3);
-                        const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(a[4 * j + 2] * p.inv_sy, a[4 * j + 3] * p.inv_sy), __NV_SATFINITE, __NV_E4M3);
-                        uint32_t w = lo | (hi << 16);
-                        const int left = nf - 4 * j;  // codes of filters that do not exist are zero
-                        if (left < 4) w = left <= 0 ? 0u : (w & (0xFFFFFFFFu >> (8 * (4 - left))));
-                        packed[j] = w;
-                    }
-                }
-                uint4* o = (uint4*)((uint8_t*)p.out + opix * p.out_pixel_stride + fo);
-                o[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                o[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-            }
+#include "ln_conv_chunk.inc"
         }
         tc_fence_before();
         __syncwarp();
@@ -787,6 +585,222 @@ __global__ void __launch_bounds__(conv_threads(PIPES), 1) conv_umma_kernel(const
 
 #undef LN_FIRST_UNIT
 #undef LN_UNIT_STEP
+
+// Small grids: layers whose tiles do not fill the GPU (a few images, or the 19 x 19 end of a network).  What bounds such a launch is
+// not a rate but one chain: launch, fill of the pipeline, the k loop of a single tile (about 180 cycles per instruction with its loads,
+// whatever its size), epilogue, exit.  So
+//   - filter tiles of 32 to 128 columns and, int8 and binary16, a long k range split over the CTAs of a cluster (see ln_conv_choose_small).  Each
+//     CTA leaves its partial accumulators in its own shared memory as pieces of 32 rows x 32 columns; piece i belongs to the CTA of rank
+//     i % ksplit, which adds the parts up through distributed shared memory -- int32 sums, the same bits in any order; binary32 sums in rank
+//     order -- and runs the epilogue on it.  FP8 keeps one chain per output, so its codes do not change.
+//   - 320 threads, bn columns of TMEM and at most 112 KB of shared memory: two CTAs fit an SM, so that in a network (plan.chained)
+//     the next layer's CTAs can set up, fetch their table and start their weight loads while this layer still runs; griddepcontrol.wait
+//     stands in front of everything that the layers before it write or still read.
+// One tile per CTA, no persistent loop.
+// YOLOv4 608 x 608 int8, one image: 102 layers, forward 1254 -> 791 us (957 without programmatic launches, 802 without the k split); 1x1
+// C512 -> K256 at 38 x 38 9.5 -> 7.5 us, 3x3 C512 -> K1024 at 19 x 19 25 -> 15 us as single cold launches.
+constexpr int kSmallEpilogueWarps = 8;
+constexpr int kSmallThreads = 32 * (2 + kSmallEpilogueWarps);
+constexpr uint32_t kSmallBarBytes = 160u;  // full[8] empty[8] done | tmem slot | abort flag
+constexpr uint32_t kPieceBytes = 4096u;    // 32 rows x 32 columns of partial sums, [4 columns][row]: consecutive lanes, consecutive 16 bytes
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
+template <int KIND, int ACT, bool EXACT>
+__global__ void __launch_bounds__(kSmallThreads, 2) conv_umma_small_kernel(const __grid_constant__ ln_conv_umma_params p) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* generic_base = smem_raw + (smem_base - smem_u32(smem_raw));
+    const int bk = p.bk, bn = p.bn, stages = p.stages, ks = p.ksplit;
+    const uint32_t a_bytes = 128u * bk, stage_bytes = a_bytes + (uint32_t)bn * bk;
+    const uint32_t bar_base = smem_base + (uint32_t)p.small_region;
+    auto full_bar = [&](int s) { return bar_base + 8u * s; };
+    auto empty_bar = [&](int s) { return bar_base + 8u * (kMaxStages + s); };
+    const uint32_t done_bar = bar_base + 16u * kMaxStages;
+    volatile uint32_t* tmem_slot = (volatile uint32_t*)(generic_base + p.small_region + 16 * kMaxStages + 8);
+    volatile int* abort_flag = (volatile int*)(tmem_slot + 2);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = ks > 1 ? (int)cluster_ctarank() : 0, tile = (int)blockIdx.x / ks;
+    const int q1 = fast_div(tile, p.magic_f), tf = tile - q1 * p.tiles_f;
+    const int q2 = fast_div(q1, p.magic_w), tw = q1 - q2 * p.tiles_w;
+    const int tn = fast_div(q2, p.magic_h), th = q2 - tn * p.tiles_h;
+    const int ow0 = tw * p.TW, oh0 = th * p.TH, n0 = tn * p.TN, f0 = tf * bn;
+    const int kblocks = p.R * p.S * p.cblocks;
+    const int kb0 = kblocks * rank / ks, nkb = kblocks * (rank + 1) / ks - kb0;  // this CTA's k-blocks (at least one: ks <= kblocks)
+    const bool folded = !EXACT && p.mb_folded != nullptr;
+    const uint32_t tab_base = bar_base + kSmallBarBytes - 8u * (uint32_t)f0;  // where filter 0 would be: the table holds this tile's filters only
+
+    if (threadIdx.x == 0) {
+        for (int m = 0; m < (p.stride == 2 ? 4 : 1); ++m) asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tmA[m]) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tmB) : "memory");
+        for (int s = 0; s < stages; ++s) {
+            mbar_init(full_bar(s), 1);
+            mbar_init(empty_bar(s), 1);
+        }
+        mbar_init(done_bar, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)), "r"((uint32_t)bn) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (!p.early) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (warp >= 2) {
+        const uint4* src = reinterpret_cast<const uint4*>((folded ? p.mb_folded : p.mb) + f0);
+        const int i = (int)threadIdx.x - 64;
+        if (i < bn / 2) {
+            const uint4 v = __ldg(src + i);
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(bar_base + kSmallBarBytes + 16u * (uint32_t)i), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            // weights of the first stages, then (they come from the layer before) the activations
+            const int pre = nkb < stages ? nkb : stages;
+            for (int i = 0; i < pre; ++i) {
+                mbar_arrive_expect_tx(full_bar(i), stage_bytes);
+                tma_load_2d(smem_base + (uint32_t)i * stage_bytes + a_bytes, &p.tmB, (kb0 + i) * bk, f0, full_bar(i));
+            }
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+            const int tap0 = kb0 / p.cblocks;
+            int r = tap0 / p.S, s = tap0 - r * p.S, cb = kb0 - tap0 * p.cblocks, stage = 0;
+            uint32_t phase = 0;
+            for (int i = 0; i < nkb; ++i) {
+                const uint32_t sa = smem_base + (uint32_t)stage * stage_bytes;
+                if (i >= stages) {
+                    if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status, LN_STATUS_PRODUCER_TIMEOUT)) break;
+                    mbar_arrive_expect_tx(full_bar(stage), stage_bytes);
+                    tma_load_2d(sa + a_bytes, &p.tmB, (kb0 + i) * bk, f0, full_bar(stage));
+                }
+                int ty = r - p.pad, tx = s - p.pad, map = 0;
+                if (p.stride == 2) {
+                    const int py = ty & 1, px = tx & 1;  // parity class of the tap (two's complement & 1 is non-negative)
+                    ty = (ty - py) >> 1;
+                    tx = (tx - px) >> 1;
+                    map = py * 2 + px;
+                }
+                tma_load_4d(sa, &p.tmA[map], cb * bk, ow0 + tx, oh0 + ty, n0, full_bar(stage));
+                if (++stage == stages) { stage = 0; phase ^= 1u; }
+                if (++cb == p.cblocks) {
+                    cb = 0;
+                    if (++s == p.S) { s = 0; ++r; }
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = (KIND == LN_KIND_I8 ? ((2u << 4) | (1u << 7) | (1u << 10)) : (1u << 4)) | ((uint32_t)(bn >> 3) << 17) | ((128u >> 4) << 24);
+            const uint64_t desc_base = make_smem_desc(0u, bk);
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            int stage = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int i = 0; i < nkb; ++i) {
+                if (!(ok = mbar_wait(full_bar(stage), phase, abort_flag, p.status, LN_STATUS_MMA_TIMEOUT))) break;
+                const uint32_t sa = smem_base + (uint32_t)stage * stage_bytes;
+                const uint64_t a_desc = desc_base + (sa >> 4), b_desc = desc_base + ((sa + a_bytes) >> 4);
+                tc_mma<KIND>(tmem_base, a_desc, b_desc, idesc, (uint32_t)(i != 0));
+                if (bk >= 64) tc_mma<KIND>(tmem_base, a_desc + 2u, b_desc + 2u, idesc, 1u);
+                if (bk == 128) {
+                    tc_mma<KIND>(tmem_base, a_desc + 4u, b_desc + 4u, idesc, 1u);
+                    tc_mma<KIND>(tmem_base, a_desc + 6u, b_desc + 6u, idesc, 1u);
+                }
+                tc_commit(empty_bar(stage));
+                if (++stage == stages) { stage = 0; phase ^= 1u; }
+            }
+            if (ok) tc_commit(done_bar);
+        }
+        __syncwarp();
+    } else {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
+
+    constexpr bool kTranscendental = ACT == LN_ACT_MISH || ACT == LN_ACT_SWISH || ACT == LN_ACT_LOGISTIC;
+    const int pieces = bn / 8;  // quadrant + 4 * chunk of 32 columns
+    bool ok = true;
+    if (warp >= 2) {
+        ok = mbar_wait(done_bar, 0u, abort_flag, p.status, LN_STATUS_EPILOGUE_TIMEOUT);
+        tc_fence_after();
+        if (ks > 1 && ok) {
+            // all MMAs have finished, so have the loads they read: the ring is free for the partial sums
+            const int quad = warp & 3;  // the TMEM lanes this warp may read
+            for (int c = (warp - 2) >> 2; c < bn / 32; c += kSmallEpilogueWarps / 4) {
+                uint32_t acc[32];
+                tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * 32), acc);
+                tmem_ld_wait();
+                const uint32_t dst = smem_base + (uint32_t)(c * 4 + quad) * kPieceBytes + 16u * (uint32_t)lane;
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + 512u * j), "r"(acc[4 * j]), "r"(acc[4 * j + 1]), "r"(acc[4 * j + 2]), "r"(acc[4 * j + 3]) : "memory");
+            }
+        }
+    }
+    if (ks > 1) {
+        cluster_arrive();
+        cluster_wait();
+        if (warp >= 2) {
+            const int own = pieces / ks, t = (int)threadIdx.x - 64;
+            for (int i = 0; i < own; ++i) {
+                const uint32_t at = smem_base + (uint32_t)(rank + ks * i) * kPieceBytes + 16u * (uint32_t)t;
+                uint32_t sum[4] = {0u, 0u, 0u, 0u};
+#pragma unroll 8
+                for (int k = 0; k < ks; ++k) {
+                    uint32_t part, v[4];
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(part) : "r"(at), "r"(k));
+                    asm volatile("ld.shared::cluster.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(part) : "memory");
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) sum[j] = KIND == LN_KIND_I8 ? sum[j] + v[j] : __float_as_uint(__uint_as_float(sum[j]) + __uint_as_float(v[j]));
+                }
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(sum[0]), "r"(sum[1]), "r"(sum[2]), "r"(sum[3]) : "memory");
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * kSmallEpilogueWarps) : "memory");
+        }
+        cluster_arrive();  // nobody leaves while its partial sums are being read: the wait is at the end
+    }
+    if (warp >= 2 && ok) {
+        const long long tq0 = 0;
+        long long dbg_ld = 0, dbg_math = 0, dbg_st = 0;
+        // one CTA: the warps of a quadrant take its chunks in turn; several: the pieces of this rank
+        for (int piece = ks > 1 ? rank + ks * (warp - 2) : (warp & 3) + 4 * ((warp - 2) >> 2); piece < pieces; piece += ks * kSmallEpilogueWarps) {
+            const int quad = piece & 3, c0 = (piece >> 2) * 32, row = quad * 32 + lane;
+            const int ow = ow0 + (row & (p.TW - 1)), oh = oh0 + ((row >> p.log_tw) & (p.TH - 1)), n = n0 + (row >> (p.log_tw + p.log_th));
+            const bool valid = ow < p.OW && oh < p.OH && n < p.N;
+            const int64_t pix = ((int64_t)n * p.OH + oh) * p.OW + ow;
+            uint32_t acc[32];
+            if (ks == 1) tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, acc);
+            else {
+                const uint32_t src = smem_base + (uint32_t)piece * kPieceBytes + 16u * (uint32_t)lane;
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(acc[4 * j]), "=r"(acc[4 * j + 1]), "=r"(acc[4 * j + 2]), "=r"(acc[4 * j + 3]) : "r"(src + 512u * j) : "memory");
+            }
+#include "ln_conv_chunk.inc"
+        }
+        (void)tq0; (void)dbg_ld; (void)dbg_math; (void)dbg_st;
+    }
+
+    tc_fence_before();
+    if (ks > 1) cluster_wait();
+    __syncthreads();
+    if (*abort_flag && warp == 0 && lane == 0) {
+        // a wait was abandoned: give copies that may still be in flight time to land before the shared memory is handed on
+        for (int i = 0; i < 64; ++i) __nanosleep(20000);
+    }
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)bn) : "memory");
+    }
+}
 
 // Tensor-pipe peak probe: one CTA per SM, one thread issuing tcgen05.mma (M = 128, N = n, 32 bytes of K per instruction)
 // back to back on operand tiles that stay in shared memory, no loads, no epilogue.  What it measures is the rate the tensor
@@ -864,6 +878,7 @@ __global__ void __launch_bounds__(128, 1) mma_peak_kernel(int iters, int n, int 
 }
 
 constexpr int kMaxDynamicSmem = 227 * 1024;
+constexpr uint32_t kSmallSmem = 112u * 1024u;     // of a CTA of the small-grid kernel: two fit an SM
 constexpr uint32_t kMaxTableBytes = 32u * 1024u;  // {multiplier, bias} pairs of at most 4096 filters
 
 template <int KIND, bool EXACT, int PIPES>
@@ -878,6 +893,45 @@ cudaError_t launch_act(ln_ctx* ctx, const ln_conv_umma_params& p, int grid, size
         }                                                                                                            \
         k<<<grid, conv_threads(PIPES), smem, stream>>>(p);                                                                           \
         return cudaGetLastError();                                                                                   \
+    }
+    switch (p.act) {
+        LN_LAUNCH_ACT(LN_ACT_LINEAR)
+        LN_LAUNCH_ACT(LN_ACT_LOGISTIC)
+        LN_LAUNCH_ACT(LN_ACT_LEAKY)
+        LN_LAUNCH_ACT(LN_ACT_MISH)
+        LN_LAUNCH_ACT(LN_ACT_SWISH)
+        LN_LAUNCH_ACT(LN_ACT_RELU)
+    }
+#undef LN_LAUNCH_ACT
+    return cudaErrorInvalidValue;
+}
+
+template <int KIND, bool EXACT>
+cudaError_t launch_small(ln_ctx* ctx, const ln_conv_umma_plan& plan) {
+    const ln_conv_umma_params& p = plan.p;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)plan.grid);
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.dynamicSmemBytes = plan.smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)p.ksplit;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = plan.chained ? 2 : 1;
+#define LN_LAUNCH_ACT(A)                                                                                             \
+    case A: {                                                                                                        \
+        auto k = conv_umma_small_kernel<KIND, A, EXACT>;                                                              \
+        if (!ctx->configured_kernels.count((const void*)k)) { /* once per kernel per context */                      \
+            cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);   \
+            if (e != cudaSuccess) return e;                                                                          \
+            ctx->configured_kernels.insert((const void*)k);                                                          \
+        }                                                                                                            \
+        return cudaLaunchKernelEx(&cfg, k, p);                                                                       \
     }
     switch (p.act) {
         LN_LAUNCH_ACT(LN_ACT_LINEAR)
@@ -1015,10 +1069,10 @@ int ln_conv_umma_plan_build(ln_ctx* ctx, ln_conv_umma_plan* plan, const ln_conv_
     ln_conv_geom g = g_in;
     float2* mb = plan->mb;
     int pack = 1;
-    // LN_CONV_DISABLE=pack,halo switches the two layout modes off (for A/B measurements)
+    // LN_CONV_DISABLE=pack,halo,resident,small switches the modes off (for A/B measurements)
     const char* disable = getenv("LN_CONV_DISABLE");
     const bool allow_pack = !(disable && strstr(disable, "pack")), allow_halo = !(disable && strstr(disable, "halo"));
-    const bool allow_resident = !(disable && strstr(disable, "resident"));
+    const bool allow_resident = !(disable && strstr(disable, "resident")), allow_small = !(disable && strstr(disable, "small"));
     const char* rms = getenv("LN_CONV_RESIDENT_MIN_STAGES");
     const uint32_t res_min_stages = rms && atoi(rms) >= 2 ? (uint32_t)atoi(rms) : 4u;
     // Space-to-depth input (see ln_conv_geom::s2d_input): 4 taps of 128-byte rows instead of 9 taps of 32-byte rows.
@@ -1107,6 +1161,15 @@ int ln_conv_umma_plan_build(ln_ctx* ctx, ln_conv_umma_plan* plan, const ln_conv_
         const int v = atoi(e);
         if ((v == 128 || v == 64) && v < bn && g.fpad % v == 0) bn = v;
     }
+    // Small grids: a kernel of their own.  (FP8 layers that the row-shifted boxes below could take stay with the persistent kernel: those
+    // sum the taps in another order, which would change codes.)
+    int box_w = 0, box_h = 0, box_n = 0, ksplit = 0, small_bn = 0;
+    choose_box(g.OW, g.OH, g.N, g.out_kind != LN_OUT_Q, &box_w, &box_h, &box_n);
+    const bool box_order = g.kind == LN_KIND_F8 && g.k == 3 && g.stride == 1 && pack == 1 && g.out_kind != LN_OUT_F32 && g.cpad <= 64;
+    const bool small = allow_small && !box_order &&
+                       ln_conv_choose_small(ctx->sm_count, g.kind, (int64_t)((g.OW + box_w - 1) / box_w) * ((g.OH + box_h - 1) / box_h) * ((g.N + box_n - 1) / box_n), g.F, g.fpad,
+                                    g.k * g.k * (g.cpad / bk), bk, &small_bn, &ksplit);
+    if (small) bn = small_bn;
     if (g.fpad % bn != 0) return ln_fail(ctx, LN_ERR_ARG, "tensor-core convolution: weights are padded to %d filters, tile needs a multiple of %d", g.fpad, bn);
     p.bk = bk; p.bn = bn;
     p.R = g.k; p.S = g.k; p.stride = g.stride; p.pad = g.pad;
@@ -1119,7 +1182,7 @@ int ln_conv_umma_plan_build(ln_ctx* ctx, ln_conv_umma_plan* plan, const ln_conv_
     while (p.subs > 1 && (bn % (32 * p.subs)) != 0) --p.subs;
     p.small_acc = g.small_acc ? 1 : 0;
     p.pack = pack; p.f_real = g_in.F;
-    choose_box(g.OW, g.OH, g.N, g.out_kind != LN_OUT_Q, &p.TW, &p.TH, &p.TN);
+    p.TW = box_w; p.TH = box_h; p.TN = box_n;
     // Row-shifted boxes for 3x3 stride-1 layers.  The nine taps of a tile read overlapping windows of the same input patch; one
     // box per tap re-reads that patch nine times from L2, which is what bounds these layers (the TMA unit's row rate for few
     // channels, L2 bandwidth for many).  Three boxes of TW x (TH + 2) pixels, shifted by 0 / 1 / 2 pixels in x, hold every
@@ -1132,7 +1195,7 @@ int ln_conv_umma_plan_build(ln_ctx* ctx, ln_conv_umma_plan* plan, const ln_conv_
     if (tab_bytes > kMaxTableBytes) return ln_fail(ctx, LN_ERR_UNSUPPORTED, "tensor-core convolution: %d filters exceed the %u the epilogue table holds", g.F, kMaxTableBytes / 8u);
     p.tab_bytes = (int)tab_bytes;
     const uint32_t smem_budget = (uint32_t)kMaxDynamicSmem - 1024u - 512u - tab_bytes;
-    if (allow_halo && g.k == 3 && g.stride == 1 && pack == 1 && g.out_kind != LN_OUT_F32 && g.cpad <= 64) {
+    if (allow_halo && !small && g.k == 3 && g.stride == 1 && pack == 1 && g.out_kind != LN_OUT_F32 && g.cpad <= 64) {
         int best_tw = 0, best_th = 0;
         int64_t best_tiles = -1;
         for (int lw = 3; lw <= 7; ++lw) {
@@ -1190,7 +1253,19 @@ int ln_conv_umma_plan_build(ln_ctx* ctx, ln_conv_umma_plan* plan, const ln_conv_
     const int b_rows = bn;
     const uint32_t b_total = (uint32_t)(g.k * g.k * (g.cpad / bk)) * (uint32_t)b_rows * bk;  // all weights of one filter tile (this CTA's part)
     // weights stay in shared memory when there is a single filter tile and they leave room for at least four activation stages
-    if (p.halo) {
+    if (small) {
+        p.ksplit = ksplit;
+        const int share = (g.k * g.k * p.cblocks + ksplit - 1) / ksplit;  // k-blocks of a CTA, rounded up
+        const uint32_t stage = (uint32_t)(128 + bn) * bk, partial = ksplit > 1 ? (uint32_t)(bn / 8) * kPieceBytes : 0u;
+        const uint32_t rest = 1024u /*alignment slack*/ + kSmallBarBytes + (uint32_t)bn * 8u;
+        p.stages = (int)((kSmallSmem - rest) / stage);
+        if (p.stages > kMaxStages) p.stages = kMaxStages;
+        if (p.stages > share) p.stages = share;
+        const uint32_t ring = (uint32_t)p.stages * stage;
+        p.small_region = (int)(ring > partial ? ring : partial);
+        plan->smem = (size_t)p.small_region + rest;
+        plan->grid = p.num_tiles * ksplit;
+    } else if (p.halo) {
         const uint32_t box = (uint32_t)p.box_bytes, b_bytes = (uint32_t)bn * bk;
         p.b_resident = (p.tiles_f == 1 && b_total + 4u * box <= smem_budget) ? 1 : 0;
         int a_stages, stages;
@@ -1252,7 +1327,7 @@ int ln_conv_umma_plan_build(ln_ctx* ctx, ln_conv_umma_plan* plan, const ln_conv_
     plan->grid = grid;
     plan->smem = (size_t)stages * stage_bytes + (p.b_resident ? b_total : 0u) + 1024 /*alignment slack*/ + 512 /*barriers*/;
     }
-    plan->smem += tab_bytes;
+    if (!small) plan->smem += tab_bytes;
     if (p.halo) plan->grid = p.num_tiles < ctx->sm_count ? p.num_tiles : ctx->sm_count;
     plan->kind = g.kind;
 
@@ -1288,7 +1363,7 @@ int ln_conv_umma_plan_build(ln_ctx* ctx, ln_conv_umma_plan* plan, const ln_conv_
     if (getenv("LN_DEBUG_PLAN"))
         fprintf(stderr, "plan: bk %d bn %d stages %d nbuf %d subs %d b_res %d halo %d a_stages %d box %d TW %d TH %d TN %d tiles %d f %d grid %d smem %zu tab %d kind %d small %d folded %d pack %d%s\n",
                 p.bk, p.bn, p.stages, p.nbuf, p.subs, p.b_resident, p.halo, p.a_stages, p.box_bytes, p.TW, p.TH, p.TN, p.num_tiles, p.tiles_f, plan->grid,
-                plan->smem, p.tab_bytes, plan->kind, p.small_acc, p.mb_folded != nullptr, p.pack, (p.pipes == 2 ? " 2 pipelines" : ""));
+                plan->smem, p.tab_bytes, plan->kind, p.small_acc, p.mb_folded != nullptr, p.pack, (p.ksplit ? " small grid" : (p.pipes == 2 ? " 2 pipelines" : "")));
     return LN_OK;
 }
 
@@ -1370,6 +1445,13 @@ extern "C" int32_t ln_debug_mma_peak_shape(ln_ctx* ctx, int32_t dtype, int32_t n
 int ln_conv_umma_launch(ln_ctx* ctx, const ln_conv_umma_plan* plan) {
     cudaError_t e;
     const bool exact = ctx->exact_epilogue;
+    if (plan->p.ksplit) {
+        if (plan->kind == LN_KIND_I8) e = exact ? launch_small<LN_KIND_I8, true>(ctx, *plan) : launch_small<LN_KIND_I8, false>(ctx, *plan);
+        else if (plan->kind == LN_KIND_F16) e = launch_small<LN_KIND_F16, false>(ctx, *plan);
+        else e = exact ? launch_small<LN_KIND_F8, true>(ctx, *plan) : launch_small<LN_KIND_F8, false>(ctx, *plan);
+        ctx->launches++;
+        return e == cudaSuccess ? LN_OK : ln_fail(ctx, LN_ERR_CUDA, "tensor-core convolution launch: %s", cudaGetErrorString(e));
+    }
     const bool two = plan->p.pipes == 2;
 #define LN_LAUNCH_KIND(K, X) (two ? launch_act<K, X, 2>(ctx, plan->p, plan->grid, plan->smem, ctx->stream) : launch_act<K, X, 1>(ctx, plan->p, plan->grid, plan->smem, ctx->stream))
     if (plan->kind == LN_KIND_I8) e = exact ? LN_LAUNCH_KIND(LN_KIND_I8, true) : LN_LAUNCH_KIND(LN_KIND_I8, false);

@@ -852,6 +852,9 @@ int build_plan(ln_net* net, int mb) {
                     st.umma.mb = st.mb;
                     rc = ln_conv_umma_plan_build(ctx, &st.umma, g);
                     if (rc) return rc;
+                    // (a step in front of it, the first layer's, separates the launch from the kernels that wrote weights and tables)
+                    st.umma.chained = !net->steps.empty();
+                    st.umma.p.early = st.umma.chained ? 1 : 0;
                 } else st.op = 1;
                 if (st.op != 0 && net->fused_into_next[i] == 1) return ln_fail(ctx, LN_ERR_UNSUPPORTED, "layer #%d: a fused shortcut needs the tensor-core convolution", i);
                 net->steps.push_back(st);
