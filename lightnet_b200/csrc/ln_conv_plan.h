@@ -120,19 +120,20 @@ inline int ln_conv_choose_bn(int64_t F) {
 // Filter tile and k split of the small-grid kernel for a layer of m pixel tiles; false: the layer is left to the persistent kernel.
 // A layer qualifies when some choice needs no more CTAs than fit the GPU at once, two per SM (beyond that the persistent kernel, which
 // overlaps epilogue and main loop, is the better one).  Among the choices the one with the shortest chain is taken, in cycles:
-// 180 per tensor instruction with its loads (half as much again where two CTAs share an SM), 1000 per piece of epilogue that a warp
-// does, 9000 for the exchange of partial sums with its two cluster barriers.  (YOLOv4 608 x 608 int8, one image, forward: 837 us with
-// 4000 for the exchange, 796 with 6500, 791 with 9000, 802 without any split.)  FP8 is not split: its codes would depend on the order of
-// the sum.
+// 130 per tensor instruction with its loads, 180 where one thread issues them all (half as much again where two CTAs share an SM), 1000
+// per piece of epilogue that a warp does, 9000 for the exchange of partial sums with its two cluster barriers.  (YOLOv4 608 x 608
+// int8, one image, forward: 837 us with 4000 for the exchange, 796 with 6500, 791 with 9000, 802 without any split; with two issuing
+// threads 780 us at 180 cycles per instruction, 757 at 130, 768 at 90.)  Only int8 is split: binary32 sums depend on
+// their order.
 inline bool ln_conv_choose_small(int sm_count, int kind, int64_t m, int64_t F, int64_t fpad, int kblocks, int bk, int* bn_out, int* ks_out) {
     int64_t best = -1;
     for (int bn = 32; bn <= 128; bn *= 2) {
         if (fpad % bn != 0 || (bn > 32 && ln_round_up(F, 32) < bn)) continue;
         const int64_t tiles = m * ((F + bn - 1) / bn);
-        for (int ks = 1; ks <= (kind == LN_KIND_F8 ? 1 : 8); ks *= 2) {
+        for (int ks = 1; ks <= (kind == LN_KIND_I8 ? 8 : 1); ks *= 2) {
             if (tiles * ks > 2 * sm_count || ks > kblocks || ks > bn / 8) break;
             const int64_t instructions = (int64_t)((kblocks + ks - 1) / ks) * (bk / 32), rounds = (bn / 8 + ks * 8 - 1) / (ks * 8);
-            const int64_t cost = instructions * 180 * (tiles * ks > sm_count ? 3 : 2) / 2 + rounds * 1000 + (ks > 1 ? 9000 : 0);
+            const int64_t cost = instructions * (kind == LN_KIND_I8 ? 130 : 180) * (tiles * ks > sm_count ? 3 : 2) / 2 + rounds * 1000 + (ks > 1 ? 9000 : 0);
             if (best < 0 || cost < best) { best = cost; *bn_out = bn; *ks_out = ks; }
         }
     }

@@ -185,6 +185,14 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32])
           "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
 // n / d for n * d < 2^40 with the precomputed multiplier ceil(2^40 / d): one wide multiply and a shift
 __device__ __forceinline__ int fast_div(int n, unsigned long long magic) { return (int)(((unsigned long long)(unsigned)n * magic) >> 40); }
 
@@ -587,17 +595,18 @@ __global__ void __launch_bounds__(conv_threads(PIPES), 1) conv_umma_kernel(const
 #undef LN_UNIT_STEP
 
 // Small grids: layers whose tiles do not fill the GPU (a few images, or the 19 x 19 end of a network).  What bounds such a launch is
-// not a rate but one chain: launch, fill of the pipeline, the k loop of a single tile (about 180 cycles per instruction with its loads,
-// whatever its size), epilogue, exit.  So
-//   - filter tiles of 32 to 128 columns and, int8 and binary16, a long k range split over the CTAs of a cluster (see ln_conv_choose_small).  Each
+// not a rate but one chain: launch, fill of the pipeline, the k loop of a single tile (about 180 cycles per instruction of one issuing
+// thread, loads included and whatever its size), epilogue, exit.  So
+//   - filter tiles of 32 to 128 columns and, int8, a long k range split over the CTAs of a cluster (see ln_conv_choose_small).  Each
 //     CTA leaves its partial accumulators in its own shared memory as pieces of 32 rows x 32 columns; piece i belongs to the CTA of rank
-//     i % ksplit, which adds the parts up through distributed shared memory -- int32 sums, the same bits in any order; binary32 sums in rank
-//     order -- and runs the epilogue on it.  FP8 keeps one chain per output, so its codes do not change.
-//   - 320 threads, bn columns of TMEM and at most 112 KB of shared memory: two CTAs fit an SM, so that in a network (plan.chained)
+//     i % ksplit, which adds the parts up through distributed shared memory -- int32 sums, the same bits in any order -- and runs the
+//     epilogue on it.  FP8 and binary16 keep one chain per output, so their results stay the same bits (a split moved binary16 heads of
+//     deep networks by up to 0.8 %: every layer's rounding carries it on).
+//   - 320 threads, bn columns of TMEM (int8: twice that) and at most 112 KB of shared memory: two CTAs fit an SM, so that in a network (plan.chained)
 //     the next layer's CTAs can set up, fetch their table and start their weight loads while this layer still runs; griddepcontrol.wait
 //     stands in front of everything that the layers before it write or still read.
 // One tile per CTA, no persistent loop.
-// YOLOv4 608 x 608 int8, one image: 102 layers, forward 1254 -> 791 us (957 without programmatic launches, 802 without the k split); 1x1
+// YOLOv4 608 x 608 int8, one image: 102 layers, forward 1254 -> 791 us, 757 with two issuing threads (957 without programmatic launches, 802 without the k split); 1x1
 // C512 -> K256 at 38 x 38 9.5 -> 7.5 us, 3x3 C512 -> K1024 at 19 x 19 25 -> 15 us as single cold launches.
 constexpr int kSmallEpilogueWarps = 8;
 constexpr int kSmallThreads = 32 * (2 + kSmallEpilogueWarps);
@@ -607,12 +616,30 @@ constexpr uint32_t kPieceBytes = 4096u;    // 32 rows x 32 columns of partial su
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 
+// 32 columns of the tile's accumulator, the sum of both issuers' where there are two (the second one's bn columns further on)
+template <int KIND>
+__device__ __forceinline__ void small_acc(uint32_t taddr, int bn, int issuers, uint32_t (&acc)[32]) {
+    tmem_ld_32x32(taddr, acc);
+    tmem_ld_wait();
+    if constexpr (KIND == LN_KIND_I8) {
+        if (issuers == 1) return;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            uint32_t v[16];
+            tmem_ld_32x16(taddr + (uint32_t)(bn + 16 * h), v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) acc[16 * h + j] += v[j];
+        }
+    }
+}
+
 template <int KIND, int ACT, bool EXACT>
 __global__ void __launch_bounds__(kSmallThreads, 2) conv_umma_small_kernel(const __grid_constant__ ln_conv_umma_params p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* generic_base = smem_raw + (smem_base - smem_u32(smem_raw));
-    const int bk = p.bk, bn = p.bn, stages = p.stages, ks = p.ksplit;
+    const int bk = p.bk, bn = p.bn, stages = p.stages, ks = KIND == LN_KIND_I8 ? p.ksplit : 1;
     const uint32_t a_bytes = 128u * bk, stage_bytes = a_bytes + (uint32_t)bn * bk;
     const uint32_t bar_base = smem_base + (uint32_t)p.small_region;
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
@@ -628,6 +655,10 @@ __global__ void __launch_bounds__(kSmallThreads, 2) conv_umma_small_kernel(const
     const int ow0 = tw * p.TW, oh0 = th * p.TH, n0 = tn * p.TN, f0 = tf * bn;
     const int kblocks = p.R * p.S * p.cblocks;
     const int kb0 = kblocks * rank / ks, nkb = kblocks * (rank + 1) / ks - kb0;  // this CTA's k-blocks (at least one: ks <= kblocks)
+    // The issuing thread costs 180 cycles per instruction, the tensor pipe less: two threads (warps 1 and 2, the latter an epilogue warp
+    // that has nothing to do yet) share the k-blocks, each into its own accumulator; the epilogue adds the two.  (int8 only.)
+    const int issuers = KIND == LN_KIND_I8 && nkb > 1 && stages > 1 ? 2 : 1;
+    const uint32_t tmem_cols = (uint32_t)bn << (KIND == LN_KIND_I8 ? 1 : 0);
     const bool folded = !EXACT && p.mb_folded != nullptr;
     const uint32_t tab_base = bar_base + kSmallBarBytes - 8u * (uint32_t)f0;  // where filter 0 would be: the table holds this tile's filters only
 
@@ -638,12 +669,12 @@ __global__ void __launch_bounds__(kSmallThreads, 2) conv_umma_small_kernel(const
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
         }
-        mbar_init(done_bar, 1);
+        mbar_init(done_bar, (uint32_t)issuers);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)), "r"((uint32_t)bn) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)), "r"(tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (!p.early) asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -696,32 +727,40 @@ __global__ void __launch_bounds__(kSmallThreads, 2) conv_umma_small_kernel(const
             }
         }
         __syncwarp();
-    } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = (KIND == LN_KIND_I8 ? ((2u << 4) | (1u << 7) | (1u << 10)) : (1u << 4)) | ((uint32_t)(bn >> 3) << 17) | ((128u >> 4) << 24);
-            const uint64_t desc_base = make_smem_desc(0u, bk);
-            asm volatile("griddepcontrol.wait;" ::: "memory");
-            int stage = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            for (int i = 0; i < nkb; ++i) {
-                if (!(ok = mbar_wait(full_bar(stage), phase, abort_flag, p.status, LN_STATUS_MMA_TIMEOUT))) break;
-                const uint32_t sa = smem_base + (uint32_t)stage * stage_bytes;
-                const uint64_t a_desc = desc_base + (sa >> 4), b_desc = desc_base + ((sa + a_bytes) >> 4);
-                tc_mma<KIND>(tmem_base, a_desc, b_desc, idesc, (uint32_t)(i != 0));
-                if (bk >= 64) tc_mma<KIND>(tmem_base, a_desc + 2u, b_desc + 2u, idesc, 1u);
-                if (bk == 128) {
-                    tc_mma<KIND>(tmem_base, a_desc + 4u, b_desc + 4u, idesc, 1u);
-                    tc_mma<KIND>(tmem_base, a_desc + 6u, b_desc + 6u, idesc, 1u);
-                }
-                tc_commit(empty_bar(stage));
-                if (++stage == stages) { stage = 0; phase ^= 1u; }
-            }
-            if (ok) tc_commit(done_bar);
-        }
-        __syncwarp();
     } else {
         asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (warp <= issuers) {
+            // Issuer w takes the k-blocks that land in the stages of its parity.  (Every second k-block would not do: with an odd number of
+            // stages an issuer could come back to a stage whose use by the other one is still to be filled, and a wait on parity would
+            // take the use before that for its own.)
+            if (lane == 0) {
+                const uint32_t idesc = (KIND == LN_KIND_I8 ? ((2u << 4) | (1u << 7) | (1u << 10)) : (1u << 4)) | ((uint32_t)(bn >> 3) << 17) | ((128u >> 4) << 24);
+                const uint64_t desc_base = make_smem_desc(0u, bk);
+                const uint32_t d_tmem = tmem_base + (uint32_t)((warp - 1) * bn);
+                int stage = 0;
+                uint32_t phase = 0, accumulate = 0u;
+                bool ok = true;
+                for (int i = 0; i < nkb; ++i) {
+                    const int at = stage;
+                    const uint32_t parity = phase;
+                    if (++stage == stages) { stage = 0; phase ^= 1u; }
+                    if (issuers == 2 && (at & 1) != warp - 1) continue;
+                    if (!(ok = mbar_wait(full_bar(at), parity, abort_flag, p.status, LN_STATUS_MMA_TIMEOUT))) break;
+                    const uint32_t sa = smem_base + (uint32_t)at * stage_bytes;
+                    const uint64_t a_desc = desc_base + (sa >> 4), b_desc = desc_base + ((sa + a_bytes) >> 4);
+                    tc_mma<KIND>(d_tmem, a_desc, b_desc, idesc, accumulate);
+                    accumulate = 1u;
+                    if (bk >= 64) tc_mma<KIND>(d_tmem, a_desc + 2u, b_desc + 2u, idesc, 1u);
+                    if (bk == 128) {
+                        tc_mma<KIND>(d_tmem, a_desc + 4u, b_desc + 4u, idesc, 1u);
+                        tc_mma<KIND>(d_tmem, a_desc + 6u, b_desc + 6u, idesc, 1u);
+                    }
+                    tc_commit(empty_bar(at));
+                }
+                if (ok) tc_commit(done_bar);
+            }
+            __syncwarp();
+        }
     }
 
     constexpr bool kTranscendental = ACT == LN_ACT_MISH || ACT == LN_ACT_SWISH || ACT == LN_ACT_LOGISTIC;
@@ -735,8 +774,7 @@ __global__ void __launch_bounds__(kSmallThreads, 2) conv_umma_small_kernel(const
             const int quad = warp & 3;  // the TMEM lanes this warp may read
             for (int c = (warp - 2) >> 2; c < bn / 32; c += kSmallEpilogueWarps / 4) {
                 uint32_t acc[32];
-                tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * 32), acc);
-                tmem_ld_wait();
+                small_acc<KIND>(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * 32), bn, issuers, acc);
                 const uint32_t dst = smem_base + (uint32_t)(c * 4 + quad) * kPieceBytes + 16u * (uint32_t)lane;
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
@@ -758,7 +796,7 @@ __global__ void __launch_bounds__(kSmallThreads, 2) conv_umma_small_kernel(const
                     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(part) : "r"(at), "r"(k));
                     asm volatile("ld.shared::cluster.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(part) : "memory");
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) sum[j] = KIND == LN_KIND_I8 ? sum[j] + v[j] : __float_as_uint(__uint_as_float(sum[j]) + __uint_as_float(v[j]));
+                    for (int j = 0; j < 4; ++j) sum[j] += v[j];
                 }
                 asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(sum[0]), "r"(sum[1]), "r"(sum[2]), "r"(sum[3]) : "memory");
             }
@@ -776,7 +814,7 @@ __global__ void __launch_bounds__(kSmallThreads, 2) conv_umma_small_kernel(const
             const bool valid = ow < p.OW && oh < p.OH && n < p.N;
             const int64_t pix = ((int64_t)n * p.OH + oh) * p.OW + ow;
             uint32_t acc[32];
-            if (ks == 1) tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, acc);
+            if (ks == 1) small_acc<KIND>(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, bn, issuers, acc);
             else {
                 const uint32_t src = smem_base + (uint32_t)piece * kPieceBytes + 16u * (uint32_t)lane;
 #pragma unroll
@@ -798,7 +836,7 @@ __global__ void __launch_bounds__(kSmallThreads, 2) conv_umma_small_kernel(const
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)bn) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
     }
 }
 
@@ -1161,11 +1199,11 @@ int ln_conv_umma_plan_build(ln_ctx* ctx, ln_conv_umma_plan* plan, const ln_conv_
         const int v = atoi(e);
         if ((v == 128 || v == 64) && v < bn && g.fpad % v == 0) bn = v;
     }
-    // Small grids: a kernel of their own.  (FP8 layers that the row-shifted boxes below could take stay with the persistent kernel: those
-    // sum the taps in another order, which would change codes.)
+    // Small grids: a kernel of their own.  (FP8 and binary16 layers that the row-shifted boxes below could take stay with the persistent kernel: those
+    // sum the taps in another order, which would change results.)
     int box_w = 0, box_h = 0, box_n = 0, ksplit = 0, small_bn = 0;
     choose_box(g.OW, g.OH, g.N, g.out_kind != LN_OUT_Q, &box_w, &box_h, &box_n);
-    const bool box_order = g.kind == LN_KIND_F8 && g.k == 3 && g.stride == 1 && pack == 1 && g.out_kind != LN_OUT_F32 && g.cpad <= 64;
+    const bool box_order = g.kind != LN_KIND_I8 && g.k == 3 && g.stride == 1 && pack == 1 && g.out_kind != LN_OUT_F32 && g.cpad <= 64;
     const bool small = allow_small && !box_order &&
                        ln_conv_choose_small(ctx->sm_count, g.kind, (int64_t)((g.OW + box_w - 1) / box_w) * ((g.OH + box_h - 1) / box_h) * ((g.N + box_n - 1) / box_n), g.F, g.fpad,
                                     g.k * g.k * (g.cpad / bk), bk, &small_bn, &ksplit);

@@ -21,6 +21,8 @@ CASES = [
     (3, 32, 20, 24, 64, 1, 1, 0),     # pixel groups
     (1, 1024, 19, 19, 512, 1, 1, 0),  # split, several pixel tiles
     (1, 32, 1, 1, 32, 1, 1, 0),       # one k-block, one pixel
+    (4, 256, 61, 61, 128, 3, 1, 1),   # 128-filter tiles: a ring of three stages shared by two issuers, 18 k-blocks
+    (1, 512, 38, 38, 256, 3, 1, 1),   # the same over 36
 ]
 
 
@@ -90,7 +92,9 @@ def test_small_grid_f16(be, monkeypatch, case):
         return be.download_f16(be.conv2d_bias_act_f16(tx, wh, bias, shape, c, h, w, f, k, s, s, 1, p, 1, "linear"))
 
     # one rounding to 11 bits of the result, binary32 accumulation: 2^-13 of the sum of magnitudes (the bound of the 8-bit float tests)
-    for got in _both(monkeypatch, conv):
+    pair = _both(monkeypatch, conv)
+    np.testing.assert_array_equal(pair[0], pair[1])  # one chain per output in either form
+    for got in pair:
         assert (np.abs(got - ref) <= 2.0 ** -11 * np.abs(ref) + 2.0 ** -13 * size + 2.0 ** -24).all()
 
 
@@ -114,7 +118,7 @@ int main() {
                         ++n;
                         split += ks > 1;
                         const long tiles = (long)m * ((F + bn - 1) / bn);
-                        if (fpad % bn || bn > 128 || bn < 32 || (ks & (ks - 1)) || ks < 1 || ks > 8 || tiles * ks > 296 || ks > kb || bn / 8 % ks || (kind == LN_KIND_F8 && ks > 1)) {
+                        if (fpad % bn || bn > 128 || bn < 32 || (ks & (ks - 1)) || ks < 1 || ks > 8 || tiles * ks > 296 || ks > kb || bn / 8 % ks || (kind != LN_KIND_I8 && ks > 1)) {
                             printf("bad choice kind %d m %d F %d kb %d bk %d: bn %d ks %d\n", kind, m, F, kb, bk, bn, ks);
                             return 1;
                         }
