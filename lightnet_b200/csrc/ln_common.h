@@ -31,6 +31,8 @@ struct ln_ctx {
     int sm_count = 0;
     std::multimap<size_t, void*> free_blocks;  // size-keyed cache of freed blocks; reuse is stream ordered
     std::map<void*, size_t> live_blocks;       // true size of every block handed out
+    // while a graph is captured: blocks freed meanwhile wait here (the graph's replays still use them) instead of going back to the cache
+    std::vector<std::pair<void*, size_t>>* held_blocks = nullptr;
     size_t pool_bytes = 0;                     // bytes held from the device: live + cached
     size_t cached_bytes = 0;
     int* h_status = nullptr;  // status word in page-locked memory, written by kernels whose bounded waits give up
@@ -79,6 +81,11 @@ struct ln_conv_weights {
 int ln_fail(ln_ctx* ctx, int code, const char* fmt, ...);
 int ln_status(ln_ctx* ctx, const char* where);        // after a synchronisation: LN_OK or LN_ERR_TIMEOUT (and clears the word)
 int ln_check_status(ln_ctx* ctx, const char* where);  // synchronises the ctx stream first
+int ln_narrow_f16_into(ln_ctx* ctx, const ln_tensor* t, ln_tensor* out_f16);  // out_f16: a binary16 tensor of t's shape
+int ln_conv_f16_table(ln_ctx* ctx, const ln_tensor* bias, float2** out);
+int ln_conv2d_bias_act_f16_enqueue(ln_ctx* ctx, const ln_tensor* x, ln_conv_weights* weights, const ln_tensor* bias, const float2* table, const int64_t output_shape[4],
+                                   int64_t channels, int64_t input_height, int64_t input_width, int64_t filters, int64_t size, int64_t stride_x,
+                                   int64_t stride_y, int64_t dilation, int64_t padding, int64_t groups, int32_t activation, ln_tensor** out);
 int ln_conv2d_bias_act_f32(ln_ctx* ctx, const ln_tensor* x, const ln_tensor* weights, const ln_tensor* bias, const int64_t output_shape[4], int64_t input_channels,
                            int64_t input_height, int64_t input_width, int64_t filters, int64_t kernel_size, int64_t stride_x, int64_t stride_y, int64_t dilation,
                            int64_t padding, int64_t groups, int activation, bool one_chain, ln_tensor** out);

@@ -278,8 +278,7 @@ int32_t ln_tensor_narrow_f16(ln_ctx* ctx, const ln_tensor* t, ln_tensor** out_f1
     cudaSetDevice(ctx->device);
     ln_tensor* q = ln_tensor_new(ctx, LN_F16, t->n, t->c, t->h, t->w);
     if (!q) return LN_ERR_CUDA;
-    f32_nchw_to_h_nhwc_kernel<<<grid_for(ctx, (int64_t)(q->bytes / 2)), kThreads, 0, ctx->stream>>>((const float*)t->ptr, (__half*)q->ptr, t->n, (int)t->c, (int)t->h, (int)t->w, hs(q));
-    int rc = check_launch(ctx, "narrow_f32");
+    int rc = ln_narrow_f16_into(ctx, t, q);
     if (rc) { ln_tensor_release(q); return rc; }
     *out_f16 = q;
     return LN_OK;
@@ -313,9 +312,30 @@ int32_t ln_conv_weights_f16(ln_ctx* ctx, const ln_tensor* weights_f32, int64_t f
     return LN_OK;
 }
 
-int32_t ln_conv2d_bias_act_f16(ln_ctx* ctx, const ln_tensor* x, ln_conv_weights* weights, const ln_tensor* bias, const int64_t output_shape[4],
-                               int64_t channels, int64_t input_height, int64_t input_width, int64_t filters, int64_t size, int64_t stride_x,
-                               int64_t stride_y, int64_t dilation, int64_t padding, int64_t groups, int32_t activation, ln_tensor** out) {
+}  // extern "C"
+
+int ln_narrow_f16_into(ln_ctx* ctx, const ln_tensor* t, ln_tensor* q) {
+    f32_nchw_to_h_nhwc_kernel<<<grid_for(ctx, (int64_t)(q->bytes / 2)), kThreads, 0, ctx->stream>>>((const float*)t->ptr, (__half*)q->ptr, t->n, (int)t->c, (int)t->h, (int)t->w, hs(q));
+    return check_launch(ctx, "narrow_f32");
+}
+
+// The {1, bias} table of a binary16 convolution, from the ctx pool.
+int ln_conv_f16_table(ln_ctx* ctx, const ln_tensor* bias, float2** out) {
+    const int64_t filters = bias->count(), fpad = ln_round_up(filters, ln_conv_choose_bn(filters));
+    float2* mb = (float2*)ln_pool_alloc(ctx, (size_t)fpad * sizeof(float2));
+    if (!mb) return LN_ERR_CUDA;
+    make_mb_unit_kernel<<<(int)((fpad + 127) / 128), 128, 0, ctx->stream>>>((const float*)bias->ptr, (int)filters, (int)fpad, mb);
+    const int rc = check_launch(ctx, "conv bias table");
+    if (rc) { ln_pool_free(ctx, mb, 0); return rc; }
+    *out = mb;
+    return LN_OK;
+}
+
+// conv2d_bias_act_f16 without the synchronisation at its end: whoever enqueues a sequence reads the status word after it.
+// table: what ln_conv_f16_table made of `bias` before, or null.
+int ln_conv2d_bias_act_f16_enqueue(ln_ctx* ctx, const ln_tensor* x, ln_conv_weights* weights, const ln_tensor* bias, const float2* table, const int64_t output_shape[4],
+                                   int64_t channels, int64_t input_height, int64_t input_width, int64_t filters, int64_t size, int64_t stride_x,
+                                   int64_t stride_y, int64_t dilation, int64_t padding, int64_t groups, int32_t activation, ln_tensor** out) {
     const char* who = "ln_conv2d_bias_act_f16";
     if (!ctx || !weights || !bias || !output_shape || !out) return ln_fail(ctx, LN_ERR_ARG, "%s: NULL argument", who);
     if (!is_h(x) || weights->dtype != LN_F16) return ln_fail(ctx, LN_ERR_ARG, "%s: binary16 input and weights required", who);
@@ -333,11 +353,13 @@ int32_t ln_conv2d_bias_act_f16(ln_ctx* ctx, const ln_tensor* x, ln_conv_weights*
     cudaSetDevice(ctx->device);
     ln_tensor* y = ln_tensor_new(ctx, LN_F16, x->n, filters, oh, ow);
     if (!y) return LN_ERR_CUDA;
-    if (y->cstride != 2 * y->c) cudaMemsetAsync(y->ptr, 0, y->bytes, ctx->stream);
+    const bool padded = y->cstride != 2 * y->c;
+    if (padded) cudaMemsetAsync(y->ptr, 0, y->bytes, ctx->stream);
     int rc = LN_OK;
     const int64_t cpad_bytes = x->cstride;  // 2 * channels padded to 32
     const bool tensor_core = groups == 1 && filters <= 4096 && ln_conv_umma_supported(cpad_bytes, size, stride_x, stride_y, dilation, groups, input_width, input_height);
     if (tensor_core) {
+        bool complete = table != nullptr;  // weights and table were finished before the kernel in front of this convolution started
         if (!weights->w || weights->channels != channels || weights->k != size) {  // first use with this geometry: pack
             if (weights->w) ln_pool_free(ctx, weights->w, 0);
             weights->channels = channels; weights->k = size;
@@ -349,13 +371,10 @@ int32_t ln_conv2d_bias_act_f16(ln_ctx* ctx, const ln_tensor* x, ln_conv_weights*
             pack_weights_h_kernel<<<grid_for(ctx, elems), kThreads, 0, ctx->stream>>>((const float*)weights->src_f32->ptr, (int)filters, (int)channels, (int)size, (int)(cpad_bytes / 2),
                                                                                     (int)weights->fpad, (__half*)weights->w);
             rc = check_launch(ctx, "conv_weights_f16");
+            complete = false;
         }
-        float2* mb = (float2*)ln_pool_alloc(ctx, (size_t)weights->fpad * sizeof(float2));
-        if (!mb) { ln_tensor_release(y); return LN_ERR_CUDA; }
-        if (rc == LN_OK) {
-            make_mb_unit_kernel<<<(int)((weights->fpad + 127) / 128), 128, 0, ctx->stream>>>((const float*)bias->ptr, (int)filters, (int)weights->fpad, mb);
-            rc = check_launch(ctx, "conv bias table");
-        }
+        float2* mb = const_cast<float2*>(table);
+        if (!mb && rc == LN_OK) rc = ln_conv_f16_table(ctx, bias, &mb);
         ln_conv_geom g;
         g.kind = LN_KIND_F16;
         g.x = x->ptr; g.x_pixel_stride = x->cstride;
@@ -367,11 +386,12 @@ int32_t ln_conv2d_bias_act_f16(ln_ctx* ctx, const ln_tensor* x, ln_conv_weights*
             ln_conv_umma_plan plan;
             plan.mb = mb;
             rc = ln_conv_umma_plan_build(ctx, &plan, g);
+            plan.chained = table != nullptr && !padded;  // (behind a kernel, not behind a memset)
+            plan.p.early = plan.chained && complete && !plan.aux_w && !plan.aux_mbf ? 1 : 0;
             if (rc == LN_OK) rc = ln_conv_umma_launch(ctx, &plan);
-            if (rc == LN_OK) rc = ln_check_status(ctx, who);
             ln_conv_umma_plan_release(ctx, &plan);
         }
-        ln_pool_free(ctx, mb, (size_t)weights->fpad * sizeof(float2));
+        if (!table) ln_pool_free(ctx, mb, 0);
     } else {
         conv_h_simt_kernel<<<grid_for(ctx, y->count()), kThreads, 0, ctx->stream>>>((const __half*)x->ptr, hs(x), (const float*)weights->src_f32->ptr, (const float*)bias->ptr,
                                                                                   (__half*)y->ptr, hs(y), x->n, (int)channels, (int)input_height, (int)input_width, (int)filters,
@@ -379,6 +399,21 @@ int32_t ln_conv2d_bias_act_f16(ln_ctx* ctx, const ln_tensor* x, ln_conv_weights*
                                                                                   activation);
         rc = check_launch(ctx, "conv2d_bias_act_f16");
     }
+    if (rc) { ln_tensor_release(y); return rc; }
+    *out = y;
+    return LN_OK;
+}
+
+extern "C" {
+
+int32_t ln_conv2d_bias_act_f16(ln_ctx* ctx, const ln_tensor* x, ln_conv_weights* weights, const ln_tensor* bias, const int64_t output_shape[4],
+                               int64_t channels, int64_t input_height, int64_t input_width, int64_t filters, int64_t size, int64_t stride_x,
+                               int64_t stride_y, int64_t dilation, int64_t padding, int64_t groups, int32_t activation, ln_tensor** out) {
+    ln_tensor* y = nullptr;
+    if (!out) return ln_fail(ctx, LN_ERR_ARG, "ln_conv2d_bias_act_f16: NULL argument");
+    int rc = ln_conv2d_bias_act_f16_enqueue(ctx, x, weights, bias, nullptr, output_shape, channels, input_height, input_width, filters, size, stride_x, stride_y, dilation,
+                                            padding, groups, activation, &y);
+    if (rc == LN_OK && weights->w) rc = ln_check_status(ctx, "ln_conv2d_bias_act_f16");  // (the tensor-core kernels report through the status word)
     if (rc) { ln_tensor_release(y); return rc; }
     *out = y;
     return LN_OK;

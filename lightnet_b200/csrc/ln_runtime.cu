@@ -59,6 +59,10 @@ void* ln_pool_alloc(ln_ctx* ctx, size_t bytes) {
 
 void ln_pool_free(ln_ctx* ctx, void* p, size_t bytes) {
     if (!p) return;
+    if (ctx->held_blocks) {
+        ctx->held_blocks->emplace_back(p, bytes);
+        return;
+    }
     auto live = ctx->live_blocks.find(p);
     const size_t real = live != ctx->live_blocks.end() ? live->second : (size_t)ln_round_up((int64_t)(bytes ? bytes : 1), 512);
     if (live != ctx->live_blocks.end()) ctx->live_blocks.erase(live);

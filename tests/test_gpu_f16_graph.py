@@ -1,0 +1,47 @@
+"""The captured binary16 forward: the values of the operator-by-operator one, and handles a caller keeps stay as they were."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def test_captured_forward_keeps_values_and_handles():
+    import lightnet_b200 as ln
+    from lightnet_b200 import synth, zoo
+    be = ln.B200Backend(0)
+    nets = [ln.GpuExecutableNetwork(be, zoo.yolov3_tiny_cfg(160, 96), 2, ln.LN_F16) for _ in range(2)]
+    blob = synth.he_weights(nets[0].layers(), 3)
+    for net in nets:
+        net.load_weights(blob)
+    nets[1].set_cuda_graph(False)
+    images = [synth.uniform_images(2, 3, 96, 160, s) for s in range(6)]
+
+    def heads(net):
+        return [be.download_f32(net.head(k)) for k in range(net.num_heads())]
+
+    want = []
+    for x in images:
+        nets[1].forward(x)
+        want.append(heads(nets[1]))
+    kept, kept_layer = None, None
+    for i, x in enumerate(images):  # eager, captured, replayed, (two with handles kept across them), replayed
+        nets[0].forward(x)
+        for got, ref in zip(heads(nets[0]), want[i]):
+            np.testing.assert_array_equal(got, ref)
+        if i == 2:
+            kept, kept_layer = nets[0].head(0), nets[0].layer_output(4)
+            before = be.download_f16(kept_layer)
+        if i in (3, 4):  # forwards since then left the kept tensors alone
+            np.testing.assert_array_equal(be.download_f32(kept), want[2][0])
+            np.testing.assert_array_equal(be.download_f16(kept_layer), before)
+        if i == 4:
+            del kept, kept_layer
+    nets[0].load_weights(blob * np.float32(0.5))  # new weights: nothing of the old graph is left
+    nets[1].load_weights(blob * np.float32(0.5))
+    for x in images[:3]:
+        for net in nets:
+            net.forward(x)
+        for got, ref in zip(heads(nets[0]), heads(nets[1])):
+            np.testing.assert_array_equal(got, ref)
+    del nets
+    be.close()
