@@ -16,7 +16,8 @@ inline int blocks_for(int64_t n, int per_block = kThreads) { return (int)((n + p
 // Convolution as a blocked GEMM: y[f][pixel] = sum over k = (channel, ky, kx) of w[f][k] * x[tap k of pixel].  Each output is one chain of
 // fused multiply-adds in k order, the order of runtime/forward_layers.rs:646-695; where tiles are few the k range is split over the
 // CTAs of a cluster (blockIdx.z), which add their chains up in order through distributed shared memory: no second pass over the
-// output and no second launch.  Taps outside the image contribute 0.
+// output and no second launch.  Taps outside the image enter the sum as zeros, which leaves it as it is while the weights are finite; an
+// output that comes out NaN next to the border is summed again without them (conv_f32_taps).
 struct ConvF32 {
     const float* x;
     const float* w;
@@ -30,6 +31,33 @@ __device__ __forceinline__ unsigned long long fma2_f32(unsigned long long a, uns
     unsigned long long d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
+}
+
+// Output (image b, filter f, pixel r) tap by tap, those outside the image skipped as in forward_layers.rs:646-695: an infinite or NaN weight
+// on such a tap must not reach the output, and a product with a zero would let it.
+__device__ __noinline__ float conv_f32_taps(const ConvF32& p, int b, int f, int r) {
+    const int iy0 = r / p.OW * p.sy - p.pad, ix0 = r % p.OW * p.sx - p.pad;
+    const float* w = p.w + (int64_t)f * p.K;
+    float acc = 0.0f;
+    for (int c = 0; c < p.C; ++c, w += p.k * p.k) {
+        const float* plane = p.x + ((int64_t)b * p.C + c) * p.H * p.W;
+        for (int ky = 0; ky < p.k; ++ky) {
+            const int iy = iy0 + ky * p.dil;
+            if (iy < 0 || iy >= p.H) continue;
+            for (int kx = 0; kx < p.k; ++kx) {
+                const int ix = ix0 + kx * p.dil;
+                if (ix >= 0 && ix < p.W) acc = fmaf(__ldg(plane + (int64_t)iy * p.W + ix), __ldg(w + ky * p.k + kx), acc);
+            }
+        }
+    }
+    return acc;
+}
+
+// Whether some tap of pixel r lies outside the image.
+__device__ __forceinline__ bool conv_f32_border(const ConvF32& p, int r) {
+    const int iy0 = r / p.OW * p.sy - p.pad, ix0 = r % p.OW * p.sx - p.pad;
+    const int64_t reach = (int64_t)(p.k - 1) * p.dil;
+    return iy0 < 0 || ix0 < 0 || iy0 + reach >= p.H || ix0 + reach >= p.W;
 }
 
 // Hands the CTA's tile (one per part of a split k range, side by side in distributed shared memory) to y: the parts added up in order,
@@ -48,6 +76,12 @@ __device__ __forceinline__ void conv_f32_finish(const ConvF32& p, float (&tile)[
         for (int s = 0; s < parts; ++s) {
             const float4 q = *reinterpret_cast<const float4*>(parts > 1 ? cluster.map_shared_rank(&tile[m][c], s) : &tile[m][c]);
             v[0] += q.x; v[1] += q.y; v[2] += q.z; v[3] += q.w;
+        }
+        if (isnan(v[0] + v[1] + v[2] + v[3])) {  // (false alarms, inf - inf, end in the conditions below)
+            for (int j = 0; j < 4; ++j) {
+                const int bj = (n + j) / P, r = n + j - bj * P;
+                if (n + j < NP && isnan(v[j]) && conv_f32_border(p, r)) v[j] = conv_f32_taps(p, bj, f, r);
+            }
         }
         const float bias = p.bias ? __ldg(p.bias + f) : 0.0f;
 #pragma unroll

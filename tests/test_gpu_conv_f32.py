@@ -58,3 +58,45 @@ def test_calibrated_scales_do_not_depend_on_the_batch(be):
         net.calibrate(np.repeat(x, batch, 0))
         scales.append(np.asarray(net.scales()))
     np.testing.assert_array_equal(scales[0], scales[1])
+
+
+@pytest.mark.parametrize("geom", [
+    (1, 36, 26, 26, 65, 3, 1, 1, 1),     # blocked, split k range
+    (2, 32, 160, 160, 128, 3, 1, 1, 1),  # 64 x 128 tiles
+    (1, 3, 30, 31, 17, 3, 2, 1, 1),      # staged through registers
+    (1, 5, 13, 13, 40, 3, 1, 1, 1),      # k range not a multiple of 4
+    (2, 64, 9, 9, 70, 1, 1, 1, 1),       # 1x1 with padding: border outputs have no tap at all
+    (1, 7, 12, 14, 9, 5, 1, 2, 1),
+    (1, 3, 15, 17, 4, 3, 1, 2, 2),       # dilated
+    (1, 4, 11, 10, 8, 3, 1, 1, 1, 2),    # grouped
+])
+def test_conv2d_f32_weights_that_are_not_finite(be, geom):
+    """Taps outside the image are skipped, so an infinite or NaN weight on them leaves the output alone: the same outputs are NaN, +inf and -inf as
+    in a sum over the taps inside, and the finite ones agree."""
+    B, C, H, W, F, k, s, pad, dil = geom[:9]
+    groups = geom[9] if len(geom) > 9 else 1
+    rng = np.random.default_rng(C + F)
+    x = rng.normal(0, 1, (B, C, H, W)).astype(np.float32)
+    w = rng.normal(0, 1, (F, C // groups, k, k)).astype(np.float32)
+    for f, tap, v in ((0, 0, np.inf), (1, 0, -np.inf), (2, k * k - 1, np.nan), (3, k * k // 2, np.inf), (F - 1, k * k - 1, np.inf)):
+        w[f, f % (C // groups), tap // k, tap % k] = v
+    oh, ow = (H + 2 * pad - k) // s + 1, (W + 2 * pad - k) // s + 1
+    got = be.download_f32(be.conv2d_f32(be.upload_f32(x.shape, x), be.upload_f32(w.shape, w), (B, F, oh, ow), C, H, W, F, k, s, s, dil, pad, groups)).astype(np.float64)
+    ref, size = np.zeros((B, F, oh, ow)), np.zeros((B, F, oh, ow))
+    fpg, cpg = F // groups, C // groups
+    with np.errstate(invalid="ignore"):
+        for ky in range(k):
+            for kx in range(k):
+                ys, xs = np.arange(oh) * s + ky * dil - pad, np.arange(ow) * s + kx * dil - pad
+                iy, ix = np.flatnonzero((ys >= 0) & (ys < H)), np.flatnonzero((xs >= 0) & (xs < W))
+                if not len(iy) or not len(ix):
+                    continue
+                patch = x[:, :, ys[iy]][:, :, :, xs[ix]].astype(np.float64)
+                for f in range(F):
+                    term = w[f, :, ky, kx].astype(np.float64)[None, :, None, None] * patch[:, f // fpg * cpg:(f // fpg + 1) * cpg]
+                    ref[:, f, iy[0]:iy[-1] + 1, ix[0]:ix[-1] + 1] += term.sum(1)
+                    size[:, f, iy[0]:iy[-1] + 1, ix[0]:ix[-1] + 1] += np.abs(term).sum(1)
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(ref))
+    np.testing.assert_array_equal(np.isinf(got) * np.sign(np.nan_to_num(got)), np.isinf(ref) * np.sign(np.nan_to_num(ref)))
+    ok = np.isfinite(ref)
+    assert (np.abs(got[ok] - ref[ok]) <= (C * k * k + 33) * 2.0 ** -24 * size[ok]).all()
