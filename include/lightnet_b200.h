@@ -347,8 +347,8 @@ int32_t ln_net_collect(ln_net* net, const int32_t* image_w, const int32_t* image
    image's own size (widths / heights), as `lightnet-rs detect-image` does (lightnet-cli/src/main.rs: load, letterbox, detect). */
 int32_t ln_net_detect_u8(ln_net* net, const uint8_t* pixels_host, const int64_t* offsets, const int32_t* widths, const int32_t* heights,
                          int32_t mode, const ln_detect_options* opts, ln_detection* records_host, int32_t* counts_host);
-/* Device time in ms of the most recent ln_net_forward* / ln_net_detect* call, by phase
-   (0 = layers, 1 = decode+NMS), measured with CUDA events on the ctx stream. */
+/* Device time in ms of the most recent ln_net_detect* / ln_net_collect call that succeeded, by phase (0 = layers, 1 = decode+NMS; both 0
+   before the first), measured with CUDA events on the ctx stream. */
 int32_t ln_net_last_times(const ln_net* net, float times_ms[2]);
 /* Per-kernel timing of 8-bit forwards.  With profiling on, every launch of the plan is bracketed by CUDA events on
    the ctx stream (the forward then synchronises).  ln_net_profile returns, for the last forward, device ms per layer

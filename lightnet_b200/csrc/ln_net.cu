@@ -262,8 +262,15 @@ struct ln_net {
     void* slot_staging[2] = {nullptr, nullptr};  // 8-bit pixels + metadata of ln_net_submit_u8, back to the pool at collect
     size_t slot_staging_bytes[2] = {0, 0};
     long long submitted = 0, collected = 0;
-    cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
-    int timed = 0;  // events ln_net_last_times has to read: 0 none, 1 of this network, 2 of the two part networks
+    // Times of a detect call, read lazily by ln_net_last_times: around its layers (those of either part, in the host-input pipeline) and after
+    // decode + NMS.  A call records into the set that is not `times_done` and makes it so when it has succeeded; nothing else records, so
+    // the figures of the last detect stay whatever runs or fails after it.
+    struct TimeSet {
+        cudaEvent_t layers[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}}, end = nullptr;
+        int parts = 0;  // 0: no call has completed into this set
+    };
+    TimeSet times[2];
+    int times_done = 0;
     // CUDA graph of the 8-bit plan (one graph = the whole batch: every micro-batch, every layer)
     bool fuse_shortcut = true;  // a linear [shortcut] whose input is a convolution nobody else reads runs in that convolution's epilogue
     std::vector<char> fused_into_next;  // per layer (8-bit plan): 1 = runs in the next layer's shortcut epilogue, no output; 2 = output kept in space-to-depth layout
@@ -1118,14 +1125,15 @@ int run_plan(ln_net* net, const float* input_dev_f32) {
     return LN_OK;
 }
 
-// `wait` = false: the caller synchronises the stream and reads the status word itself (the detect calls, after decode + NMS).
-int forward_any(ln_net* net, const ln_tensor* input, bool wait = true) {
+// `around` = the detect calls: events to record in front of and behind the layers; the caller synchronises the stream and reads the
+// status word itself, after decode + NMS.
+int forward_any(ln_net* net, const ln_tensor* input, cudaEvent_t* around = nullptr) {
     ln_ctx* ctx = net->ctx;
     if (!net->weights_loaded) return ln_fail(ctx, LN_ERR_ARG, "weights are not loaded");
     if (!input || input->dtype != LN_F32 || input->n != net->batch || input->c != net->channels || input->h != net->height || input->w != net->width)
         return ln_fail(ctx, LN_ERR_SHAPE, "input tensor must be f32 [%d,%d,%d,%d]", net->batch, net->channels, net->height, net->width);
     cudaSetDevice(ctx->device);
-    LN_CUDA(ctx, cudaEventRecord(net->ev[0], ctx->stream));
+    if (around) LN_CUDA(ctx, cudaEventRecord(around[0], ctx->stream));
     int rc;
     if (net->precision == LN_F32) rc = forward_f32(net, input, nullptr);
     else if (net->precision == LN_F16) rc = forward_f16(net, input);
@@ -1135,7 +1143,7 @@ int forward_any(ln_net* net, const ln_tensor* input, bool wait = true) {
         if (!net->plan_valid || net->plan_mb != mb) {
             rc = build_plan(net, mb);
             if (rc) { release_plan(net); return rc; }
-            LN_CUDA(ctx, cudaEventRecord(net->ev[0], ctx->stream));
+            if (around) LN_CUDA(ctx, cudaEventRecord(around[0], ctx->stream));
         }
         if (!net->use_graph || net->profile) rc = run_plan(net, (const float*)input->ptr);
         else {
@@ -1193,8 +1201,8 @@ int forward_any(ln_net* net, const ln_tensor* input, bool wait = true) {
             net->modern_heads[k] = boxes;
         }
     }
-    LN_CUDA(ctx, cudaEventRecord(net->ev[1], ctx->stream));
-    return wait && net->precision != LN_F32 ? ln_check_status(ctx, "ln_net_forward") : LN_OK;
+    if (around) LN_CUDA(ctx, cudaEventRecord(around[1], ctx->stream));
+    return !around && net->precision != LN_F32 ? ln_check_status(ctx, "ln_net_forward") : LN_OK;
 }
 
 int fill_heads(ln_net* net, std::vector<ln_yolo_head>& hs, const std::vector<ln_tensor*>* tensors = nullptr) {
@@ -1282,6 +1290,16 @@ int ensure_pipe(ln_net* net) {
     return LN_OK;
 }
 
+// The end of a detect call that has succeeded, `parts` networks having run its layers.
+int times_complete(ln_net* net, int parts) {
+    ln_ctx* ctx = net->ctx;
+    ln_net::TimeSet& t = net->times[1 - net->times_done];
+    LN_CUDA(ctx, cudaEventRecord(t.end, ctx->stream));
+    t.parts = parts;
+    net->times_done = 1 - net->times_done;
+    return LN_OK;
+}
+
 int stage_input(ln_net* net, const float* host) {
     ln_ctx* ctx = net->ctx;
     cudaSetDevice(ctx->device);
@@ -1313,8 +1331,9 @@ int32_t ln_net_create(ln_ctx* ctx, const char* cfg_text, int32_t batch, int32_t 
         return ln_fail(ctx, LN_ERR_PARSE, "%s", e.what());
     }
     cudaSetDevice(ctx->device);
-    for (auto& e : net->ev)
-        if (cudaEventCreate(&e) != cudaSuccess) return ln_fail(ctx, LN_ERR_CUDA, "cudaEventCreate failed");
+    for (auto& t : net->times)
+        for (cudaEvent_t* e : {&t.layers[0][0], &t.layers[0][1], &t.layers[1][0], &t.layers[1][1], &t.end})
+            if (cudaEventCreate(e) != cudaSuccess) return ln_fail(ctx, LN_ERR_CUDA, "cudaEventCreate failed");
     *out = net.release();
     return LN_OK;
 }
@@ -1343,7 +1362,9 @@ int32_t ln_net_destroy(ln_net* net) {
         ln_conv_weights_release(L.wq);
         ln_pool_free(net->ctx, L.table_f16, 0);
     }
-    for (auto& e : net->ev) if (e) cudaEventDestroy(e);
+    for (auto& t : net->times)
+        for (cudaEvent_t e : {t.layers[0][0], t.layers[0][1], t.layers[1][0], t.layers[1][1], t.end})
+            if (e) cudaEventDestroy(e);
     for (auto& e : net->prof_events) cudaEventDestroy(e);
     delete net;
     return LN_OK;
@@ -1538,7 +1559,8 @@ int32_t ln_net_layer_output(ln_net* net, int32_t layer, ln_tensor** out) {
 int32_t ln_net_detect_device(ln_net* net, const ln_tensor* input, const int32_t* image_w, const int32_t* image_h, const ln_detect_options* opts,
                              ln_detection* records_host, int32_t* counts_host) {
     if (!net || !image_w || !image_h || !opts || !records_host || !counts_host) return ln_fail(net ? net->ctx : nullptr, LN_ERR_ARG, "ln_net_detect: NULL argument");
-    int rc = forward_any(net, input, false);
+    ln_net::TimeSet& times = net->times[1 - net->times_done];
+    int rc = forward_any(net, input, times.layers[0]);
     if (rc) return rc;
     std::vector<ln_yolo_head> hs;
     rc = fill_heads(net, hs);
@@ -1547,9 +1569,7 @@ int32_t ln_net_detect_device(ln_net* net, const ln_tensor* input, const int32_t*
     rc = ln_yolo_decode_nms(ctx, hs.data(), (int)hs.size(), net->width, net->height, image_w, image_h, opts, records_host, counts_host);
     const int waited = ln_check_status(ctx, "ln_net_forward");
     if (waited || rc) return waited ? waited : rc;
-    LN_CUDA(ctx, cudaEventRecord(net->ev[2], ctx->stream));
-    net->timed = 1;
-    return LN_OK;
+    return times_complete(net, 1);
 }
 
 int32_t ln_net_detect(ln_net* net, const float* input_host, const int32_t* image_w, const int32_t* image_h, const ln_detect_options* opts,
@@ -1581,7 +1601,7 @@ int32_t ln_net_detect(ln_net* net, const float* input_host, const int32_t* image
         for (int h = 0; h < 2; ++h) {
             ln_net* c = net->pipe[h];
             LN_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, net->copy_ev[h], 0));
-            rc = forward_any(c, c->input_dev, false);
+            rc = forward_any(c, c->input_dev, net->times[1 - net->times_done].layers[h]);
             if (rc) return rc;
         }
         std::vector<ln_yolo_head> hs;
@@ -1590,9 +1610,7 @@ int32_t ln_net_detect(ln_net* net, const float* input_host, const int32_t* image
         rc = ln_yolo_decode_nms(ctx, hs.data(), (int)hs.size(), net->width, net->height, image_w, image_h, opts, records_host, counts_host);
         const int waited = ln_check_status(ctx, "ln_net_forward");
         if (waited || rc) return waited ? waited : rc;
-        LN_CUDA(ctx, cudaEventRecord(net->ev[2], ctx->stream));
-        net->timed = 2;
-        return LN_OK;
+        return times_complete(net, 2);
     }
     int rc = stage_input(net, input_host);
     if (rc) return rc;
@@ -1744,16 +1762,16 @@ int32_t ln_net_profile(const ln_net* net, float* per_layer_ms, int32_t num_layer
 int32_t ln_net_last_times(const ln_net* net, float times_ms[2]) {
     if (!net || !times_ms) return LN_ERR_ARG;
     times_ms[0] = times_ms[1] = 0.0f;
-    if (net->timed && cudaEventSynchronize(net->ev[2]) == cudaSuccess) {
-        for (int h = 0; h < net->timed; ++h) {
-            const ln_net* c = net->timed == 1 ? net : net->pipe[h];
-            float ms = 0.0f;
-            if (!c || cudaEventElapsedTime(&ms, c->ev[0], c->ev[1]) != cudaSuccess) continue;
-            times_ms[0] += ms;
-            if (cudaEventElapsedTime(&ms, c->ev[1], net->ev[2]) == cudaSuccess) times_ms[1] = ms;
-        }
-        (void)cudaGetLastError();
+    const ln_net::TimeSet& t = net->times[net->times_done];
+    if (t.parts == 0) return LN_OK;
+    cudaError_t e = cudaEventSynchronize(t.end);
+    for (int h = 0; h < t.parts && e == cudaSuccess; ++h) {
+        float ms = 0.0f;
+        e = cudaEventElapsedTime(&ms, t.layers[h][0], t.layers[h][1]);
+        times_ms[0] += ms;
     }
+    if (e == cudaSuccess) e = cudaEventElapsedTime(&times_ms[1], t.layers[t.parts - 1][1], t.end);
+    if (e != cudaSuccess) return ln_fail(net->ctx, LN_ERR_CUDA, "ln_net_last_times: %s", cudaGetErrorString(e));
     return LN_OK;
 }
 

@@ -137,3 +137,28 @@ def test_region_forward_and_yolo_activate(be):
     for new_coords, s in ((False, 1.2), (True, 2.0)):
         got = be.download_f32(be.yolo_activate_f32(t, classes, s, new_coords))
         assert np.allclose(got, orc.yolo_activate(x, classes, s, new_coords), rtol=3e-6, atol=1e-7)
+
+
+def test_last_times_are_those_of_the_last_detect(be):
+    """ln_net_last_times keeps the figures of the last detect call through forwards, failed detects and the release of part networks."""
+    from lightnet_b200 import zoo
+    x = synth.uniform_images(8, 3, 96, 160, 7)
+    net = ln.GpuExecutableNetwork(be, zoo.yolov3_tiny_cfg(160, 96), 8, ln.LN_Q8)
+    net.load_weights(synth.he_weights(net.layers(), 3))
+    assert net.last_times_ms() == (0.0, 0.0)
+    net.calibrate(x)
+    scales = net.scales()
+    size = (np.full(8, 160, np.int32), np.full(8, 96, np.int32))
+    t = be.upload_f32(x.shape, x)
+    for call in (lambda: net.detect_device(t, *size), lambda: net.detect(x, *size)):  # whole batch, two parts
+        call()
+        before = net.last_times_ms()
+        assert min(before) > 0.0
+        net.forward(x)
+        net.forward_device(t)
+        with pytest.raises(ln.BackendError):
+            net.detect_device(t, *size, max_per_image=5000)  # fails after its layers are enqueued
+        net.set_scales(scales)  # releases the part networks
+        assert net.last_times_ms() == before
+    call()
+    assert min(net.last_times_ms()) > 0.0
