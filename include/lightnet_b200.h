@@ -401,6 +401,8 @@ int32_t ln_debug_mma_peak_shape(ln_ctx* ctx, int32_t dtype, int32_t n, int32_t p
    a library built with -DLN_CONV_ROLE_TIMING and LN_DEBUG_CYCLES=1 in the environment at ln_ctx_create; LN_ERR_UNSUPPORTED
    otherwise. */
 int32_t ln_ctx_debug_cycles(ln_ctx* ctx, int64_t cycles[32]);
+/* The n-th request for device memory that the ctx makes from now on fails, once, as if the device had none left (0 = none does). */
+int32_t ln_debug_fail_alloc(ln_ctx* ctx, int64_t n);
 
 #ifdef __cplusplus
 }

@@ -160,6 +160,7 @@ SYMBOLS = {
     "ln_channel_affine_act_f16": (C.c_int32, [_VP, _VP, _VP, _VP, C.c_int64, C.c_int64, C.c_int32, _PP]),
     "ln_debug_score_key_error": (C.c_int32, [_VP, C.c_float, C.c_float, C.c_float, C.c_float, C.c_int32, C.c_int32, C.POINTER(C.c_uint32)]),
     "ln_ctx_debug_cycles": (C.c_int32, [_VP, _I64P]),
+    "ln_debug_fail_alloc": (C.c_int32, [_VP, C.c_int64]),
     "ln_modern_yolo_forward_f32": (C.c_int32, [_VP, _VP, C.c_int64, _VP]),
     "ln_modern_yolo_predecode_f32": (C.c_int32, [_VP, _VP, C.c_int64, C.c_int64, C.c_int32, _VP]),
     "ln_debug_mma_peak": (C.c_int32, [_VP, C.c_int32, C.c_int32, C.POINTER(C.c_float)]),
@@ -310,6 +311,10 @@ class B200Backend:
         else:
             self._check(self.lib.ln_debug_mma_peak_shape(self.ctx, dtype, n, 1 if pair else 0, iters, C.byref(t)))
         return float(t.value)
+
+    def debug_fail_alloc(self, n):
+        """The n-th device allocation of this backend from now on fails, once (0: none does)."""
+        self._check(self.lib.ln_debug_fail_alloc(self.ctx, n))
 
     def debug_cycles(self):
         """The 32 role-timing counters of the last tensor-core convolution (needs a -DLN_CONV_ROLE_TIMING build and LN_DEBUG_CYCLES=1)."""

@@ -35,6 +35,7 @@ struct ln_ctx {
     std::vector<std::pair<void*, size_t>>* held_blocks = nullptr;
     size_t pool_bytes = 0;                     // bytes held from the device: live + cached
     size_t cached_bytes = 0;
+    int64_t fail_alloc = 0;                    // test aid: that many allocations from now one fails (ln_debug_fail_alloc)
     int* h_status = nullptr;  // status word in page-locked memory, written by kernels whose bounded waits give up
     ln_encode_tiled_fn encode_tiled = nullptr;
     long long* debug_cycles = nullptr;  // when set (LN_DEBUG_CYCLES=1), the tensor-core convolution records role timings of CTA 0

@@ -295,7 +295,9 @@ struct ln_net {
         std::vector<std::pair<ln_tensor*, int>> refs;      // every tensor of out and heads with the references the graph holds
         std::vector<std::pair<void*, size_t>> held;        // working memory of the captured kernels
         int64_t launches = 0;
-        bool seen = false, failed = false;                 // one forward has run since the weights were loaded; the capture failed
+        // seen: a forward has run to its end since the weights were loaded, so that every layer's weights are packed (the packing of a
+        // first use must not be captured: it would not have happened should the capture fail later on); failed: the capture failed
+        bool seen = false, failed = false;
     };
     GraphF16 graph_f16;
     // optional per-launch timing
@@ -717,12 +719,12 @@ int forward_f16(ln_net* net, const ln_tensor* input) {
         for (auto* t : net->heads) ln_tensor_retain(t);
         return LN_OK;
     }
-    g.seen = true;
     ln_tensor* in16 = nullptr;
     rc = ln_tensor_narrow_f16(ctx, input, &in16);
     if (rc) return rc;
     rc = forward_f16_layers(net, in16);
     ln_tensor_release(in16);
+    g.seen = g.seen || rc == LN_OK;
     return rc;
 }
 

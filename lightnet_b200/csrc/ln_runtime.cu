@@ -31,6 +31,10 @@ static void pool_drop_cached(ln_ctx* ctx, std::multimap<size_t, void*>::iterator
 
 void* ln_pool_alloc(ln_ctx* ctx, size_t bytes) {
     bytes = (size_t)ln_round_up((int64_t)(bytes ? bytes : 1), 512);
+    if (ctx->fail_alloc > 0 && --ctx->fail_alloc == 0) {
+        ln_fail(ctx, LN_ERR_CUDA, "cudaMalloc(%zu bytes): refused by ln_debug_fail_alloc", bytes);
+        return nullptr;
+    }
     auto it = ctx->free_blocks.lower_bound(bytes);
     if (it != ctx->free_blocks.end() && it->first <= 2 * bytes) {
         void* p = it->second;
@@ -202,6 +206,13 @@ int32_t ln_ctx_debug_cycles(ln_ctx* ctx, int64_t cycles[32]) {
     if (!ctx->debug_cycles) return ln_fail(ctx, LN_ERR_UNSUPPORTED, "ln_ctx_debug_cycles: role timing is off (set LN_DEBUG_CYCLES=1 before ln_ctx_create)");
     LN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     for (int i = 0; i < 32; ++i) cycles[i] = (int64_t)ctx->debug_cycles[i];
+    return LN_OK;
+}
+
+// Test aid: the n-th device allocation of the ctx from now on is refused, once.
+int32_t ln_debug_fail_alloc(ln_ctx* ctx, int64_t n) {
+    if (!ctx || n < 0) return ln_fail(ctx, LN_ERR_ARG, "ln_debug_fail_alloc: n must not be negative");
+    ctx->fail_alloc = n;
     return LN_OK;
 }
 

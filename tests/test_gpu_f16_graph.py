@@ -45,3 +45,46 @@ def test_captured_forward_keeps_values_and_handles():
             np.testing.assert_array_equal(got, ref)
     del nets
     be.close()
+
+
+def test_first_forward_out_of_memory_then_capture_out_of_memory():
+    """A first forward that runs out of memory half way, then a capture that does: the forwards after them compute with packed weights."""
+    import lightnet_b200 as ln
+    from lightnet_b200 import synth, zoo
+    be = ln.B200Backend(0)
+    cfg = zoo.yolov3_tiny_cfg(160, 96)
+    blob = synth.he_weights(ln.GpuExecutableNetwork(be, cfg, 2, ln.LN_F16).layers(), 3)
+    x = synth.uniform_images(2, 3, 96, 160, 4)
+
+    def heads(net):
+        net.forward(x)
+        return [be.download_f32(net.head(k)) for k in range(net.num_heads())]
+
+    ref_net = ln.GpuExecutableNetwork(be, cfg, 2, ln.LN_F16)
+    ref_net.load_weights(blob)
+    ref_net.set_cuda_graph(False)
+    want = heads(ref_net)
+    garbage = be.upload_f32((1, 1, 2048, 4096), np.full(2048 * 4096, 1e3, np.float32))  # what a block of the pool holds before it is packed
+    del garbage
+    refused = 0
+    for first in range(20, 60, 6):
+        for second in range(first, 60, 6):
+            net = ln.GpuExecutableNetwork(be, cfg, 2, ln.LN_F16)
+            net.load_weights(blob)
+            for n in (first, second):
+                be.debug_fail_alloc(n)
+                try:
+                    got = heads(net)
+                except ln.BackendError as e:
+                    assert "refused" in str(e)
+                    refused += 1
+                else:
+                    for g, w in zip(got, want):
+                        np.testing.assert_array_equal(g, w)
+            be.debug_fail_alloc(0)
+            for _ in range(3):
+                for g, w in zip(heads(net), want):
+                    np.testing.assert_array_equal(g, w)
+            del net
+    assert refused > 0
+    be.close()
