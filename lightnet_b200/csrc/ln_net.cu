@@ -719,12 +719,21 @@ int forward_f16(ln_net* net, const ln_tensor* input) {
         for (auto* t : net->heads) ln_tensor_retain(t);
         return LN_OK;
     }
-    ln_tensor* in16 = nullptr;
-    rc = ln_tensor_narrow_f16(ctx, input, &in16);
-    if (rc) return rc;
-    rc = forward_f16_layers(net, in16);
-    ln_tensor_release(in16);
-    g.seen = g.seen || rc == LN_OK;
+    auto by_operator = [&]() {
+        ln_tensor* in16 = nullptr;
+        int r = ln_tensor_narrow_f16(ctx, input, &in16);
+        if (r == LN_OK) r = forward_f16_layers(net, in16);
+        ln_tensor_release(in16);
+        g.seen = g.seen || r == LN_OK;
+        return r;
+    };
+    rc = by_operator();
+    if (rc == LN_ERR_CUDA && g.exec) {  // perhaps no room for a second set of outputs: without the graph and its set, once more
+        release_outputs(net);
+        release_heads(net);
+        release_graph_f16(net);
+        rc = by_operator();
+    }
     return rc;
 }
 

@@ -88,3 +88,34 @@ def test_first_forward_out_of_memory_then_capture_out_of_memory():
             del net
     assert refused > 0
     be.close()
+
+
+def test_kept_handle_and_no_room_for_a_second_set_of_outputs():
+    """A forward that may not replay the graph (a head of it is kept) and runs out of memory gives the graph's tensors back and succeeds."""
+    import lightnet_b200 as ln
+    from lightnet_b200 import synth, zoo
+    be = ln.B200Backend(0)
+    cfg = zoo.yolov3_tiny_cfg(160, 96)
+    nets = [ln.GpuExecutableNetwork(be, cfg, 2, ln.LN_F16) for _ in range(2)]
+    for net in nets:
+        net.load_weights(synth.he_weights(net.layers(), 3))
+    nets[1].set_cuda_graph(False)
+    x = [synth.uniform_images(2, 3, 96, 160, s) for s in range(2)]
+
+    def heads(net, x):
+        net.forward(x)
+        return [be.download_f32(net.head(k)) for k in range(net.num_heads())]
+
+    want = [heads(nets[1], v) for v in x]
+    for n in (1, 2, 11):
+        for _ in range(3):  # operator by operator, captured, replayed
+            heads(nets[0], x[0])
+        kept = nets[0].head(0)
+        be.debug_fail_alloc(n)
+        for g, w in zip(heads(nets[0], x[1]), want[1]):
+            np.testing.assert_array_equal(g, w)
+        be.debug_fail_alloc(0)
+        np.testing.assert_array_equal(be.download_f32(kept), want[0][0])
+        del kept
+    del nets, net
+    be.close()
