@@ -403,6 +403,8 @@ int32_t ln_debug_mma_peak_shape(ln_ctx* ctx, int32_t dtype, int32_t n, int32_t p
 int32_t ln_ctx_debug_cycles(ln_ctx* ctx, int64_t cycles[32]);
 /* The n-th request for device memory that the ctx makes from now on fails, once, as if the device had none left (0 = none does). */
 int32_t ln_debug_fail_alloc(ln_ctx* ctx, int64_t n);
+/* Forwards of the network so far whose layers were one launch of a captured graph (8-bit and binary16; the others ran kernel by kernel). */
+int64_t ln_debug_net_replays(const ln_net* net);
 
 #ifdef __cplusplus
 }

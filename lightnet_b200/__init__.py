@@ -160,6 +160,7 @@ SYMBOLS = {
     "ln_channel_affine_act_f16": (C.c_int32, [_VP, _VP, _VP, _VP, C.c_int64, C.c_int64, C.c_int32, _PP]),
     "ln_debug_score_key_error": (C.c_int32, [_VP, C.c_float, C.c_float, C.c_float, C.c_float, C.c_int32, C.c_int32, C.POINTER(C.c_uint32)]),
     "ln_ctx_debug_cycles": (C.c_int32, [_VP, _I64P]),
+    "ln_debug_net_replays": (C.c_int64, [_VP]),
     "ln_debug_fail_alloc": (C.c_int32, [_VP, C.c_int64]),
     "ln_modern_yolo_forward_f32": (C.c_int32, [_VP, _VP, C.c_int64, _VP]),
     "ln_modern_yolo_predecode_f32": (C.c_int32, [_VP, _VP, C.c_int64, C.c_int64, C.c_int32, _VP]),
@@ -725,6 +726,10 @@ class GpuExecutableNetwork:
         launches = np.zeros(8, np.int32)
         self.backend._check(self.lib.ln_net_profile(self.h, _ptr(per_layer), self.num_layers, _ptr(per_op), _ptr(launches)))
         return per_layer, {n: (float(per_op[i]), int(launches[i])) for i, n in enumerate(self.OP_CLASSES)}
+
+    def debug_replays(self):
+        """Forwards so far that launched a captured graph."""
+        return self.lib.ln_debug_net_replays(self.h)
 
     def last_times_ms(self):
         t = np.zeros(2, np.float32)

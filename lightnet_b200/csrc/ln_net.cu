@@ -296,10 +296,12 @@ struct ln_net {
         std::vector<std::pair<void*, size_t>> held;        // working memory of the captured kernels
         int64_t launches = 0;
         // seen: a forward has run to its end since the weights were loaded, so that every layer's weights are packed (the packing of a
-        // first use must not be captured: it would not have happened should the capture fail later on); failed: the capture failed
-        bool seen = false, failed = false;
+        // first use must not be captured: it would not have happened should the capture fail later on)
+        bool seen = false;
+        int failures = 0;                                  // captures that failed since the weights were loaded: no fourth one is tried
     };
     GraphF16 graph_f16;
+    int64_t replays = 0;  // forwards that were a graph launch (ln_debug_net_replays)
     // optional per-launch timing
     bool profile = false;
     std::vector<cudaEvent_t> prof_events;
@@ -652,7 +654,8 @@ int forward_f16_layers(ln_net* net, ln_tensor* in16) {
     return rc;
 }
 
-// Captures the layers of a second forward: graph_f16.exec ready to be launched, or graph_f16.failed and nothing kept.
+// Captures the layers of a second forward: graph_f16.exec ready to be launched, or nothing kept and one more in graph_f16.failures (the
+// forward then runs operator by operator and reports what is wrong itself; the next ones try again, since memory may have been short).
 int capture_f16(ln_net* net, const ln_tensor* input) {
     ln_ctx* ctx = net->ctx;
     ln_net::GraphF16& g = net->graph_f16;
@@ -676,8 +679,10 @@ int capture_f16(ln_net* net, const ln_tensor* input) {
         g.exec = nullptr;
         release_outputs(net);
         release_heads(net);
+        const int failures = g.failures + 1;
         release_graph_f16(net);
-        g.seen = g.failed = true;
+        g.seen = true;
+        g.failures = failures;
         return LN_OK;
     }
     std::map<ln_tensor*, int> refs;
@@ -701,7 +706,7 @@ int forward_f16(ln_net* net, const ln_tensor* input) {
     for (auto& L : net->layers)
         if (L.kind == K_CONV && !L.table_f16 && rc == LN_OK) rc = ln_conv_f16_table(ctx, L.b_f32, &L.table_f16);
     if (rc) return rc;
-    bool replay = net->use_graph && !g.failed && g.seen;
+    bool replay = net->use_graph && g.failures < 3 && g.seen;
     if (replay && g.exec) {
         for (auto& r : g.refs) replay = replay && r.first->refcount == r.second;
         if (replay) rc = ln_narrow_f16_into(ctx, input, g.input);  // upload_f16: the f32 input rounded to binary16 on the device
@@ -713,6 +718,7 @@ int forward_f16(ln_net* net, const ln_tensor* input) {
     if (replay) {
         LN_CUDA(ctx, cudaGraphLaunch(g.exec, ctx->stream));
         ctx->launches += g.launches;
+        net->replays++;
         net->out = g.out;
         net->heads = g.heads;
         for (auto* t : net->out) ln_tensor_retain(t);
@@ -1164,6 +1170,7 @@ int forward_any(ln_net* net, const ln_tensor* input, cudaEvent_t* around = nullp
                 if (g.used && g.input == input->ptr && g.exact == ctx->exact_epilogue) slot = &g;
             if (slot && slot->exec) {
                 LN_CUDA(ctx, cudaGraphLaunch(slot->exec, ctx->stream));
+                net->replays++;
                 ctx->launches += (int64_t)net->steps.size() * (net->batch / mb);
                 rc = LN_OK;
             } else if (!slot) {
@@ -1187,7 +1194,10 @@ int forward_any(ln_net* net, const ln_tensor* input, cudaEvent_t* around = nullp
                     if (e != cudaSuccess) { slot->exec = nullptr; rc = ln_fail(ctx, LN_ERR_CUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(e)); }
                 }
                 if (graph) cudaGraphDestroy(graph);
-                if (rc == LN_OK) LN_CUDA(ctx, cudaGraphLaunch(slot->exec, ctx->stream));
+                if (rc == LN_OK) {
+                    LN_CUDA(ctx, cudaGraphLaunch(slot->exec, ctx->stream));
+                    net->replays++;
+                }
             }
             slot->used = ++net->graph_clock;
         }
@@ -1769,6 +1779,8 @@ int32_t ln_net_profile(const ln_net* net, float* per_layer_ms, int32_t num_layer
     memcpy(per_op_launches, net->prof_op_launches, sizeof net->prof_op_launches);
     return LN_OK;
 }
+
+int64_t ln_debug_net_replays(const ln_net* net) { return net ? net->replays : 0; }
 
 int32_t ln_net_last_times(const ln_net* net, float times_ms[2]) {
     if (!net || !times_ms) return LN_ERR_ARG;

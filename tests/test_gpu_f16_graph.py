@@ -26,6 +26,7 @@ def test_captured_forward_keeps_values_and_handles():
     kept, kept_layer = None, None
     for i, x in enumerate(images):  # eager, captured, replayed, (two with handles kept across them), replayed
         nets[0].forward(x)
+        assert nets[0].debug_replays() == [0, 1, 2, 2, 2, 3][i]
         for got, ref in zip(heads(nets[0]), want[i]):
             np.testing.assert_array_equal(got, ref)
         if i == 2:
@@ -43,7 +44,28 @@ def test_captured_forward_keeps_values_and_handles():
             net.forward(x)
         for got, ref in zip(heads(nets[0]), heads(nets[1])):
             np.testing.assert_array_equal(got, ref)
+    assert nets[0].debug_replays() == 5 and nets[1].debug_replays() == 0
     del nets
+    be.close()
+
+
+def test_a_capture_that_failed_is_tried_again():
+    import lightnet_b200 as ln
+    from lightnet_b200 import synth, zoo
+    be = ln.B200Backend(0)
+    net = ln.GpuExecutableNetwork(be, zoo.yolov3_tiny_cfg(160, 96), 2, ln.LN_F16)
+    net.load_weights(synth.he_weights(net.layers(), 3))
+    x = synth.uniform_images(2, 3, 96, 160, 4)
+    net.forward(x)
+    want = be.download_f32(net.head(0))
+    be.debug_fail_alloc(12)  # in the middle of the captured layers
+    net.forward(x)
+    assert net.debug_replays() == 0
+    np.testing.assert_array_equal(be.download_f32(net.head(0)), want)
+    net.forward(x)
+    assert net.debug_replays() == 1
+    np.testing.assert_array_equal(be.download_f32(net.head(0)), want)
+    del net
     be.close()
 
 
