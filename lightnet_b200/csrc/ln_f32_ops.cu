@@ -5,6 +5,7 @@
 #include <cooperative_groups.h>
 
 #include "ln_common.h"
+#include "ln_conv_f32_plan.h"
 
 namespace cg = cooperative_groups;
 
@@ -388,7 +389,7 @@ __global__ void __launch_bounds__(BM * BN / 64, 32768 / (BM * BN)) conv2d_f32_ge
     conv_f32_finish<BM, BN, T>(p, sm.tile, f0, n0);
 }
 
-// Grouped convolutions: one thread per (pixel, group of FPT filters).  Semantics of runtime/forward_layers.rs:646-695: taps outside
+// Grouped convolutions, and sizes that the blocked kernels do not number (ln_conv_f32_blocked): one thread per (pixel, group of FPT filters).  Semantics of runtime/forward_layers.rs:646-695: taps outside
 // the image are skipped, groups partition channels, weights are [filters][C/groups][k][k].
 template <int FPT>
 __global__ void conv2d_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y, int B, int C,
@@ -749,7 +750,7 @@ int ln_conv2d_bias_act_f32(ln_ctx* ctx, const ln_tensor* x, const ln_tensor* wei
     if (!y) return LN_ERR_CUDA;
     const float* b = bias ? (const float*)bias->ptr : nullptr;
     int rc = LN_OK;
-    if (groups == 1 && x->n * oh * ow < (1ll << 30) && x->count() < (1ll << 40) && input_channels * kernel_size * kernel_size < (1ll << 24)) {
+    if (groups == 1 && ln_conv_f32_blocked(x->n, input_channels, input_height, input_width, filters, kernel_size, oh, ow)) {
         ConvF32 p = {};
         p.x = (const float*)x->ptr; p.w = (const float*)weights->ptr; p.bias = b; p.y = (float*)y->ptr;
         p.B = (int)x->n; p.C = (int)input_channels; p.H = (int)input_height; p.W = (int)input_width; p.F = (int)filters; p.k = (int)kernel_size;

@@ -45,3 +45,31 @@ def test_acc_shift_rule(tmp_path):
     args = [repr(float(v)) for c, _ in cases for v in c]
     out = subprocess.run([str(exe)] + args, check=True, capture_output=True, text=True).stdout.split()
     assert [int(v) for v in out] == [want for _, want in cases]
+
+
+F32_PROGRAM = r"""
+#include <cstdio>
+#include "ln_conv_f32_plan.h"
+int main() {
+    // n, c, h, w, f, k, oh, ow
+    printf("%d", ln_conv_f32_blocked(1, 1, 46400, 46400, 1, 1, 23200, 23200));  // a plane beyond 2^31 values, read with a stride
+    printf("%d", ln_conv_f32_blocked(1, 1, 46340, 46340, 1, 1, 23170, 23170));  // just below
+    printf("%d", ln_conv_f32_blocked(1, 3, 46400, 46400, 8, 3, 11600, 11600));
+    printf("%d", ln_conv_f32_blocked(1, 1, 32768, 32768, 1, 1, 32768, 32768));  // 2^30 output pixels
+    printf("%d", ln_conv_f32_blocked(4, 1 << 22, 1, 1, 8, 2, 1, 1));            // k range of 2^24
+    printf("%d\n", ln_conv_f32_blocked(64, 512, 19, 19, 1024, 3, 19, 19));
+    return 0;
+}
+"""
+
+
+def _run(tmp_path, program):
+    src, exe = tmp_path / "p.cpp", tmp_path / "p"
+    src.write_text(program)
+    subprocess.run(["g++", "-std=c++17", "-I" + os.path.join(ROOT, "lightnet_b200", "csrc"), str(src), "-o", str(exe)], check=True)
+    return subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_f32_convolutions_beyond_32_bit_indices_are_not_blocked(tmp_path):
+    assert _run(tmp_path, F32_PROGRAM) == ["010001"]
