@@ -706,7 +706,9 @@ int conv_f32_run(ln_ctx* ctx, ConvF32 p, bool one_chain, const char* who) {
                                  : (ks == 3 ? launch_conv_f32(ctx, conv2d_f32_gemm_kernel<32, 128, 3>, p, 64, 0, grid) : launch_conv_f32(ctx, conv2d_f32_gemm_kernel<32, 128, 0>, p, 64, 0, grid));
     else e = ks == 1 ? launch_conv_f32(ctx, conv2d_f32_gemm_kernel<64, 64, 1>, p, 64, 0, grid)
                      : (ks == 3 ? launch_conv_f32(ctx, conv2d_f32_gemm_kernel<64, 64, 3>, p, 64, 0, grid) : launch_conv_f32(ctx, conv2d_f32_gemm_kernel<64, 64, 0>, p, 64, 0, grid));
-    return e == cudaSuccess ? LN_OK : ln_fail(ctx, LN_ERR_CUDA, "%s launch: %s", who, cudaGetErrorString(e));
+    if (e == cudaSuccess) return LN_OK;
+    (void)cudaGetLastError();  // (the next launch is checked for its own error)
+    return ln_fail(ctx, LN_ERR_CUDA, "%s launch: %s", who, cudaGetErrorString(e));
 }
 
 }  // namespace

@@ -46,6 +46,14 @@ def test_conv2d_f32_tiles(be, geom):
     assert (np.abs(got - ref) <= (C * k * k + 33) * 2.0 ** -24 * size).all()
 
 
+@pytest.mark.parametrize("filters", [64 * 65535, 64 * 65535 + 1])
+def test_conv2d_f32_millions_of_filters(be, filters):
+    """The last filter tile that the grid of the blocked kernel numbers, and one filter more: a product per output, the same bits."""
+    w = np.random.default_rng(1).normal(0, 1, filters).astype(np.float32)
+    t = be.conv2d_f32(be.upload_f32((1, 1, 1, 1), np.full(1, 1.5, np.float32)), be.upload_f32((filters, 1, 1, 1), w), (1, filters, 1, 1), 1, 1, 1, filters, 1, 1, 1, 1, 0, 1)
+    np.testing.assert_array_equal(be.download_f32(t).ravel(), w * np.float32(1.5))
+
+
 def test_calibrated_scales_do_not_depend_on_the_batch(be):
     """One image, alone and eight times in a batch: the f32 convolutions cut their work differently, the scales stay bit for bit."""
     import lightnet_b200 as ln

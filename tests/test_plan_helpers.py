@@ -57,6 +57,8 @@ int main() {
     printf("%d", ln_conv_f32_blocked(1, 3, 46400, 46400, 8, 3, 11600, 11600));
     printf("%d", ln_conv_f32_blocked(1, 1, 32768, 32768, 1, 1, 32768, 32768));  // 2^30 output pixels
     printf("%d", ln_conv_f32_blocked(4, 1 << 22, 1, 1, 8, 2, 1, 1));            // k range of 2^24
+    printf("%d", ln_conv_f32_blocked(1, 1, 1, 1, 64 * 65535, 1, 1, 1));         // the last filter tile of the grid, and one more
+    printf("%d", ln_conv_f32_blocked(1, 1, 1, 1, 64 * 65535 + 1, 1, 1, 1));
     printf("%d\n", ln_conv_f32_blocked(64, 512, 19, 19, 1024, 3, 19, 19));
     return 0;
 }
@@ -72,4 +74,4 @@ def _run(tmp_path, program):
 
 @pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
 def test_f32_convolutions_beyond_32_bit_indices_are_not_blocked(tmp_path):
-    assert _run(tmp_path, F32_PROGRAM) == ["010001"]
+    assert _run(tmp_path, F32_PROGRAM) == ["01000101"]
