@@ -266,12 +266,12 @@ __global__ void __launch_bounds__(BM * BN / 64, 32768 / (BM * BN)) conv2d_f32_ge
         const int n = n0 + tid + j * T;
         const bool real = n < NP;
         const int b = n / P, r = n - b * P, oy = r / p.OW, ox = r - oy * p.OW;
-        oy0[j] = real ? oy * p.sy - p.pad : -(1 << 28);
+        oy0[j] = real ? oy * p.sy - p.pad : 0;
         ox0[j] = ox * p.sx - p.pad;
-        px[j] = p.x + ((int64_t)(real ? b : 0) * p.C + c_begin) * HW + (int64_t)(real ? oy0[j] : 0) * p.W + ox0[j];
-        inside[j] = 0u;
-        if (KS == 1) inside[j] = real ? 1u : 0u;
-        if (KS == 3)
+        px[j] = p.x + ((int64_t)(real ? b : 0) * p.C + c_begin) * HW + (int64_t)oy0[j] * p.W + ox0[j];
+        inside[j] = real ? 1u : 0u;  // (KS = 3: a bit per tap instead)
+        if (KS == 3) inside[j] = 0u;
+        if (KS == 3 && real)
 #pragma unroll
             for (int t = 0; t < 9; ++t) {
                 const int iy = oy0[j] + t / 3, ix = ox0[j] + t % 3;
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(BM * BN / 64, 32768 / (BM * BN)) conv2d_f32_ge
                     for (int i = 0; i < 8; ++i) {
                         const int kr = k0 + i, c = kr / (p.k * p.k), tap = kr - c * p.k * p.k, ky = tap / p.k, kx = tap - ky * p.k;
                         const int iy = oy0[j] + ky * p.dil, ix = ox0[j] + kx * p.dil;
-                        const bool ok = kr < k_end && iy >= 0 && iy < p.H && ix >= 0 && ix < p.W;
+                        const bool ok = inside[j] && kr < k_end && iy >= 0 && iy < p.H && ix >= 0 && ix < p.W;
                         gx[i][j] = ok ? __ldg(px[j] + (int64_t)c * HW + (int64_t)(ky * p.dil) * p.W + kx * p.dil) : 0.0f;
                     }
                 }

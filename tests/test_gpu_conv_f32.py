@@ -54,6 +54,16 @@ def test_conv2d_f32_millions_of_filters(be, filters):
     np.testing.assert_array_equal(be.download_f32(t).ravel(), w * np.float32(1.5))
 
 
+@pytest.mark.parametrize("filters", [3, 40])
+def test_conv2d_f32_dilation_far_beyond_the_image(be, filters):
+    """Only tap (0, 0) lies inside; the pixels of the tile behind the last output read nothing, however far the dilation reaches."""
+    rng = np.random.default_rng(filters)
+    x, w = rng.normal(0, 1, (1, 2, 5, 6)).astype(np.float32), rng.normal(0, 1, (filters, 2, 3, 3)).astype(np.float32)
+    t = be.conv2d_f32(be.upload_f32(x.shape, x), be.upload_f32(w.shape, w), (1, filters, 3, 4), 2, 5, 6, filters, 3, 1, 1, 1 << 27, 0, 1)
+    ref = np.einsum("fc,chw->fhw", w[:, :, 0, 0].astype(np.float64), x[0, :, :3, :4].astype(np.float64))
+    assert (np.abs(be.download_f32(t)[0] - ref) <= 35 * 2.0 ** -24 * 2 * np.abs(x).max() * np.abs(w).max()).all()
+
+
 def test_calibrated_scales_do_not_depend_on_the_batch(be):
     """One image, alone and eight times in a batch: the f32 convolutions cut their work differently, the scales stay bit for bit."""
     import lightnet_b200 as ln
