@@ -1488,7 +1488,9 @@ int ln_conv_umma_launch(ln_ctx* ctx, const ln_conv_umma_plan* plan) {
         else if (plan->kind == LN_KIND_F16) e = launch_small<LN_KIND_F16, false>(ctx, *plan);
         else e = exact ? launch_small<LN_KIND_F8, true>(ctx, *plan) : launch_small<LN_KIND_F8, false>(ctx, *plan);
         ctx->launches++;
-        return e == cudaSuccess ? LN_OK : ln_fail(ctx, LN_ERR_CUDA, "tensor-core convolution launch: %s", cudaGetErrorString(e));
+        if (e == cudaSuccess) return LN_OK;
+        (void)cudaGetLastError();  // (the next launch is checked for its own error)
+        return ln_fail(ctx, LN_ERR_CUDA, "tensor-core convolution launch: %s", cudaGetErrorString(e));
     }
     const bool two = plan->p.pipes == 2;
 #define LN_LAUNCH_KIND(K, X) (two ? launch_act<K, X, 2>(ctx, plan->p, plan->grid, plan->smem, ctx->stream) : launch_act<K, X, 1>(ctx, plan->p, plan->grid, plan->smem, ctx->stream))
