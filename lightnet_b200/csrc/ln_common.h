@@ -38,6 +38,7 @@ struct ln_ctx {
     int64_t fail_alloc = 0;                    // test aid: that many allocations from now one fails (ln_debug_fail_alloc)
     int* h_status = nullptr;  // status word in page-locked memory, written by kernels whose bounded waits give up
     ln_encode_tiled_fn encode_tiled = nullptr;
+    CUresult(CUDAAPI* pointer_attribute)(void*, CUpointer_attribute, CUdeviceptr) = nullptr;  // cuPointerGetAttribute
     long long* debug_cycles = nullptr;  // when set (LN_DEBUG_CYCLES=1), the tensor-core convolution records role timings of CTA 0
     std::set<const void*> configured_kernels;  // kernels whose dynamic shared memory limit has been raised
     // ln_ctx_set_kernel_timing: the operator-level convolution brackets its main kernel with these events

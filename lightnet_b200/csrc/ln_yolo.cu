@@ -1182,12 +1182,20 @@ int check_options(ln_ctx* ctx, YoloParams* p, const ln_detect_options* opts, con
 // Page-locked host memory of one call: image sizes in, outcome per image and records out.  Kernels read and write it directly.
 size_t stage_bytes(const YoloParams& p) { return (size_t)ln_round_up((int64_t)p.batch * 12, 128) + (size_t)p.batch * p.max_per_image * sizeof(ln_detection); }
 
-// Device address of page-locked host memory, or null for any other pointer.
-void* mapped_pointer(void* host) {
+// Device address of `bytes` of page-locked host memory that a kernel may write as floats; null when any of it is not (a caller may have
+// registered only the beginning of its array, and a kernel that runs past the end faults where a copy would have returned an error).
+void* mapped_floats(const ln_ctx* ctx, void* host, size_t bytes) {
     cudaPointerAttributes a;
     const bool ok = cudaPointerGetAttributes(&a, host) == cudaSuccess && a.type == cudaMemoryTypeHost && a.devicePointer;
     (void)cudaGetLastError();  // (an unregistered pointer is not an error here)
-    return ok ? a.devicePointer : nullptr;
+    if (!ok || ((uintptr_t)a.devicePointer & 3) != 0) return nullptr;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    const CUdeviceptr at = (CUdeviceptr)a.devicePointer;
+    if (ctx->pointer_attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) != CUDA_SUCCESS ||
+        ctx->pointer_attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS)
+        return nullptr;
+    return at >= start && at - start <= size && bytes <= size - (at - start) ? a.devicePointer : nullptr;
 }
 
 // The whole decode + NMS call over working memory that the caller provides (s.total bytes at `scratch`, 256-byte aligned).
@@ -1225,7 +1233,7 @@ int run_decode_nms(ln_ctx* ctx, const YoloParams& p, const Scratch& s, unsigned 
         counts = st + 2 * B;
         outcome = counts;
         // a caller that passes a page-locked record array gets its records written in place
-        if (void* m = mapped_pointer(records_host)) records = (float*)m;
+        if (void* m = mapped_floats(ctx, records_host, (size_t)B * p.max_per_image * sizeof(ln_detection))) records = (float*)m;
         else records = stage_records = (float*)((unsigned char*)stage + ln_round_up((int64_t)B * 12, 128));
     } else {
         LN_Y(cudaMemcpyAsync(dims, image_w, (size_t)B * 4, cudaMemcpyHostToDevice, ctx->stream));

@@ -162,3 +162,37 @@ def test_last_times_are_those_of_the_last_detect(be):
         assert net.last_times_ms() == before
     call()
     assert min(net.last_times_ms()) > 0.0
+
+
+def test_records_into_page_locked_arrays(be):
+    """Record arrays page-locked as a whole, in their first page only, and at an odd address: the records of an ordinary array."""
+    import torch
+    from lightnet_b200 import zoo
+    x = synth.uniform_images(4, 3, 96, 160, 7)
+    net = ln.GpuExecutableNetwork(be, zoo.yolov3_tiny_cfg(160, 96), 4, ln.LN_Q8)
+    net.load_weights(synth.he_weights(net.layers(), 3))
+    net.calibrate(x)
+    t = be.upload_f32(x.shape, x)
+    most = 600
+    ref = net.detect_device(t, 160, 96, 0.05, max_per_image=most)
+    assert sum(len(r) for r in ref) > 200  # beyond the first page
+    nbytes = 4 * most * 28
+
+    def check(address, keep):
+        import ctypes
+        rec = np.ndarray((4, most, 7), np.float32, (ctypes.c_uint8 * nbytes).from_address(address))
+        got = net.detect_device(t, 160, 96, 0.05, max_per_image=most, out=(rec, np.zeros(4, np.int32)))
+        for g, w in zip(got, ref):
+            np.testing.assert_array_equal(np.array(g), w)
+
+    pinned = torch.zeros(nbytes + 64, dtype=torch.uint8).pin_memory()
+    check(pinned.data_ptr(), pinned)
+    check(pinned.data_ptr() + 2, pinned)
+    plain = np.zeros(nbytes + 8192, np.uint8)
+    base = (plain.ctypes.data + 4095) & ~4095
+    rt = torch.cuda.cudart()
+    assert int(rt.cudaHostRegister(base, 4096, 0)) == 0
+    try:
+        check(base, plain)
+    finally:
+        rt.cudaHostUnregister(base)
