@@ -347,18 +347,21 @@ __global__ void __launch_bounds__(256) yolo_head_fill_kernel(const __grid_consta
     __shared__ float s_obj[256];
     __shared__ int s_stride[256];
     __shared__ int s_ca[256];   // slot index, with the head's new_coords flag in bit 31
-    __shared__ int s_n;
+    __shared__ int s_n, s_over;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int* fill = st.direct ? band_fill + img : pool_fill + img;
+    const int dst_cap = st.direct ? p.band_max : p.pool_max;
     if (lane == 0) s_cnt[warp] = 0;
-    if (threadIdx.x == 0) s_n = 0;
+    if (threadIdx.x == 0) {
+        s_n = 0;
+        s_over = *(volatile int*)fill > dst_cap;  // (other blocks are counting it up: one thread decides for the block)
+    }
     __syncthreads();
+    if (s_over) return;  // overflowed already: the image starts over, what is missing does not matter
     const ScanRange r = scan_range<1>(st);
     const unsigned kthr = conf_key(p.thr);
     const bool approx_ok = p.thr >= 1e-30f;
     unsigned long long* dst = st.direct ? band + (size_t)img * p.band_max : pool + (size_t)img * p.pool_max;
-    int* fill = st.direct ? band_fill + img : pool_fill + img;
-    const int dst_cap = st.direct ? p.band_max : p.pool_max;
-    if (*(volatile int*)fill > dst_cap) return;  // overflowed already: the image starts over, what is missing does not matter
     const int ca = blockIdx.x * blockDim.x + threadIdx.x;
     if (ca < p.total_ca) {
         const HeadDev& h = p.heads[find_head(p, ca)];
