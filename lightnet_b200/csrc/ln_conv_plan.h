@@ -140,6 +140,29 @@ inline bool ln_conv_choose_small(int sm_count, int kind, int64_t m, int64_t F, i
     return best >= 0;
 }
 
+constexpr int kMaxStages = 8;
+constexpr uint32_t kSmallSmem = 112u * 1024u;        // most shared memory of a CTA of the small-grid kernel: two fit an SM
+constexpr uint32_t kSmallClusterSmem = 77u * 1024u;  // least of one that waits for others of its cluster: three do not fit
+constexpr uint32_t kSmallBarBytes = 160u;            // full[8] empty[8] done | tmem slot | abort flag
+constexpr uint32_t kPieceBytes = 4096u;              // 32 rows x 32 columns of partial sums, [4 columns][row]: consecutive lanes, consecutive 16 bytes
+
+// Shared memory of a CTA of the small-grid kernel, and what it is for: the ring of stages or the tile's partial sums, whichever is larger, then
+// barriers and table.  An int8 CTA allocates up to 256 of an SM's 512 TMEM columns and waits while there are none; the CTAs of a cluster
+// wait for each other besides.  With a third such CTA on every SM two clusters could each hold what the other one waits for, so a
+// cluster launch asks for more than a third of an SM's 228 KB (of which every CTA takes 1 KB for itself).
+inline size_t ln_conv_small_smem(int bk, int bn, int ksplit, int kblocks, int* stages, int* region) {
+    const int share = (kblocks + ksplit - 1) / ksplit;  // k-blocks of a CTA, rounded up
+    const uint32_t stage = (uint32_t)(128 + bn) * bk, partial = ksplit > 1 ? (uint32_t)(bn / 8) * kPieceBytes : 0u;
+    const uint32_t rest = 1024u /*alignment slack*/ + kSmallBarBytes + (uint32_t)bn * 8u;
+    *stages = (int)((kSmallSmem - rest) / stage);
+    if (*stages > kMaxStages) *stages = kMaxStages;
+    if (*stages > share) *stages = share;
+    const uint32_t ring = (uint32_t)*stages * stage;
+    *region = (int)(ring > partial ? ring : partial);
+    const uint32_t all = (uint32_t)*region + rest;
+    return ksplit > 1 && all < kSmallClusterSmem ? kSmallClusterSmem : all;
+}
+
 bool ln_conv_umma_supported(int64_t channels_padded, int64_t k, int64_t stride_x, int64_t stride_y, int64_t dilation, int64_t groups,
                             int64_t in_w, int64_t in_h);
 // plan->mb must point at device storage for fpad float2 before the build.

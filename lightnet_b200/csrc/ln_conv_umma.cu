@@ -28,7 +28,6 @@
 
 namespace {
 
-constexpr int kMaxStages = 8;
 #ifndef LN_EPILOGUE_GROUPS
 #define LN_EPILOGUE_GROUPS 4
 #endif
@@ -602,7 +601,8 @@ __global__ void __launch_bounds__(conv_threads(PIPES), 1) conv_umma_kernel(const
 //     i % ksplit, which adds the parts up through distributed shared memory -- int32 sums, the same bits in any order -- and runs the
 //     epilogue on it.  FP8 and binary16 keep one chain per output, so their results stay the same bits (a split moved binary16 heads of
 //     deep networks by up to 0.8 %: every layer's rounding carries it on).
-//   - 320 threads, bn columns of TMEM (int8: twice that) and at most 112 KB of shared memory: two CTAs fit an SM, so that in a network (plan.chained)
+//   - 320 threads, bn columns of TMEM (int8: twice that) and at most 112 KB of shared memory: two CTAs fit an SM (and never three of a
+//     cluster launch, see ln_conv_small_smem), so that in a network (plan.chained)
 //     the next layer's CTAs can set up, fetch their table and start their weight loads while this layer still runs; griddepcontrol.wait
 //     stands in front of everything that the layers before it write or still read.
 // One tile per CTA, no persistent loop.
@@ -610,8 +610,6 @@ __global__ void __launch_bounds__(conv_threads(PIPES), 1) conv_umma_kernel(const
 // C512 -> K256 at 38 x 38 9.5 -> 7.5 us, 3x3 C512 -> K1024 at 19 x 19 25 -> 15 us as single cold launches.
 constexpr int kSmallEpilogueWarps = 8;
 constexpr int kSmallThreads = 32 * (2 + kSmallEpilogueWarps);
-constexpr uint32_t kSmallBarBytes = 160u;  // full[8] empty[8] done | tmem slot | abort flag
-constexpr uint32_t kPieceBytes = 4096u;    // 32 rows x 32 columns of partial sums, [4 columns][row]: consecutive lanes, consecutive 16 bytes
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
@@ -916,7 +914,6 @@ __global__ void __launch_bounds__(128, 1) mma_peak_kernel(int iters, int n, int 
 }
 
 constexpr int kMaxDynamicSmem = 227 * 1024;
-constexpr uint32_t kSmallSmem = 112u * 1024u;     // of a CTA of the small-grid kernel: two fit an SM
 constexpr uint32_t kMaxTableBytes = 32u * 1024u;  // {multiplier, bias} pairs of at most 4096 filters
 
 template <int KIND, bool EXACT, int PIPES>
@@ -1293,15 +1290,7 @@ int ln_conv_umma_plan_build(ln_ctx* ctx, ln_conv_umma_plan* plan, const ln_conv_
     // weights stay in shared memory when there is a single filter tile and they leave room for at least four activation stages
     if (small) {
         p.ksplit = ksplit;
-        const int share = (g.k * g.k * p.cblocks + ksplit - 1) / ksplit;  // k-blocks of a CTA, rounded up
-        const uint32_t stage = (uint32_t)(128 + bn) * bk, partial = ksplit > 1 ? (uint32_t)(bn / 8) * kPieceBytes : 0u;
-        const uint32_t rest = 1024u /*alignment slack*/ + kSmallBarBytes + (uint32_t)bn * 8u;
-        p.stages = (int)((kSmallSmem - rest) / stage);
-        if (p.stages > kMaxStages) p.stages = kMaxStages;
-        if (p.stages > share) p.stages = share;
-        const uint32_t ring = (uint32_t)p.stages * stage;
-        p.small_region = (int)(ring > partial ? ring : partial);
-        plan->smem = (size_t)p.small_region + rest;
+        plan->smem = ln_conv_small_smem(bk, bn, ksplit, g.k * g.k * p.cblocks, &p.stages, &p.small_region);
         plan->grid = p.num_tiles * ksplit;
     } else if (p.halo) {
         const uint32_t box = (uint32_t)p.box_bytes, b_bytes = (uint32_t)bn * bk;

@@ -102,7 +102,7 @@ PROGRAM = r"""
 #include <cstdio>
 #include "ln_conv_plan.h"
 int main() {
-    long n = 0, split = 0;
+    long n = 0, split = 0, padded = 0;
     for (int kind = 0; kind < 3; ++kind)
         for (int m = 1; m <= 400; m += m < 8 ? 1 : 7)
             for (int F = 1; F <= 1100; F += F < 300 ? 31 : 97)
@@ -122,8 +122,17 @@ int main() {
                             printf("bad choice kind %d m %d F %d kb %d bk %d: bn %d ks %d\n", kind, m, F, kb, bk, bn, ks);
                             return 1;
                         }
+                        // two CTAs fit an SM (228 KB, 1 KB of it per CTA), and three of a cluster launch never do: each may hold half of its TMEM
+                        int stages = 0, region = 0;
+                        const long smem = (long)ln_conv_small_smem(bk, bn, ks, kb, &stages, &region), sm = 228 * 1024;
+                        padded += smem > region + 1024 + (long)kSmallBarBytes + bn * 8;
+                        if (2 * (smem + 1024) > sm || (ks > 1 && 3 * (smem + 1024) <= sm) || stages < 1 || stages > kMaxStages || region < stages * (128 + bn) * bk ||
+                            (ks > 1 && region < bn / 8 * (long)kPieceBytes) || smem < region + 1024 + (long)kSmallBarBytes + bn * 8) {
+                            printf("bad shared memory: bn %d ks %d kb %d bk %d: %ld bytes, %d stages, region %d\n", bn, ks, kb, bk, smem, stages, region);
+                            return 1;
+                        }
                     }
-    printf("%d\n", n > 1000 && split > 100);
+    printf("%d\n", n > 1000 && split > 100 && padded > 0);
     return 0;
 }
 """
