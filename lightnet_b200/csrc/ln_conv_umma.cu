@@ -957,7 +957,7 @@ cudaError_t launch_small(ln_ctx* ctx, const ln_conv_umma_plan& plan) {
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = plan.chained ? 2 : 1;
+    cfg.numAttrs = plan.chained && !p.debug ? 2 : 1;  // (with role timing on, a memset comes first)
 #define LN_LAUNCH_ACT(A)                                                                                             \
     case A: {                                                                                                        \
         auto k = conv_umma_small_kernel<KIND, A, EXACT>;                                                              \
@@ -1473,6 +1473,7 @@ int ln_conv_umma_launch(ln_ctx* ctx, const ln_conv_umma_plan* plan) {
     cudaError_t e;
     const bool exact = ctx->exact_epilogue;
     if (plan->p.ksplit) {
+        if (plan->p.debug) LN_CUDA(ctx, cudaMemsetAsync(plan->p.debug, 0, 32 * sizeof(long long), ctx->stream));  // (this kernel records none: not those of an earlier layer)
         if (plan->kind == LN_KIND_I8) e = exact ? launch_small<LN_KIND_I8, true>(ctx, *plan) : launch_small<LN_KIND_I8, false>(ctx, *plan);
         else if (plan->kind == LN_KIND_F16) e = launch_small<LN_KIND_F16, false>(ctx, *plan);
         else e = exact ? launch_small<LN_KIND_F8, true>(ctx, *plan) : launch_small<LN_KIND_F8, false>(ctx, *plan);
