@@ -9,3 +9,33 @@
 inline bool ln_conv_f32_blocked(int64_t n, int64_t c, int64_t h, int64_t w, int64_t f, int64_t k, int64_t oh, int64_t ow) {
     return n * oh * ow < (1ll << 30) && h * w < (1ll << 31) && n * c * h * w < (1ll << 40) && c * k * k < (1ll << 24) && (f + 63) / 64 <= 65535;
 }
+
+// Slice of the k range that a kernel holds in shared memory: four channels of a 3x3 kernel or 32 of a 1x1 one where operands are copied
+// asynchronously (`async`), else one channel, or eight k of any other kernel (ks = 1: 1x1 without padding, 3: 3x3 without dilation, 0: anything).
+constexpr int ln_conv_f32_slice(bool async, int ks) { return async ? (ks == 3 ? 36 : 32) : (ks == 3 ? 9 : 8); }
+
+// Part z of a k range of `slices` slices cut into `parts` begins with this one: whole slices, as evenly as they go.
+constexpr int ln_conv_f32_first_slice(int slices, int z, int parts) { return slices * z / parts; }  // (at most 2^21 slices)
+
+struct ln_conv_f32_cut {
+    int bm, bn, parts;  // filters and pixels of a tile; CTAs of the cluster over which a tile's k range is split
+};
+
+// Ungrouped convolution with optional bias and activation.  Tile: 64 filters x 128 pixels while that gives every SM four CTAs (of four
+// warps) even without splitting, 64 x 64 below; layers of at most 32 filters 32 x 128.  The k range is split over clusters of up to eight
+// CTAs until there are about eight CTAs of two warps per SM, in parts of at least two slices (four
+// of the short ones of operands staged through registers).
+// one_chain: no split, so that every output is one chain of fused multiply-adds whatever the batch and the number of SMs.  Calibration
+// asks for it: the scales of an 8-bit network, and with them its codes, must not depend on how the work was cut.
+inline ln_conv_f32_cut ln_conv_f32_choose(int sm_count, int64_t images, int64_t plane, int64_t F, int64_t K, int ks, bool async, bool one_chain) {
+    const int64_t NP = images * plane, tail = (NP + 127) / 128 * 128 - NP;
+    const bool narrow = !async && F <= 32;
+    auto tiles = [&](int bm, int bn) { return ((NP + bn - 1) / bn) * ((F + bm - 1) / bm); };
+    const bool wide = async && tail * 10 <= NP && tiles(64, 128) * 8 >= 2ll * sm_count;
+    ln_conv_f32_cut c;
+    c.bm = narrow ? 32 : 64;
+    c.bn = narrow || wide ? 128 : 64;
+    c.parts = 1;
+    while (!one_chain && c.parts < 8 && tiles(c.bm, c.bn) * c.parts * 2 <= (wide ? 4ll : 8ll) * sm_count && K / (c.parts * 2) >= (async ? 2 : 4) * ln_conv_f32_slice(async, ks)) c.parts *= 2;
+    return c;
+}

@@ -25,7 +25,6 @@ struct ConvF32 {
     const float* bias;  // null = none
     float* y;
     int B, C, H, W, F, k, sx, sy, dil, pad, OH, OW, K, act;
-    int k_part;  // k range of one part, a multiple of the slice
 };
 
 __device__ __forceinline__ unsigned long long fma2_f32(unsigned long long a, unsigned long long b, unsigned long long c) {
@@ -114,7 +113,7 @@ __device__ __forceinline__ void conv_f32_finish(const ConvF32& p, float (&tile)[
 // FMAs --, 139 us with weights transposed into shared memory four bytes at a time: the scatter filled the shared-memory port.)
 template <int BN, int KS>
 struct ConvF32Shared {
-    static constexpr int SL = KS == 3 ? 36 : 32, WL = SL + 4;
+    static constexpr int SL = ln_conv_f32_slice(true, KS), WL = SL + 4;
     union {
         struct { float w[2][64][WL]; float x[2][SL][BN]; } op;
         float tile[64][BN];
@@ -130,7 +129,8 @@ __global__ void __launch_bounds__(BN, 512 / BN) conv2d_f32_async_kernel(const __
     const int tid = (int)threadIdx.x, tx = tid % TX, ty = tid / TX;
     const int P = p.OH * p.OW, HW = p.H * p.W, NP = p.B * P;
     const int n0 = (int)blockIdx.x * BN, f0 = (int)blockIdx.y * 64;
-    const int k_begin = (int)blockIdx.z * p.k_part, k_end = min(p.K, k_begin + p.k_part);
+    const int slices = (p.K + SL - 1) / SL, z = (int)blockIdx.z, parts = (int)gridDim.z;
+    const int k_begin = ln_conv_f32_first_slice(slices, z, parts) * SL, k_end = min(p.K, ln_conv_f32_first_slice(slices, z + 1, parts) * SL);
     // this thread's pixel: address of tap (0, 0) of the first channel of the range, and the taps inside the image as 4-byte copy sizes
     const int n = n0 + tid;
     const bool real = n < NP;
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(BN, 512 / BN) conv2d_f32_async_kernel(const __
     for (int m = 0; m < 8; ++m)
 #pragma unroll
         for (int q = 0; q < 4; ++q) acc[m][q] = 0ull;
-    if (k_begin < k_end) copy_slice(k_begin, 0);  // (rounding the parts to whole slices can leave the last one empty)
+    copy_slice(k_begin, 0);
     int buf = 0;
     for (int k0 = k_begin; k0 < k_end; k0 += SL) {
         if (k0 + SL < k_end) {
@@ -241,11 +241,9 @@ __global__ void __launch_bounds__(BN, 512 / BN) conv2d_f32_async_kernel(const __
 
 // Layers of few filters and every other geometry: BM filters x BN pixels, operands staged through registers (the weights with 4-byte
 // copies), slices of one channel for 3x3 kernels (KS = 3) and of eight k otherwise (KS = 1: 1x1 without padding, 0: anything).
-constexpr int conv_slice(int ks) { return ks == 3 ? 9 : 8; }
-
 template <int BM, int BN, int KS>
 __global__ void __launch_bounds__(BM * BN / 64, 32768 / (BM * BN)) conv2d_f32_gemm_kernel(const __grid_constant__ ConvF32 p) {
-    constexpr int T = BM * BN / 64, TX = BN / 8, SL = conv_slice(KS);
+    constexpr int T = BM * BN / 64, TX = BN / 8, SL = ln_conv_f32_slice(false, KS);
     static_assert(BN % T == 0, "every thread gathers whole columns of x");
     constexpr int PIX = BN / T;                   // pixels a thread gathers
     constexpr int WQ = (BM * SL + T - 1) / T;     // weights a thread copies: element tid + q * T of [filter][k of the slice]
@@ -255,7 +253,8 @@ __global__ void __launch_bounds__(BM * BN / 64, 32768 / (BM * BN)) conv2d_f32_ge
     const int tid = (int)threadIdx.x, tx = tid % TX, ty = tid / TX;
     const int P = p.OH * p.OW, HW = p.H * p.W, NP = p.B * P;
     const int n0 = (int)blockIdx.x * BN, f0 = (int)blockIdx.y * BM;
-    const int k_begin = (int)blockIdx.z * p.k_part, k_end = min(p.K, k_begin + p.k_part);
+    const int slices = (p.K + SL - 1) / SL, z = (int)blockIdx.z, parts = (int)gridDim.z;
+    const int k_begin = ln_conv_f32_first_slice(slices, z, parts) * SL, k_end = min(p.K, ln_conv_f32_first_slice(slices, z + 1, parts) * SL);
     // the pixels this thread gathers: address of tap (0, 0) of the first channel of the range, and which taps are inside the image
     const float* px[PIX];
     unsigned inside[PIX];
@@ -343,11 +342,9 @@ __global__ void __launch_bounds__(BM * BN / 64, 32768 / (BM * BN)) conv2d_f32_ge
     for (int m = 0; m < 4; ++m)
 #pragma unroll
         for (int n = 0; n < 8; ++n) acc[m][n] = 0ull;
-    if (k_begin < k_end) {  // (rounding the parts to whole slices can leave the last one empty)
-        copy_weights(k_begin, 0);
-        fetch(k_begin);
-        store(0);
-    }
+    copy_weights(k_begin, 0);
+    fetch(k_begin);
+    store(0);
     __syncthreads();
     int buf = 0;
     for (int k0 = k_begin; k0 < k_end; k0 += SL) {
@@ -679,24 +676,14 @@ cudaError_t launch_conv_f32(ln_ctx* ctx, K kernel, const ConvF32& p, int threads
     return cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
-// Ungrouped convolution with optional bias and activation.  Tile: 64 filters x 128 pixels while that gives every SM four CTAs (of four
-// warps) even without splitting, 64 x 64 below; layers of at most 32 filters 32 x 128.  The k range is split over clusters of up to eight
-// CTAs until there are about eight CTAs of two warps per SM, in parts of at least two slices.
-// one_chain: no split, so that every output is one chain of fused multiply-adds whatever the batch and the number of SMs.  Calibration
-// asks for it: the scales of an 8-bit network, and with them its codes, must not depend on how the work was cut.
+// Ungrouped convolution with optional bias and activation, cut as ln_conv_f32_choose says.
 int conv_f32_run(ln_ctx* ctx, ConvF32 p, bool one_chain, const char* who) {
     const int64_t NP = (int64_t)p.B * p.OH * p.OW;
     const int ks = p.k == 1 && p.pad == 0 ? 1 : (p.k == 3 && p.dil == 1 ? 3 : 0);
     const bool async = ks != 0 && p.F > 32 && (p.K & 3) == 0 && (((uintptr_t)p.w) & 15) == 0;
-    auto tiles = [&](int bm, int bn) { return ((NP + bn - 1) / bn) * ((p.F + bm - 1) / bm); };
-    const bool narrow = !async && p.F <= 32;
-    const int64_t tail = ln_round_up(NP, 128) - NP;
-    const bool wide = async && tail * 10 <= NP && tiles(64, 128) * 8 >= 2ll * ctx->sm_count;
-    const int bm = narrow ? 32 : 64, bn = narrow || wide ? 128 : 64, slice = async ? (ks == 3 ? 36 : 32) : conv_slice(ks);
-    int parts = 1;
-    while (!one_chain && parts < 8 && tiles(bm, bn) * parts * 2 <= (wide ? 4ll : 8ll) * ctx->sm_count && p.K / (parts * 2) >= (async ? 2 : 4) * slice) parts *= 2;
-    p.k_part = (int)ln_round_up((p.K + parts - 1) / parts, slice);
-    const dim3 grid((unsigned)((NP + bn - 1) / bn), (unsigned)((p.F + bm - 1) / bm), (unsigned)parts);
+    const ln_conv_f32_cut cut = ln_conv_f32_choose(ctx->sm_count, p.B, (int64_t)p.OH * p.OW, p.F, p.K, ks, async, one_chain);
+    const bool wide = async && cut.bn == 128, narrow = cut.bm == 32;
+    const dim3 grid((unsigned)((NP + cut.bn - 1) / cut.bn), (unsigned)((p.F + cut.bm - 1) / cut.bm), (unsigned)cut.parts);
     cudaError_t e;
     if (wide) e = ks == 1 ? launch_conv_f32(ctx, conv2d_f32_async_kernel<128, 1>, p, 128, sizeof(ConvF32Shared<128, 1>), grid)
                           : launch_conv_f32(ctx, conv2d_f32_async_kernel<128, 3>, p, 128, sizeof(ConvF32Shared<128, 3>), grid);

@@ -75,3 +75,44 @@ def _run(tmp_path, program):
 @pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
 def test_f32_convolutions_beyond_32_bit_indices_are_not_blocked(tmp_path):
     assert _run(tmp_path, F32_PROGRAM) == ["01000101"]
+
+
+F32_CUT_PROGRAM = r"""
+#include <cstdio>
+#include <initializer_list>
+#include "ln_conv_f32_plan.h"
+int main() {
+    long split = 0, uneven = 0;
+    for (int ks : {0, 1, 3})
+        for (int async = 0; async <= (ks ? 1 : 0); ++async)
+            for (long F : {8, 33, 70, 255, 512})
+                for (long plane : {1, 49, 361, 1444, 23104})
+                    for (long images : {1, 3, 16})
+                        for (int c = 4; c <= 1100; c += c < 80 ? 4 : 52) {
+                            const int K = c * (ks == 1 ? 1 : 9), SL = ln_conv_f32_slice(async, ks), slices = (K + SL - 1) / SL;
+                            if (async && F <= 32) continue;
+                            const ln_conv_f32_cut cut = ln_conv_f32_choose(148, images, plane, F, K, ks, async, false);
+                            split += cut.parts > 1;
+                            int most = 0, least = 1 << 30;
+                            for (int z = 0; z < cut.parts; ++z) {
+                                const int n = ln_conv_f32_first_slice(slices, z + 1, cut.parts) - ln_conv_f32_first_slice(slices, z, cut.parts);
+                                most = n > most ? n : most;
+                                least = n < least ? n : least;
+                            }
+                            uneven += most != least;
+                            if (ln_conv_f32_first_slice(slices, 0, cut.parts) != 0 || ln_conv_f32_first_slice(slices, cut.parts, cut.parts) != slices || least < 1 || most - least > 1 ||
+                                (cut.parts > 1 && least < (async ? 2 : 4)) || ln_conv_f32_choose(148, images, plane, F, K, ks, async, true).parts != 1) {
+                                printf("ks %d async %d F %ld plane %ld images %ld c %d: %d parts of %d to %d slices\n", ks, async, F, plane, images, c, cut.parts, least, most);
+                                return 0;
+                            }
+                        }
+    printf("%d\n", split > 500 && uneven > 200);
+    return 0;
+}
+"""
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_f32_k_ranges_are_split_evenly(tmp_path):
+    """Every CTA of a cluster has slices to sum, as many as the others or one more or less."""
+    assert _run(tmp_path, F32_CUT_PROGRAM) == ["1"]
