@@ -60,6 +60,24 @@ __device__ __forceinline__ bool conv_f32_border(const ConvF32& p, int r) {
     return iy0 < 0 || ix0 < 0 || iy0 + reach >= p.H || ix0 + reach >= p.W;
 }
 
+// The groups of four outputs that a thread of conv_f32_finish found a NaN in (bit = its turn) and left in y as plain sums: NaNs next to the
+// border summed again, then bias and activation.  Out of line: inside the loop that hands tiles over it cost 1 % of a forward.
+template <int BN, int T>
+__device__ __noinline__ void conv_f32_finish_nan(const ConvF32& p, unsigned bad, int m0, int f0, int n0) {
+    const int P = p.OH * p.OW, NP = p.B * P;
+    for (; bad; bad &= bad - 1u) {
+        const int i = (int)threadIdx.x + (__ffs(bad) - 1) * T, f = f0 + m0 + i / (BN / 4), n = n0 + i % (BN / 4) * 4;
+        const float bias = p.bias ? __ldg(p.bias + f) : 0.0f;
+        for (int j = 0; j < 4 && n + j < NP; ++j) {
+            const int b = (n + j) / P, r = n + j - b * P;
+            float* y = p.y + ((int64_t)b * p.F + f) * P + r;
+            float v = *y;
+            if (isnan(v) && conv_f32_border(p, r)) v = conv_f32_taps(p, b, f, r);
+            *y = ln_act_f32(p.act, p.bias ? v + bias : v);
+        }
+    }
+}
+
 // Hands the CTA's tile (one per part of a split k range, side by side in distributed shared memory) to y: the parts added up in order,
 // bias, activation, 16-byte stores where the planes allow them.  Called by all threads after the tile is written.
 template <int BM, int BN, int T>
@@ -69,7 +87,9 @@ __device__ __forceinline__ void conv_f32_finish(const ConvF32& p, float (&tile)[
     if (parts > 1) cluster.sync();
     else __syncthreads();
     const bool vec = (P & 3) == 0;  // four consecutive pixels lie in one image then, at a 16-byte boundary
-    for (int i = (int)threadIdx.x; i < share * (BN / 4); i += T) {
+    static_assert(BM * (BN / 4) <= 32 * T, "a bit for every turn of the loop");
+    unsigned bad = 0u, turn = 1u;
+    for (int i = (int)threadIdx.x; i < share * (BN / 4); i += T, turn <<= 1) {
         const int m = (int)blockIdx.z * share + i / (BN / 4), c = i % (BN / 4) * 4, f = f0 + m, n = n0 + c;
         if (f >= p.F || n >= NP) continue;
         float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -77,15 +97,12 @@ __device__ __forceinline__ void conv_f32_finish(const ConvF32& p, float (&tile)[
             const float4 q = *reinterpret_cast<const float4*>(parts > 1 ? cluster.map_shared_rank(&tile[m][c], s) : &tile[m][c]);
             v[0] += q.x; v[1] += q.y; v[2] += q.z; v[3] += q.w;
         }
-        if (isnan(v[0] + v[1] + v[2] + v[3])) {  // (false alarms, inf - inf, end in the conditions below)
-            for (int j = 0; j < 4; ++j) {
-                const int bj = (n + j) / P, r = n + j - bj * P;
-                if (n + j < NP && isnan(v[j]) && conv_f32_border(p, r)) v[j] = conv_f32_taps(p, bj, f, r);
-            }
-        }
-        const float bias = p.bias ? __ldg(p.bias + f) : 0.0f;
+        if (isnan(v[0] + v[1] + v[2] + v[3])) bad |= turn;  // (inf - inf too, which does no harm)
+        else {
+            const float bias = p.bias ? __ldg(p.bias + f) : 0.0f;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = ln_act_f32(p.act, p.bias ? v[j] + bias : v[j]);
+            for (int j = 0; j < 4; ++j) v[j] = ln_act_f32(p.act, p.bias ? v[j] + bias : v[j]);
+        }
         const int b = n / P;
         if (vec) *reinterpret_cast<float4*>(p.y + ((int64_t)b * p.F + f) * P + (n - b * P)) = make_float4(v[0], v[1], v[2], v[3]);
         else {
@@ -97,6 +114,7 @@ __device__ __forceinline__ void conv_f32_finish(const ConvF32& p, float (&tile)[
                 }
         }
     }
+    if (bad) conv_f32_finish_nan<BN, T>(p, bad, (int)blockIdx.z * share, f0, n0);
     if (parts > 1) cluster.sync();  // nobody leaves while its tile is being read
 }
 
