@@ -23,19 +23,22 @@ struct ln_conv_f32_cut {
 
 // Ungrouped convolution with optional bias and activation.  Tile: 64 filters x 128 pixels while that gives every SM four CTAs (of four
 // warps) even without splitting, 64 x 64 below; layers of at most 32 filters 32 x 128.  The k range is split over clusters of up to eight
-// CTAs until there are about eight CTAs of two warps per SM, in parts of at least two slices (four
-// of the short ones of operands staged through registers).
-// one_chain: no split, so that every output is one chain of fused multiply-adds whatever the batch and the number of SMs.  Calibration
-// asks for it: the scales of an 8-bit network, and with them its codes, must not depend on how the work was cut.
+// CTAs until a single image has about eight CTAs of two warps per SM of a B200, in parts of at least two slices (four of the short ones of
+// operands staged through registers).  The split looks at one image and not at the batch: it is what the order of a sum depends on, and an
+// image has the same outputs in any batch.
+// one_chain: no split, so that every output is one chain of fused multiply-adds.  Calibration asks for it: the scales of an 8-bit
+// network, and with them its codes, must not depend on how the work was cut.
 inline ln_conv_f32_cut ln_conv_f32_choose(int sm_count, int64_t images, int64_t plane, int64_t F, int64_t K, int ks, bool async, bool one_chain) {
-    const int64_t NP = images * plane, tail = (NP + 127) / 128 * 128 - NP;
     const bool narrow = !async && F <= 32;
-    auto tiles = [&](int bm, int bn) { return ((NP + bn - 1) / bn) * ((F + bm - 1) / bm); };
-    const bool wide = async && tail * 10 <= NP && tiles(64, 128) * 8 >= 2ll * sm_count;
+    auto tiles = [&](int64_t pixels, int bm, int bn) { return ((pixels + bn - 1) / bn) * ((F + bm - 1) / bm); };
+    auto wide = [&](int64_t pixels, int sms) { return async && ((pixels + 127) / 128 * 128 - pixels) * 10 <= pixels && tiles(pixels, 64, 128) * 8 >= 2ll * sms; };
     ln_conv_f32_cut c;
     c.bm = narrow ? 32 : 64;
-    c.bn = narrow || wide ? 128 : 64;
+    c.bn = narrow || wide(images * plane, sm_count) ? 128 : 64;
+    constexpr int kSms = 148;
+    const bool wide1 = wide(plane, kSms);
+    const int64_t tiles1 = tiles(plane, c.bm, narrow || wide1 ? 128 : 64), most = (wide1 ? 4ll : 8ll) * kSms;
     c.parts = 1;
-    while (!one_chain && c.parts < 8 && tiles(c.bm, c.bn) * c.parts * 2 <= (wide ? 4ll : 8ll) * sm_count && K / (c.parts * 2) >= (async ? 2 : 4) * ln_conv_f32_slice(async, ks)) c.parts *= 2;
+    while (!one_chain && c.parts < 8 && tiles1 * c.parts * 2 <= most && K / (c.parts * 2) >= (async ? 2 : 4) * ln_conv_f32_slice(async, ks)) c.parts *= 2;
     return c;
 }

@@ -118,3 +118,35 @@ def test_conv2d_f32_weights_that_are_not_finite(be, geom):
     np.testing.assert_array_equal(np.isinf(got) * np.sign(np.nan_to_num(got)), np.isinf(ref) * np.sign(np.nan_to_num(ref)))
     ok = np.isfinite(ref)
     assert (np.abs(got[ok] - ref[ok]) <= (C * k * k + 33) * 2.0 ** -24 * size[ok]).all()
+
+
+@pytest.mark.parametrize("geom", [(512, 13, 13, 256, 3), (256, 26, 20, 512, 1), (1024, 4, 4, 255, 1), (68, 19, 21, 40, 3), (7, 20, 23, 9, 5), (35, 30, 30, 17, 3)])
+def test_conv2d_f32_does_not_depend_on_the_batch(be, geom):
+    """An image has the same bits alone and as any of 2, 9 or 40 images: the order of a sum is cut by the size of one image."""
+    C, H, W, F, k = geom
+    rng = np.random.default_rng(C)
+    x, w = rng.normal(0, 1, (2, C, H, W)).astype(np.float32), rng.normal(0, 1, (F, C, k, k)).astype(np.float32)
+    tw = be.upload_f32(w.shape, w)
+
+    def conv(x):
+        x = np.ascontiguousarray(x)
+        return be.download_f32(be.conv2d_f32(be.upload_f32(x.shape, x), tw, (len(x), F, H, W), C, H, W, F, k, 1, 1, 1, k // 2, 1))
+
+    alone = np.concatenate([conv(x[:1]), conv(x[1:])])
+    for n in (2, 9, 40):
+        got = conv(np.resize(x, (n, C, H, W)))
+        np.testing.assert_array_equal(got, np.resize(alone, got.shape))
+
+
+def test_f32_heads_do_not_depend_on_the_batch(be):
+    import lightnet_b200 as ln
+    from lightnet_b200 import synth, zoo
+    x = synth.uniform_images(1, 3, 160, 224, 5)
+    heads = []
+    for batch in (1, 12):
+        net = ln.GpuExecutableNetwork(be, zoo.yolov3_tiny_cfg(224, 160), batch, ln.LN_F32)
+        net.load_weights(synth.he_weights(net.layers(), 3))
+        net.forward(np.repeat(x, batch, 0))
+        heads.append([be.download_f32(net.head(k)) for k in range(net.num_heads())])
+    for a, b in zip(*heads):
+        np.testing.assert_array_equal(np.repeat(a, 12, 0), b)
