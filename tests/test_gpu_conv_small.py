@@ -98,6 +98,54 @@ def test_small_grid_f16(be, monkeypatch, case):
         assert (np.abs(got - ref) <= 2.0 ** -11 * np.abs(ref) + 2.0 ** -13 * size + 2.0 ** -24).all()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("model,kind", [("yolov4", "int8"), ("yolov4", "fp8"), ("yolov7", "fp8")])
+@pytest.mark.parametrize("exact", [False, True])
+def test_small_grid_networks_layer_by_layer(be, monkeypatch, capfd, model, kind, exact):
+    """Plans of a network, layer by layer against the persistent kernel's: space-to-depth input, pixel groups of 1x1 and 3x3 layers, fused shortcuts
+    (int8), inputs and outputs that are channel slices of a concatenated buffer."""
+    import lightnet_b200 as ln
+    from lightnet_b200 import synth, zoo
+    cfg = (zoo.yolov4_cfg if model == "yolov4" else zoo.yolov7_cfg)(192, 160).replace("activation=logistic", "activation=linear")
+    prec = ln.LN_Q8 if kind == "int8" else ln.LN_F8
+    x = synth.uniform_images(2, 3, 160, 192, 9)
+    outs, plans, scales = [], [], None
+    monkeypatch.setenv("LN_DEBUG_PLAN", "1")
+    be.set_exact_epilogue(exact)
+    try:
+        for off in ("", "small"):
+            monkeypatch.setenv("LN_CONV_DISABLE", off)
+            net = ln.GpuExecutableNetwork(be, cfg, 2, prec)
+            net.load_weights(synth.he_weights(net.layers(), 3))
+            if scales is None:
+                net.calibrate(x)
+                scales = net.scales()
+            net.set_scales(scales)
+            capfd.readouterr()
+            net.forward(x)
+            plans.append([line for line in capfd.readouterr().err.splitlines() if line.startswith("plan:")])
+            got, fused = {}, 0
+            for i, layer in enumerate(net.layers()):
+                try:
+                    t = net.layer_output(i)
+                except ln.BackendError as e:
+                    assert e.kind == "unsupported"  # fused into the layer after it, or kept in space-to-depth layout
+                    fused += 1
+                    continue
+                got[i] = be.download_f32(t) if t.dtype == ln.LN_F32 else be.download_q(t)[0]
+            outs.append(got)
+            del net
+    finally:
+        be.set_exact_epilogue(False)
+    small = [line for line in plans[0] if "small grid" in line]
+    assert len(small) > 40 and not any("small grid" in line for line in plans[1])
+    assert any("pack 4" in line or "pack 2" in line for line in small)
+    assert fused >= (20 if model == "yolov4" and kind == "int8" else 1 if model == "yolov4" else 0)
+    assert outs[0].keys() == outs[1].keys()
+    for i in outs[0]:
+        np.testing.assert_array_equal(outs[0][i], outs[1][i], err_msg="layer %d" % i)
+
+
 PROGRAM = r"""
 #include <cstdio>
 #include "ln_conv_plan.h"

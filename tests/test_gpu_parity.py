@@ -168,6 +168,13 @@ def test_q8_conv_accumulators_bit_exact(be, case):
         assert d.max() <= 1 and (d > 0).mean() < 0.05, (act_name, d.max(), (d > 0).mean())
 
 
+@pytest.mark.parametrize("case", Q8_CASES)
+def test_q8_conv_persistent_kernel_bit_exact(be, case, monkeypatch):
+    """The same layers with the kernel for small grids off: the modes of the persistent kernel that the list names, whatever the size."""
+    monkeypatch.setenv("LN_CONV_DISABLE", "small")
+    test_q8_conv_accumulators_bit_exact(be, case)
+
+
 TWO_ISSUER_CASES = [  # every CTA gets two or three tiles, so both the paired and the lone last tile of the two-issuer kernel are run
     (8, 128, 76, 76, 128, 3, 1, 1),    # resident weights, 361 tiles: the planner's own choice of two issuers
     (8, 128, 76, 76, 256, 3, 1, 1),    # 256-filter tile, weight tiles shared through the ring (forced)
@@ -939,6 +946,12 @@ def test_f8_conv_matches_oracle(be, case):
         key = lambda z: np.where(z & 0x80, -(z & 0x7F).astype(np.int32), (z & 0x7F).astype(np.int32))
         d = np.abs(key(q) - key(q_ref))
         assert d.max() <= 1 and (d > 0).mean() < 0.05, (act_name, d.max(), (d > 0).mean())
+
+
+@pytest.mark.parametrize("case", F8_CASES)
+def test_f8_conv_persistent_kernel_matches_oracle(be, case, monkeypatch):
+    monkeypatch.setenv("LN_CONV_DISABLE", "small")
+    test_f8_conv_matches_oracle(be, case)
 
 
 def test_f8_glue_matches_oracle(be):
