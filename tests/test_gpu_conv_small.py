@@ -140,6 +140,7 @@ def test_small_grid_networks_layer_by_layer(be, monkeypatch, capfd, model, kind,
     small = [line for line in plans[0] if "small grid" in line]
     assert len(small) > 40 and not any("small grid" in line for line in plans[1])
     assert any("pack 4" in line or "pack 2" in line for line in small)
+    assert model != "yolov4" or any("bk 64" in line and "pack 2" in line for line in small)  # two pixels of 32 channels per row: a 3x3 layer
     assert fused >= (20 if model == "yolov4" and kind == "int8" else 1 if model == "yolov4" else 0)
     assert outs[0].keys() == outs[1].keys()
     for i in outs[0]:
