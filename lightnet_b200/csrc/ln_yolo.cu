@@ -396,20 +396,23 @@ __global__ void __launch_bounds__(256) yolo_head_fill_kernel(const __grid_consta
         }
         if (lane == 0 && t_or != 0ull) { atomicAnd(&key_and_or[2 * img], t_and); atomicOr(&key_and_or[2 * img + 1], t_or); }
     };
-    auto flush_if = [&](int limit, bool last) {
-        // the warp writes its buffered keys out when the next step could overflow the buffer, and at the end
+    auto flush_if = [&](int limit, bool last) -> bool {
+        // the warp writes its buffered keys out when the next step could overflow the buffer, and at the end; false (for the whole warp)
+        // once the image has overflowed: it starts over, so that the rest of the pass would be for nothing
         __syncwarp();
         const int n = s_cnt[warp];
         if (n > limit || (n > 0 && last)) {
             int at = 0;
             if (lane == 0) at = atomicAdd(fill, n);
             at = __shfl_sync(0xffffffffu, at, 0);
+            if (at > dst_cap) return false;
             for (int k = lane; k < n; k += 32)
                 if (at + k < dst_cap) dst[at + k] = s_buf[warp * kWarpBuf + k];
             __syncwarp();
             if (lane == 0) s_cnt[warp] = 0;
         }
         __syncwarp();
+        return true;
     };
     if (n_listed >= 64) {
         // many listed slots: thread t takes listed slot t and walks its classes, eight loads in flight
@@ -437,7 +440,7 @@ __global__ void __launch_bounds__(256) yolo_head_fill_kernel(const __grid_consta
                     }
                 }
             }
-            flush_if(kWarpBuf - 256, c0 + 8 >= p.classes);  // a step adds at most 8 x 32 keys
+            if (!flush_if(kWarpBuf - 256, c0 + 8 >= p.classes)) return;  // a step adds at most 8 x 32 keys
         }
         publish_and_or();
         return;
@@ -460,7 +463,7 @@ __global__ void __launch_bounds__(256) yolo_head_fill_kernel(const __grid_consta
                 if (key != 0ull) emit(key);
             }
         }
-        flush_if(kWarpBuf - 32, base + 256 >= items);  // a step adds at most 32 keys
+        if (!flush_if(kWarpBuf - 32, base + 256 >= items)) return;  // a step adds at most 32 keys
     }
     publish_and_or();
 }
