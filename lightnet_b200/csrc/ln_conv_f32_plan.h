@@ -10,6 +10,23 @@ inline bool ln_conv_f32_blocked(int64_t n, int64_t c, int64_t h, int64_t w, int6
     return n * oh * ow < (1ll << 30) && h * w < (1ll << 31) && n * c * h * w < (1ll << 40) && c * k * k < (1ll << 24) && (f + 63) / 64 <= 65535;
 }
 
+// Whether a convolution of that many images and pixels, F filters and K products per output is for the per-tap kernel: one thread per pixel and four
+// filters, one chain of K steps each, and a second launch for bias and activation (`follow`).  The blocked kernels compute whole tiles of 32 or 64 filters, and a launch of theirs takes about
+// 8 us however little it has to do (ks as in ln_conv_f32_slice).
+//   - little work: 32 filters of 1x1 over one channel, 64 x 64 pixels: 4.2 us against 12.4; 16 of 3x3 over one: 6.2 / 8.4; 32 over four (K = 36): 12.4 /
+//     16.5, over eight (K = 72): 18.5 / 14.5; two filters over four: 12.4 / 10.3
+//   - few filters of a general kernel, which pays for finding every tap: one 5x5 filter over eight channels, 256 x 256: 23 / 66 us, four of them
+//     43 / 66, eight 70 / 68; 64 x 64 pixels: 21 / 21, 35 / 21; one over four
+//     channels, 32 x 32 (K = 100): 12 / 21
+//   - a single 3x3 filter on a large image: 16 channels, 512 x 512: 66 / 93 us, 256 x 256: 27 / 31; two filters: 117 / 94
+// Up to 63 products neither kernel splits a sum and both add in the same order, so the batch may decide; beyond, one image does.
+inline bool ln_conv_f32_per_tap(int64_t images, int64_t plane, int64_t F, int64_t K, int ks, bool follow) {
+    if (!follow && K <= 36 && (ks == 0 || 4 * F >= K) && images * plane * ((F + 3) / 4) <= 65536) return true;
+    const int64_t pixels = K < 64 ? images * plane : plane;
+    if (ks == 0) return (F <= (K < 64 ? 8 : 4) && pixels >= 8192 * F) || (F == 1 && K <= 128);
+    return F == 1 && (ks == 3 || K == 1) && pixels >= 65536;
+}
+
 // Slice of the k range that a kernel holds in shared memory: four channels of a 3x3 kernel or 32 of a 1x1 one where operands are copied
 // asynchronously (`async`), else one channel, or eight k of any other kernel (ks = 1: 1x1 without padding, 3: 3x3 without dilation, 0: anything).
 constexpr int ln_conv_f32_slice(bool async, int ks) { return async ? (ks == 3 ? 36 : 32) : (ks == 3 ? 9 : 8); }

@@ -404,7 +404,8 @@ __global__ void __launch_bounds__(BM * BN / 64, 32768 / (BM * BN)) conv2d_f32_ge
     conv_f32_finish<BM, BN, T>(p, sm.tile, f0, n0);
 }
 
-// Grouped convolutions, and sizes that the blocked kernels do not number (ln_conv_f32_blocked): one thread per (pixel, group of FPT filters).  Semantics of runtime/forward_layers.rs:646-695: taps outside
+// Grouped convolutions, sizes that the blocked kernels do not number (ln_conv_f32_blocked) and those where their tiles are mostly empty
+// (ln_conv_f32_per_tap): one thread per (pixel, group of FPT filters).  Semantics of runtime/forward_layers.rs:646-695: taps outside
 // the image are skipped, groups partition channels, weights are [filters][C/groups][k][k].
 template <int FPT>
 __global__ void conv2d_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y, int B, int C,
@@ -694,10 +695,13 @@ cudaError_t launch_conv_f32(ln_ctx* ctx, K kernel, const ConvF32& p, int threads
     return cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
+// 1: 1x1 without padding, 3: 3x3 without dilation, 0: any other kernel.
+int conv_f32_kind(int k, int pad, int dil) { return k == 1 && pad == 0 ? 1 : (k == 3 && dil == 1 ? 3 : 0); }
+
 // Ungrouped convolution with optional bias and activation, cut as ln_conv_f32_choose says.
 int conv_f32_run(ln_ctx* ctx, ConvF32 p, bool one_chain, const char* who) {
     const int64_t NP = (int64_t)p.B * p.OH * p.OW;
-    const int ks = p.k == 1 && p.pad == 0 ? 1 : (p.k == 3 && p.dil == 1 ? 3 : 0);
+    const int ks = conv_f32_kind(p.k, p.pad, p.dil);
     const bool async = ks != 0 && p.F > 32 && (p.K & 3) == 0 && (((uintptr_t)p.w) & 15) == 0;
     const ln_conv_f32_cut cut = ln_conv_f32_choose(ctx->sm_count, p.B, (int64_t)p.OH * p.OW, p.F, p.K, ks, async, one_chain);
     const bool wide = async && cut.bn == 128, narrow = cut.bm == 32;
@@ -757,7 +761,9 @@ int ln_conv2d_bias_act_f32(ln_ctx* ctx, const ln_tensor* x, const ln_tensor* wei
     if (!y) return LN_ERR_CUDA;
     const float* b = bias ? (const float*)bias->ptr : nullptr;
     int rc = LN_OK;
-    if (groups == 1 && ln_conv_f32_blocked(x->n, input_channels, input_height, input_width, filters, kernel_size, oh, ow)) {
+    const int ks = conv_f32_kind((int)kernel_size, (int)padding, (int)dilation);
+    if (groups == 1 && ln_conv_f32_blocked(x->n, input_channels, input_height, input_width, filters, kernel_size, oh, ow) &&
+        !ln_conv_f32_per_tap(x->n, oh * ow, filters, input_channels * kernel_size * kernel_size, ks, b || activation != LN_ACT_LINEAR)) {
         ConvF32 p = {};
         p.x = (const float*)x->ptr; p.w = (const float*)weights->ptr; p.bias = b; p.y = (float*)y->ptr;
         p.B = (int)x->n; p.C = (int)input_channels; p.H = (int)input_height; p.W = (int)input_width; p.F = (int)filters; p.k = (int)kernel_size;

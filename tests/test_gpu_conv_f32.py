@@ -26,6 +26,12 @@ def be():
     (2, 20, 13, 11, 65, 3, 2, 1, 1),
     (1, 7, 20, 23, 9, 5, 2, 2, 1),       # any kernel size
     (1, 3, 21, 25, 4, 3, 1, 2, 2),       # dilated
+    (1, 9, 21, 25, 12, 3, 1, 2, 2),      # dilated, beyond the little work that the per-tap kernel takes
+    (2, 3, 90, 100, 4, 5, 1, 2, 1),      # four filters of a general kernel, an image too small for the per-tap kernel
+    (1, 2, 200, 190, 3, 5, 1, 2, 1),     # three, large enough
+    (1, 16, 256, 257, 1, 3, 1, 1, 1),    # one 3x3 filter on a large image
+    (1, 1, 300, 220, 1, 1, 1, 0, 1),     # one product
+    (1, 4, 32, 32, 62, 3, 1, 1, 1),      # 36 products, a last group of two filters
     (1, 2, 24, 24, 3, 9, 1, 4, 1),       # more than 64 taps
     (1, 1, 1, 1, 1, 1, 1, 0, 1),
 ])
@@ -58,10 +64,10 @@ def test_conv2d_f32_millions_of_filters(be, filters):
 def test_conv2d_f32_dilation_far_beyond_the_image(be, filters):
     """Only tap (0, 0) lies inside; the pixels of the tile behind the last output read nothing, however far the dilation reaches."""
     rng = np.random.default_rng(filters)
-    x, w = rng.normal(0, 1, (1, 2, 5, 6)).astype(np.float32), rng.normal(0, 1, (filters, 2, 3, 3)).astype(np.float32)
-    t = be.conv2d_f32(be.upload_f32(x.shape, x), be.upload_f32(w.shape, w), (1, filters, 3, 4), 2, 5, 6, filters, 3, 1, 1, 1 << 27, 0, 1)
+    x, w = rng.normal(0, 1, (1, 5, 5, 6)).astype(np.float32), rng.normal(0, 1, (filters, 5, 3, 3)).astype(np.float32)
+    t = be.conv2d_f32(be.upload_f32(x.shape, x), be.upload_f32(w.shape, w), (1, filters, 3, 4), 5, 5, 6, filters, 3, 1, 1, 1 << 27, 0, 1)
     ref = np.einsum("fc,chw->fhw", w[:, :, 0, 0].astype(np.float64), x[0, :, :3, :4].astype(np.float64))
-    assert (np.abs(be.download_f32(t)[0] - ref) <= 35 * 2.0 ** -24 * 2 * np.abs(x).max() * np.abs(w).max()).all()
+    assert (np.abs(be.download_f32(t)[0] - ref) <= 78 * 2.0 ** -24 * 5 * np.abs(x).max() * np.abs(w).max()).all()
 
 
 def test_calibrated_scales_do_not_depend_on_the_batch(be):
@@ -81,11 +87,12 @@ def test_calibrated_scales_do_not_depend_on_the_batch(be):
 @pytest.mark.parametrize("geom", [
     (1, 36, 26, 26, 65, 3, 1, 1, 1),     # blocked, split k range
     (2, 32, 160, 160, 128, 3, 1, 1, 1),  # 64 x 128 tiles
-    (1, 3, 30, 31, 17, 3, 2, 1, 1),      # staged through registers
+    (1, 5, 30, 31, 17, 3, 2, 1, 1),      # staged through registers
+    (1, 3, 30, 31, 17, 3, 2, 1, 1),      # per tap
     (1, 5, 13, 13, 40, 3, 1, 1, 1),      # k range not a multiple of 4
     (2, 64, 9, 9, 70, 1, 1, 1, 1),       # 1x1 with padding: border outputs have no tap at all
     (1, 7, 12, 14, 9, 5, 1, 2, 1),
-    (1, 3, 15, 17, 4, 3, 1, 2, 2),       # dilated
+    (1, 6, 15, 17, 4, 3, 1, 2, 2),       # dilated
     (1, 4, 11, 10, 8, 3, 1, 1, 1, 2),    # grouped
 ])
 def test_conv2d_f32_weights_that_are_not_finite(be, geom):
@@ -120,7 +127,8 @@ def test_conv2d_f32_weights_that_are_not_finite(be, geom):
     assert (np.abs(got[ok] - ref[ok]) <= (C * k * k + 33) * 2.0 ** -24 * size[ok]).all()
 
 
-@pytest.mark.parametrize("geom", [(512, 13, 13, 256, 3), (256, 26, 20, 512, 1), (1024, 4, 4, 255, 1), (68, 19, 21, 40, 3), (7, 20, 23, 9, 5), (35, 30, 30, 17, 3)])
+@pytest.mark.parametrize("geom", [(512, 13, 13, 256, 3), (256, 26, 20, 512, 1), (1024, 4, 4, 255, 1), (68, 19, 21, 40, 3), (7, 20, 23, 9, 5), (35, 30, 30, 17, 3),
+                                  (2, 60, 60, 16, 3), (1, 40, 41, 2, 5), (3, 90, 95, 1, 5), (3, 60, 65, 4, 7), (1, 120, 100, 1, 3)])  # where the choice of the kernel looks at sizes
 def test_conv2d_f32_does_not_depend_on_the_batch(be, geom):
     """An image has the same bits alone and as any of 2, 9 or 40 images: the order of a sum is cut by the size of one image."""
     C, H, W, F, k = geom
