@@ -124,7 +124,10 @@ inline int ln_conv_choose_bn(int64_t F) {
 // per piece of epilogue that a warp does, 9000 for the exchange of partial sums with its two cluster barriers.  (YOLOv4 608 x 608
 // int8, one image, forward: 837 us with 4000 for the exchange, 796 with 6500, 791 with 9000, 802 without any split; with two issuing
 // threads 780 us at 180 cycles per instruction, 757 at 130, 768 at 90.)  Only int8 is split: binary32 sums depend on
-// their order.
+// their order.  The limit of two CTAs per SM holds for all operand types: chains of 25 equal layers in a replayed graph, 26 shapes each from 10 to
+// 180 pixel tiles, took 43 % less to 2 % more time per layer than with the persistent kernel (int8), 41 % less to the same (FP8), 39 % less to
+// 2 % more (binary16); 3x3 C64 at 76x76, four images: 9.3 / 9.2 / 12.5 us persistent, 7.0 / 6.8 / 8.1 here, and level where k ranges are
+// long (3x3 C512 at 19x19, 16 images: 19.8 / 21.8 / 32.8 against 20.2 / 21.5 / 32.5).
 inline bool ln_conv_choose_small(int sm_count, int kind, int64_t m, int64_t F, int64_t fpad, int kblocks, int bk, int* bn_out, int* ks_out) {
     int64_t best = -1;
     for (int bn = 32; bn <= 128; bn *= 2) {

@@ -183,7 +183,7 @@ int ln_image_preprocess_enqueue(ln_ctx* ctx, cudaStream_t stream, const uint8_t*
     return LN_OK;
 }
 
-// Shared by the entry point below and by ln_net_detect_u8: fills `dst` (f32 [count, 3, dst_h, dst_w] on the device) and waits for it.
+// Fills `dst` (f32 [count, 3, dst_h, dst_w] on the device) and waits for it.  (ln_net_detect_u8 enqueues the same and waits after its NMS.)
 int ln_image_preprocess_into(ln_ctx* ctx, const uint8_t* pixels_host, const int64_t* offsets, const int32_t* widths, const int32_t* heights,
                              int32_t count, int32_t mode, int32_t dst_w, int32_t dst_h, float* dst) {
     void* staging = nullptr;

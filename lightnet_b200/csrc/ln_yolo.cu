@@ -16,9 +16,10 @@
 //           compact per-image pool (or, when they fit, straight into the band).  Should one histogram bin hold
 //           more than a pool can (massive ties), the selection descends a digit with another pass.
 //   band  - inside the pool a radix selection over the compact keys (cheap: the pool sits in L2) cuts bands
-//           that fit in shared memory; each band is sorted (bitonic) and resolved by one CTA per image: every
-//           512-candidate chunk is tested against the survivors so far, a 512 x 512 same-class IoU bitmask is
-//           built, and one warp resolves it with shuffles.
+//           that fit in shared memory; each band is sorted (a bitonic network mostly in registers) and resolved
+//           by one CTA per image in chunks of 512 candidates: each is tested against the survivors of its class
+//           bucket, gets a row of bits with the earlier candidates of the chunk that suppress it, and the chunk is
+//           resolved in rounds (kept once all its suppressors are out, out once one is kept).
 //
 // An image stops as soon as it has top_k survivors or runs out of candidates; a pool that is used up before
 // that is followed by the next one further down.  The head tensors are the only large input: they are read
@@ -50,7 +51,7 @@ namespace {
 constexpr int kMaxHeads = 8;
 constexpr int kBandMaxLarge = 16384;  // candidates of one band (sorted in shared memory) when at most 1024 survivors are wanted
 constexpr int kBandMaxSmall = 8192;   // ... when more are wanted (their boxes need the room)
-constexpr int kChunk = 512;      // candidates resolved per bitmask step
+constexpr int kChunk = 512;      // candidates resolved together
 constexpr int kBins = 4096;      // 12-bit radix digits
 constexpr unsigned kPoolChunk = 8192;  // pool keys one block of the pool passes walks
 constexpr int kLevels = 6;       // 5 x 12 bits + 4 bits = 64
@@ -555,8 +556,8 @@ __global__ void __launch_bounds__(256) yolo_pool_select_kernel(const __grid_cons
 }
 
 // After the fill pass: a filled pool goes to band selection, a directly filled band to NMS.  A fill that found more
-// keys than its destination holds (possible only after a sampled histogram) is thrown away and the image starts over
-// with the full histogram.
+// keys than its destination holds (after a histogram, possible only where that was sampled) is thrown away and the image starts
+// over with the full histogram.
 __global__ void yolo_after_fill_kernel(ImgState* __restrict__ states, int* __restrict__ band_fill, int* __restrict__ pool_fill, int batch,
                                        int band_max, int pool_max, int hist_stride, unsigned long long* __restrict__ key_and_or) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
