@@ -364,7 +364,9 @@ int32_t ln_net_set_profile(ln_net* net, int32_t on);
    tensors, and one decode + NMS runs over the whole batch.  Detections are the same as with the pipeline off.  No counterpart
    in the reference. */
 int32_t ln_net_set_host_pipeline(ln_net* net, int32_t on);
-/* 8-bit forwards replay one captured CUDA graph of the whole batch (default on); 0 = launch kernel by kernel. */
+/* 8-bit and binary16 forwards replay one captured CUDA graph of the whole batch (default on); 0 = launch kernel by kernel.  The graph of a
+   binary16 network owns its input, layer outputs and working memory until the weights are loaded again; while the caller holds a
+   head or a layer output of it, forwards run kernel by kernel into tensors of their own (and take the graph's memory where there is no other). */
 int32_t ln_net_set_cuda_graph(ln_net* net, int32_t on);
 int32_t ln_net_profile(const ln_net* net, float* per_layer_ms, int32_t num_layers, float per_op_ms[8], int32_t per_op_launches[8]);
 
